@@ -28,7 +28,7 @@ REFSRC_ENV = "RSGPU_REFERENCE_SRC"
 def build(ref: bool = True) -> None:
     """Build the checkers (the reference part only where its sources exist)."""
     refsrc = os.environ.get(REFSRC_ENV, "")
-    use_ref = ref and bool(refsrc) and os.path.isdir(refsrc)
+    use_ref = ref and bool(refsrc) and os.path.exists(os.path.join(refsrc, "lib", "der.cpp"))
     targets = ["oracle"] + (["ref", f"REFSRC={refsrc}"] if use_ref else [])
     subprocess.run(["make", "-s", "-C", HERE, f"-j{os.cpu_count() or 4}"] + targets, check=True)
     gpu_lib = os.path.join(os.path.dirname(HERE), "rockseis_b200", "librsgpu.so")
