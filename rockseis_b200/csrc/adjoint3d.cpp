@@ -239,6 +239,7 @@ rsgpu_status Adjoint3D::create(const rsgpu_config *c, const rsgpu_adjoint_opts *
         nx[i] = s[i].shot.nx; ny[i] = s[i].shot.ny; nz[i] = s[i].shot.nz; nrec[i] = s[i].shot.nrec;
         nxmax = std::max(nxmax, nx[i]);
         nymax = std::max(nymax, ny[i]);
+        nzmax = std::max(nzmax, nz[i]);
         const size_t n3 = (size_t)nx[i] * ny[i] * nz[i];
         o_img[i] = take(n3 * nhx * nhy * nhz * gs);     // RTM image, or FWI vp gradient
         if (fwi()) {
@@ -473,9 +474,9 @@ rsgpu_status Adjoint3D::slot_io(bool save, int slot)
 
 rsgpu_status Adjoint3D::correlate()
 {
-    cudaError_t e = elastic() ? launch_corr_fwi_e3d(prec, acc, D(o_corr), nshots, nxmax, nymax, cfg.dx, cfg.dy, cfg.dz, stream)
-                    : fwi()   ? launch_corr_fwi_a3d(prec, acc, D(o_corr), nshots, nxmax, nymax, cfg.dx, cfg.dy, cfg.dz, stream)
-                              : launch_corr_rtm_a3d(prec, acc, D(o_corr), nshots, nxmax, nymax, nhx, nhy, nhz, stream);
+    cudaError_t e = elastic() ? launch_corr_fwi_e3d(prec, acc, D(o_corr), nshots, nxmax, nymax, nzmax, cfg.dx, cfg.dy, cfg.dz, stream)
+                    : fwi()   ? launch_corr_fwi_a3d(prec, acc, D(o_corr), nshots, nxmax, nymax, nzmax, cfg.dx, cfg.dy, cfg.dz, stream)
+                              : launch_corr_rtm_a3d(prec, acc, D(o_corr), nshots, nxmax, nymax, nzmax, nhx, nhy, nhz, stream);
     if (e != cudaSuccess) { set_error("correlation launch: %s", cudaGetErrorString(e)); return RSGPU_ERR_CUDA; }
     launches += 1;
     return RSGPU_OK;

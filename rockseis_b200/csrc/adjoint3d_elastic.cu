@@ -49,10 +49,11 @@ __device__ __forceinline__ T half_acc(T u, T w, T r, T dd, double h)
 }
 
 template <typename T, typename G>
-__global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, T dx, T dy, T dz)
+__global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, int nc, T dx, T dy, T dz)
 {
     using O = X<T>;
-    const Corr3DE<T> c = desc[blockIdx.z];
+    const Corr3DE<T> c = desc[blockIdx.z / nc];
+    const int zs = blockIdx.z % nc * CORR_ZC;
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix < 1 || iy < 1 || ix >= c.nx - 1 || iy >= c.ny - 1) return;
@@ -63,7 +64,7 @@ __global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, T dx
     const T *wrx = c.wr[0], *wry = c.wr[1], *wrz = c.wr[2];
     const T *rsxx = c.wr[3], *rsyy = c.wr[4], *rszz = c.wr[5], *rsyz = c.wr[6], *rsxz = c.wr[7], *rsxy = c.wr[8];
     const double DX = (double)dx, DY = (double)dy, DZ = (double)dz;
-    for (int iz = 1; iz < c.nz - 1; iz++) {
+    for (int iz = max(1, zs); iz < min(c.nz - 1, zs + CORR_ZC); iz++) {
         const long long q = (long long)(iz + L) * PL + (long long)(iy + L) * P + (ix + L);
         const long long u = ((long long)iz * c.ny + iy) * c.nx + ix;
         // offsets of the neighbours: x +-1, y +-P, z +-PL
@@ -141,12 +142,13 @@ __global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, T dx
 // columns whose z-derivatives appear, and the rz of the plane below), so a point
 // loads 49 values instead of about 100; x and y neighbours come from L1.
 template <typename G>
-__global__ void __launch_bounds__(256) corr_fwi_e3d_fast(const Corr3DE<float> *desc, float idx, float idy, float idz)
+__global__ void __launch_bounds__(256) corr_fwi_e3d_fast(const Corr3DE<float> *desc, int nc, float idx, float idy, float idz)
 {
-    const Corr3DE<float> c = desc[blockIdx.z];
+    const Corr3DE<float> c = desc[blockIdx.z / nc];
+    const int z0 = max(1, (int)(blockIdx.z % nc) * CORR_ZC), ze = min(c.nz - 1, (int)(blockIdx.z % nc + 1) * CORR_ZC);
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (ix < 1 || iy < 1 || ix >= c.nx - 1 || iy >= c.ny - 1 || c.nz < 3) return;
+    if (ix < 1 || iy < 1 || ix >= c.nx - 1 || iy >= c.ny - 1 || z0 >= ze) return;
     const long long P = c.pitch, PL = c.plane;
     const int L = c.lpml;
     const float *__restrict__ wsx = c.ws[0], *__restrict__ wsy = c.ws[1], *__restrict__ wsz = c.ws[2];
@@ -156,8 +158,8 @@ __global__ void __launch_bounds__(256) corr_fwi_e3d_fast(const Corr3DE<float> *d
     const float *__restrict__ rsxx = c.wr[3], *__restrict__ rsyy = c.wr[4], *__restrict__ rszz = c.wr[5];
     const float *__restrict__ rsyz = c.wr[6], *__restrict__ rsxz = c.wr[7], *__restrict__ rsxy = c.wr[8];
     const float *__restrict__ rx = c.rx, *__restrict__ ry = c.ry, *__restrict__ rz = c.rz;
-    long long q = (long long)(1 + L) * PL + (long long)(iy + L) * P + (ix + L);
-    long long u = ((long long)c.ny + iy) * c.nx + ix;
+    long long q = (long long)(z0 + L) * PL + (long long)(iy + L) * P + (ix + L);
+    long long u = ((long long)z0 * c.ny + iy) * c.nx + ix;
     const long long un = (long long)c.ny * c.nx;
     // values carried from plane to plane: (array, column) at z-1 ("m") and z
     float sx0m = wsx[q - PL], sx0 = wsx[q], sx1m = wsx[q - 1 - PL], sx1 = wsx[q - 1];
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(256) corr_fwi_e3d_fast(const Corr3DE<float> *d
     float szxmm = wsz[q - 1 - PL], szxpm = wsz[q + 1 - PL];
     float xz0m = fsxz[q - PL], xz1m = fsxz[q - 1 - PL], yz0m = fsyz[q - PL], yz1m = fsyz[q - P - PL];
     float zzm = fszz[q - PL], zz0 = fszz[q], rzm = rz[q - PL];
-    for (int iz = 1; iz < c.nz - 1; iz++, q += PL, u += un) {
+    for (int iz = z0; iz < ze; iz++, q += PL, u += un) {
         const float sx0p = wsx[q + PL], sx1p = wsx[q - 1 + PL], sy0p = wsy[q + PL], sy1p = wsy[q - P + PL];
         const float zzp = fszz[q + PL];
         const float sz0 = wsz[q], szym = wsz[q - P], szyp = wsz[q + P], szxm = wsz[q - 1], szxp = wsz[q + 1];
@@ -286,21 +288,22 @@ __global__ void __launch_bounds__(256) residual_misfit_e3d(const Resid3E<T> *des
 
 }  // namespace
 
-cudaError_t launch_corr_fwi_e3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, double dx,
+cudaError_t launch_corr_fwi_e3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, int nzmax, double dx,
                                 double dy, double dz, cudaStream_t st)
 {
-    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots);
+    const int nc = corr_chunks(nzmax);
+    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots * nc);
     if (prec == PREC_F32_FAST) {
         const float ix = (float)(1.0 / dx), iy = (float)(1.0 / dy), iz = (float)(1.0 / dz);
-        if (acc == ACC_F64) corr_fwi_e3d_fast<double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, ix, iy, iz);
-        else corr_fwi_e3d_fast<float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, ix, iy, iz);
+        if (acc == ACC_F64) corr_fwi_e3d_fast<double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, ix, iy, iz);
+        else corr_fwi_e3d_fast<float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, ix, iy, iz);
     } else if (prec == PREC_F64)
-        corr_fwi_e3d<double, double><<<grid, block, 0, st>>>((const Corr3DE<double> *)desc, dx, dy, dz);
+        corr_fwi_e3d<double, double><<<grid, block, 0, st>>>((const Corr3DE<double> *)desc, nc, dx, dy, dz);
     else if (acc == ACC_F64)
-        corr_fwi_e3d<float, double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, (float)dx, (float)dy,
+        corr_fwi_e3d<float, double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, (float)dx, (float)dy,
                                                             (float)dz);
     else
-        corr_fwi_e3d<float, float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, (float)dx, (float)dy,
+        corr_fwi_e3d<float, float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, (float)dx, (float)dy,
                                                            (float)dz);
     return cudaGetLastError();
 }
