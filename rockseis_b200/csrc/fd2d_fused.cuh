@@ -80,7 +80,7 @@ struct ZmGeo {
 // at column c-8 (16-byte aligned pairs).  FW: f[i+k+1]-f[i-k]; BW: f[i+k]-f[i-k-1]
 // (lib/der.cpp:183-188, 378-383), summed in the reference's order.
 template <typename T, int MODE, bool FW>
-__device__ __forceinline__ void dx_pair(const T *row, const T (&cu)[NCOEF], T d, T r, T (&out)[2])
+__device__ __forceinline__ void dx_pair(const T *row, const T (&cu)[NCOEF], T d, const Rcp<T> &r, T (&out)[2])
 {
     using A = Ar<T, MODE>;
     using P = typename Pair<T>::t;
@@ -118,7 +118,7 @@ __device__ __forceinline__ const T *ring_row(const T *s0, const T *s1, const T *
 // four accumulators with paired FMAs (c*w+ and -c*w- as separate terms); other
 // modes: the reference's order with separately rounded operations.
 template <typename T, int MODE, bool FW, int H, int RS>
-__device__ __forceinline__ void dz_ring(const T *s0, const T *s1, const T *s2, const T (&cu)[NCOEF], T d, T r,
+__device__ __forceinline__ void dz_ring(const T *s0, const T *s1, const T *s2, const T (&cu)[NCOEF], T d, const Rcp<T> &r,
                                         T (&out)[4][2])
 {
     using P = typename Pair<T>::t;
@@ -146,7 +146,6 @@ __device__ __forceinline__ void dz_ring(const T *s0, const T *s1, const T *s2, c
         P w[20];
 #pragma unroll
         for (int q = 0; q < 20; q++) w[q] = *reinterpret_cast<const P *>(ring_row<RS>(s0, s1, s2, 4 * H + q));
-        const P d2 = A2::mk(d), r2 = A2::mk(r);
 #pragma unroll
         for (int rr = 0; rr < 4; rr++) {
             P acc;
@@ -156,7 +155,7 @@ __device__ __forceinline__ void dz_ring(const T *s0, const T *s1, const T *s2, c
                 const P c = A2::mk(cu[k]);
                 acc = (k == 0) ? A2::mul(dl, c) : A2::acc(acc, dl, c);
             }
-            const P o = (MODE == MODE_FAST) ? acc : A2::div(acc, d2, r2);
+            const P o = (MODE == MODE_FAST) ? acc : A2::div(acc, d, r);
             out[rr][0] = o.x;
             out[rr][1] = o.y;
         }
@@ -167,7 +166,7 @@ __device__ __forceinline__ void dz_ring(const T *s0, const T *s1, const T *s2, c
 // array ends), reading through the three ring slabs.
 template <typename T, int MODE>
 __device__ __noinline__ T stencil_k_ring(const T *s0, const T *s1, const T *s2, int rs, int Wc, int K, const T *c,
-                                         bool fw, T d, T r)
+                                         bool fw, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     auto at = [&](int W) -> T { return (W < 8 ? s0 : W < 16 ? s1 : s2)[(W & 7) * rs]; };
@@ -186,7 +185,7 @@ __device__ __forceinline__ int kbw_in(int i, int n, int order) { return (i < 0 |
 
 // z-derivative dispatch on the thread's row half (uniform per warp).
 template <typename T, int MODE, bool FW, int RS>
-__device__ __forceinline__ void dz_half(int h, const T *s0, const T *s1, const T *s2, const T (&cu)[NCOEF], T d, T r,
+__device__ __forceinline__ void dz_half(int h, const T *s0, const T *s1, const T *s2, const T (&cu)[NCOEF], T d, const Rcp<T> &r,
                                         T (&out)[4][2])
 {
     if (h == 0) dz_ring<T, MODE, FW, 0, RS>(s0, s1, s2, cu, d, r, out);

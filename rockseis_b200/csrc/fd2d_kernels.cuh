@@ -18,11 +18,10 @@
 // lib/der.cpp:155-540, WavesAcoustic2D/WavesElastic2D::forwardstep* in
 // lib/waves.cpp:217-404, 1416-1735, backwardstep* in lib/waves.cpp:1738-2080):
 //   MODE_IEEE : every add/sub/mul is a separately rounded IEEE op in the
-//               reference's order and the final division is __fdiv_rn;
-//   MODE_RCP  : as MODE_IEEE, but x/d is computed as q=x*r, e=fma(-q,d,x),
-//               q+=e*r (Markstein's correction with r = RN(1/d)); the host only
-//               selects it after checking on the device, for all 2^32 float x,
-//               that it returns exactly what IEEE division returns for this d;
+//               reference's order, and so is the final division by the spacing: in
+//               float by the two-operation formula of Rcp (rsgpu_internal.h), in
+//               double where that does not serve.  Against __fdiv_rn on B200: 24 shots of
+//               641 x 241, 400 steps 69 -> 43 ms, four elastic ones of 461 x 361 43 -> 23;
 //   MODE_FAST : FMA contraction, coefficients pre-divided by the spacing.
 #pragma once
 #include <cuda.h>
@@ -34,7 +33,50 @@
 
 namespace rsgpu {
 
-enum { MODE_IEEE = 0, MODE_RCP = 1, MODE_FAST = 2 };
+enum { MODE_IEEE = 0, MODE_FAST = 2 };
+
+// ------------------------------------------------------------------ division by the spacing
+// Operands that the Rcp formula does not serve (tiny ones, whose error terms underflow;
+// all of them when the divisor failed its check), in double: the quotient is corrected
+// once, so it is exact where x/d is a double (ties of subnormal results among these) and
+// within 2^-52 elsewhere, where x/d is at least 2^-49 from any tie between floats.  A
+// travelling wave is preceded by a fringe of such values: dividing them with __fdiv_rn
+// took a 32 x 32 tile 23,000 cycles instead of 3,700 (its scaled path, lane by lane).
+static __device__ __noinline__ float div_slow(float x, float d, double rd)
+{
+    double q = __dmul_rn((double)x, rd);
+    q = __fma_rn(__fma_rn(-q, (double)d, (double)x), rd, q);
+    return isinf(x) ? x : __double2float_rn(q);
+}
+static __device__ __noinline__ float4 div_slow4(float4 x, float d, double rd)
+{
+    return make_float4(div_slow(x.x, d, rd), div_slow(x.y, d, rd), div_slow(x.z, d, rd), div_slow(x.w, d, rd));
+}
+// 2*bits - 1 of x: above r.lo for the operands the formula serves (zero wraps to the top)
+__device__ __forceinline__ unsigned div_key(float x) { return 2u * __float_as_uint(x) - 1u; }
+__device__ __forceinline__ float div_by(float x, float d, const Rcp<float> &r)
+{
+    float q = __fmaf_rn(x, r.h, __fmul_rn(x, r.l));
+    if (div_key(x) < r.lo) q = div_slow(x, d, r.rd);
+    return q;
+}
+__device__ __forceinline__ double div_by(double x, double d, const Rcp<double> &) { return __ddiv_rn(x, d); }
+// Four quotients with one test between them.
+__device__ __forceinline__ void div_by4(float (&x)[4], float d, const Rcp<float> &r)
+{
+    const float4 v = make_float4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+    for (int j = 0; j < 4; j++) x[j] = __fmaf_rn(x[j], r.h, __fmul_rn(x[j], r.l));
+    if (min(min(div_key(v.x), div_key(v.y)), min(div_key(v.z), div_key(v.w))) < r.lo) {
+        const float4 s = div_slow4(v, d, r.rd);
+        x[0] = s.x; x[1] = s.y; x[2] = s.z; x[3] = s.w;
+    }
+}
+__device__ __forceinline__ void div_by4(double (&x)[4], double d, const Rcp<double> &)
+{
+#pragma unroll
+    for (int j = 0; j < 4; j++) x[j] = __ddiv_rn(x[j], d);
+}
 
 // ------------------------------------------------------------------ scalar arithmetic
 template <typename T, int MODE> struct Ar;
@@ -53,13 +95,7 @@ template <int MODE> struct Ar<float, MODE> {
     {
         return exact ? __fsub_rn(a, __fmul_rn(b, c)) : fmaf(-b, c, a);
     }
-    static __device__ __forceinline__ float div(float a, float d, float r)
-    {
-        if (MODE == MODE_IEEE) return __fdiv_rn(a, d);
-        const float q = __fmul_rn(a, r);
-        const float e = fmaf(-q, d, a);
-        return fmaf(e, r, q);
-    }
+    static __device__ __forceinline__ float div(float a, float d, const Rcp<float> &r) { return div_by(a, d, r); }
 };
 template <int MODE> struct Ar<double, MODE> {
     static constexpr bool exact = true;
@@ -68,7 +104,7 @@ template <int MODE> struct Ar<double, MODE> {
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double mad(double a, double b, double c) { return __dadd_rn(a, __dmul_rn(b, c)); }
     static __device__ __forceinline__ double msub(double a, double b, double c) { return __dsub_rn(a, __dmul_rn(b, c)); }
-    static __device__ __forceinline__ double div(double a, double d, double) { return __ddiv_rn(a, d); }
+    static __device__ __forceinline__ double div(double a, double d, const Rcp<double> &r) { return div_by(a, d, r); }
 };
 
 // ------------------------------------------------------------------ paired arithmetic (x-neighbour columns)
@@ -100,9 +136,9 @@ template <int MODE> struct Ar2<float, MODE> {
         return exact ? make_float2(__fadd_rn(s.x, __fmul_rn(d.x, c.x)), __fadd_rn(s.y, __fmul_rn(d.y, c.y)))
                      : __ffma2_rn(d, c, s);
     }
-    static __device__ __forceinline__ P div(P a, P d, P r)
+    static __device__ __forceinline__ P div(P a, float d, const Rcp<float> &r)
     {
-        return make_float2(Ar<float, MODE>::div(a.x, d.x, r.x), Ar<float, MODE>::div(a.y, d.y, r.y));
+        return make_float2(div_by(a.x, d, r), div_by(a.y, d, r));
     }
 };
 template <int MODE> struct Ar2<double, MODE> {
@@ -113,7 +149,7 @@ template <int MODE> struct Ar2<double, MODE> {
     static __device__ __forceinline__ P sub(P a, P b) { return make_double2(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y)); }
     static __device__ __forceinline__ P mul(P a, P b) { return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)); }
     static __device__ __forceinline__ P acc(P s, P d, P c) { return add(s, mul(d, c)); }
-    static __device__ __forceinline__ P div(P a, P d, P) { return make_double2(__ddiv_rn(a.x, d.x), __ddiv_rn(a.y, d.y)); }
+    static __device__ __forceinline__ P div(P a, double d, const Rcp<double> &) { return make_double2(__ddiv_rn(a.x, d), __ddiv_rn(a.y, d)); }
 };
 
 template <typename T> struct Vec4;
@@ -220,7 +256,7 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, u
 // (lib/der.cpp:183-188, 378-383).  `cu` = uniform coefficients (interior), or
 // per-point rows `ce[j]` (edge tiles).
 template <typename T, int MODE, bool FW, bool EDGE>
-__device__ __forceinline__ void dx_quad(const T *srow, const T (&cu)[NCOEF], const T *const (&ce)[4], T d, T r,
+__device__ __forceinline__ void dx_quad(const T *srow, const T (&cu)[NCOEF], const T *const (&ce)[4], T d, const Rcp<T> &r,
                                         T (&out)[4])
 {
     using A = Ar<T, MODE>;
@@ -240,22 +276,22 @@ __device__ __forceinline__ void dx_quad(const T *srow, const T (&cu)[NCOEF], con
             const T c = EDGE ? ce[j][k] : cu[k];
             acc = (k == 0) ? A::mul(dl, c) : A::mad(acc, dl, c);
         }
-        out[j] = (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
+        out[j] = acc;
     }
+    if (MODE != MODE_FAST) div_by4(out, d, r);
 }
 
-// z-derivatives of a column pair (local columns c, c+1 of the tile, as one
+// z-differences (before the division by the spacing) of a column pair (local columns c, c+1 of the tile, as one
 // 64-bit lane pair) for RZ rows starting at tile row zr.  Window of RZ+16 rows.
 template <typename T, int MODE, bool FW, bool EDGE, int W, int RZ>
 __device__ __forceinline__ void dz_pair(const T *s, int zr, int col, const T (&cu)[NCOEF], const T *const (&ce)[RZ],
-                                        T d, T r, typename Pair<T>::t (&out)[RZ])
+                                        typename Pair<T>::t (&out)[RZ])
 {
     using A2 = Ar2<T, MODE>;
     using P = typename Pair<T>::t;
     P w[RZ + 16];
 #pragma unroll
     for (int q = 0; q < RZ + 16; q++) w[q] = *reinterpret_cast<const P *>(s + (zr + q) * W + col);
-    const P d2 = A2::mk(d), r2 = A2::mk(r);
 #pragma unroll
     for (int rr = 0; rr < RZ; rr++) {
         P acc;
@@ -265,7 +301,7 @@ __device__ __forceinline__ void dz_pair(const T *s, int zr, int col, const T (&c
             const P c = A2::mk(EDGE ? ce[rr][k] : cu[k]);
             acc = (k == 0) ? A2::mul(dl, c) : A2::acc(acc, dl, c);
         }
-        out[rr] = (MODE == MODE_FAST) ? acc : A2::div(acc, d2, r2);
+        out[rr] = acc;
     }
 }
 
@@ -363,7 +399,7 @@ constexpr int NMAP = 5;
 // acoustic 3D kernels (+14 %), slower in the acoustic 2D tile kernels of a
 // 64-shot FWI batch (-6 %) and in the elastic 3D kernels (-17 %).
 template <typename T, int MODE>
-__device__ __noinline__ T stencil_k(const T *center, int stride, int K, const T *c, bool fw, T d, T r)
+__device__ __noinline__ T stencil_k(const T *center, int stride, int K, const T *c, bool fw, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     if (K == 0) return T(0);
@@ -376,7 +412,7 @@ __device__ __noinline__ T stencil_k(const T *center, int stride, int K, const T 
     return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
 }
 template <typename T, int MODE>
-__device__ __forceinline__ T stencil_ki(const T *center, int stride, int K, const T *c, bool fw, T d, T r)
+__device__ __forceinline__ T stencil_ki(const T *center, int stride, int K, const T *c, bool fw, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     if (K == 0) return T(0);
@@ -392,14 +428,14 @@ __device__ __forceinline__ T stencil_ki(const T *center, int stride, int K, cons
     return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
 }
 template <bool INL, typename T, int MODE>
-__device__ __forceinline__ T stencil_sel(const T *center, int stride, int K, const T *c, bool fw, T d, T r)
+__device__ __forceinline__ T stencil_sel(const T *center, int stride, int K, const T *c, bool fw, T d, const Rcp<T> &r)
 {
     return INL ? stencil_ki<T, MODE>(center, stride, K, c, fw, d, r) : stencil_k<T, MODE>(center, stride, K, c, fw, d, r);
 }
 
 template <typename T, int MODE, int TX, int TZ, int RZ, bool INL = false>
 __device__ __forceinline__ void row_dx(const T *tile, int row, int xq, const CoefSet<T> &cs, const T (&cu)[NCOEF],
-                                       bool fw, bool xedge, int gx, int nxp, int order, T d, T r, T (&out)[4])
+                                       bool fw, bool xedge, int gx, int nxp, int order, T d, const Rcp<T> &r, T (&out)[4])
 {
     using G = Geo2D<T, TX, TZ, RZ>;
     const T *ce[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -456,7 +492,7 @@ __device__ __forceinline__ void dz_stream_f32(const float *s, int zr, int col, c
 
 template <typename T, int MODE, int TX, int TZ, int RZ, bool FW, bool INL = false>
 __device__ __forceinline__ void block_dz(const T *tile, int zr, int xq, const CoefSet<T> &cs, const T (&cu)[NCOEF],
-                                         bool zedge, int gz, int nzp, int order, T d, T r, T (&out)[RZ][4])
+                                         bool zedge, int gz, int nzp, int order, T d, const Rcp<T> &r, T (&out)[RZ][4])
 {
     using G = Geo2D<T, TX, TZ, RZ>;
     using P = typename Pair<T>::t;
@@ -469,10 +505,13 @@ __device__ __forceinline__ void block_dz(const T *tile, int zr, int xq, const Co
 #pragma unroll
         for (int cp = 0; cp < 2; cp++) {
             P o[RZ];
-            dz_pair<T, MODE, FW, false, G::W, RZ>(tile, zr, xq + GUARD + 2 * cp, cu, ce, d, r, o);
+            dz_pair<T, MODE, FW, false, G::W, RZ>(tile, zr, xq + GUARD + 2 * cp, cu, ce, o);
 #pragma unroll
             for (int q = 0; q < RZ; q++) { out[q][2 * cp] = o[q].x; out[q][2 * cp + 1] = o[q].y; }
         }
+#pragma unroll
+        for (int q = 0; q < RZ; q++)
+            if (MODE != MODE_FAST) div_by4(out[q], d, r);
     }
     if (zedge) {
 #pragma unroll

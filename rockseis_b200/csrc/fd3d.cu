@@ -39,7 +39,7 @@ __device__ __forceinline__ void load_coefs3(CoefSet3<T> &s, const CoefSet3<T> *g
 // coefficients are read from shared memory (one broadcast per tap), which keeps
 // them out of the register file.
 template <typename T, int MODE>
-__device__ __forceinline__ T taps(const T *b, int s, const T *cu, T d, T r)
+__device__ __forceinline__ T taps(const T *b, int s, const T *cu, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     T acc = A::mul(A::sub(b[8 * s], b[7 * s]), cu[0]);
@@ -48,7 +48,7 @@ __device__ __forceinline__ T taps(const T *b, int s, const T *cu, T d, T r)
     return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
 }
 template <typename T, int MODE>
-__device__ __forceinline__ T taps_reg(const T (&q)[16], const T *cu, T d, T r)
+__device__ __forceinline__ T taps_reg(const T (&q)[16], const T *cu, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     T acc = A::mul(A::sub(q[8], q[7]), cu[0]);

@@ -56,7 +56,7 @@ __device__ __forceinline__ void stage_shot(Shot3D<T> &dst, const Shot3D<T> *src)
 // Staggered derivative with all NCOEF taps: b[0] = f[i-7] (forward) or f[i-8]
 // (backward); sum_k (b[8+k] - b[7-k]) c_k in the reference's order.
 template <typename T, int MODE>
-__device__ __forceinline__ T taps3(const T *b, int s, const T *cu, T d, T r)
+__device__ __forceinline__ T taps3(const T *b, int s, const T *cu, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     T acc = A::mul(A::sub(b[8 * s], b[7 * s]), cu[0]);
@@ -65,7 +65,7 @@ __device__ __forceinline__ T taps3(const T *b, int s, const T *cu, T d, T r)
     return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
 }
 template <typename T, int MODE>
-__device__ __forceinline__ T taps3_reg(const T (&q)[16], const T *cu, T d, T r)
+__device__ __forceinline__ T taps3_reg(const T (&q)[16], const T *cu, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     T acc = A::mul(A::sub(q[8], q[7]), cu[0]);
@@ -100,7 +100,7 @@ __device__ __forceinline__ T opnd(const Shot3D<T> &sh, I o, int kind)
 // rule near the array ends; rarely taken).
 template <typename T, int MODE, bool ADJ>
 __device__ __noinline__ T stencil_z_op(const Shot3D<T> &sh, long long o, long long plane, int K, const T *c, bool fw,
-                                       int kind, T d, T r)
+                                       int kind, T d, const Rcp<T> &r)
 {
     using A = Ar<T, MODE>;
     if (K <= 0) return T(0);

@@ -296,6 +296,8 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
     }
     cfg = *c;
     cfg.order = std::min(std::max(c->order, 1), 8);
+    rcp[0] = divisor((float)cfg.dx);
+    rcp[2] = divisor((float)cfg.dz);
     prec = c->precision;
     phys = c->physics;
     nshots = ns;
@@ -668,16 +670,15 @@ static void make_args(void *out, const Plan &p)
     a.ntiles = p.ntiles;
     a.order = p.cfg.order;
     a.dt = (T)p.cfg.dt; a.dx = (T)p.cfg.dx; a.dz = (T)p.cfg.dz;
-    a.rdx = (T)1 / a.dx; a.rdz = (T)1 / a.dz;
+    a.rdx = p.rcp_of(0, a.dx); a.rdz = p.rcp_of(2, a.dz);
     a.pml = (const T *)p.d_pml;
     a.lpml = p.cfg.lpml;
-    static_assert(sizeof a <= 128, "argument block");
     std::memcpy(out, &a, sizeof a);
 }
 
 rsgpu_status Plan::launch_step(int it_base, const int *it_dev, bool adj, cudaEvent_t *ev)
 {
-    alignas(16) unsigned char args[128];
+    alignas(16) unsigned char args[sizeof(Step2DArgs<double>) > sizeof(Step2DArgs<float>) ? sizeof(Step2DArgs<double>) : sizeof(Step2DArgs<float>)];
     if (prec == PREC_F64) make_args<double>(args, *this);
     else make_args<float>(args, *this);
     const int grid = ntiles;

@@ -134,6 +134,9 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
     }
     cfg = *c;
     cfg.order = order;
+    rcp[0] = divisor((float)cfg.dx);
+    rcp[1] = divisor((float)cfg.dy);
+    rcp[2] = divisor((float)cfg.dz);
     prec = c->precision;
     nshots = ns;
     es = prec == PREC_F64 ? 8 : 4;
@@ -545,7 +548,7 @@ static void make_args3(void *out, const Plan3D &p)
     a.zc = p.zc;
     a.lpml = p.cfg.lpml;
     a.dt = (T)p.cfg.dt; a.dx = (T)p.cfg.dx; a.dy = (T)p.cfg.dy; a.dz = (T)p.cfg.dz;
-    a.rdx = (T)1 / a.dx; a.rdy = (T)1 / a.dy; a.rdz = (T)1 / a.dz;
+    a.rdx = p.rcp_of(0, a.dx); a.rdy = p.rcp_of(1, a.dy); a.rdz = p.rcp_of(2, a.dz);
     a.pml = (const T *)p.d_pml;
     a.maps = p.d_maps;
     a.err = p.d_err;

@@ -50,7 +50,7 @@ static void fill_zm_args(std::vector<unsigned char> &out, const Plan &p, const v
     a.maps = maps;
     a.order = p.cfg.order;
     a.dt = (T)p.cfg.dt; a.dx = (T)p.cfg.dx; a.dz = (T)p.cfg.dz;
-    a.rdx = (T)1 / a.dx; a.rdz = (T)1 / a.dz;
+    a.rdx = p.rcp_of(0, a.dx); a.rdz = p.rcp_of(2, a.dz);
     a.pml = (const T *)p.d_pml;
     a.lpml = p.cfg.lpml;
     out.resize(sizeof a);

@@ -5,6 +5,7 @@
 // to the reference's for T = float and T = double.  Callers that already hold
 // reference objects pass the reference's own arrays to the plan instead.
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <vector>
 
@@ -12,6 +13,50 @@
 #include "rsgpu_host.h"
 
 namespace rsgpu {
+
+// Constants of RN(x*h + RN(x*l)) = RN(x/d) (see Rcp), checked for this d.  The computed
+// sum is within 2^-46 relative of x/d: l is rounded to 2^-24 of a value below 2^-23 h,
+// and so is x*l.  With integer mantissas X and D of 24 bits, x/d can only round wrongly
+// if a midpoint M (odd, 25 bits) of two floats lies that close, i.e. if
+// |X 2^S - M D| <= 8 for S = 24 (X >= D) or 25 (X < D); never 0, since M and the odd
+// part of D share no factor two.  Each such X is found from M = -n D^-1 mod 2^S and
+// tried.  x below d*2^-97 (quotients whose error terms underflow) are divided by the
+// caller's slow path, as is everything when a trial fails.
+Rcp<float> divisor(float d)
+{
+    Rcp<float> r = {0.0f, 0.0f, 0xffffffffu, 1.0 / (double)d};
+    if (!(d > 0x1p-28f && d < 0x1p28f)) return r;
+    r.h = (float)(1.0 / (double)d);
+    if ((double)r.h > 1.0 / (double)d) r.h = std::nextafterf(r.h, 0.0f);
+    r.l = (float)((1.0 - (double)d * (double)r.h) / (double)d);   // the numerator is exact
+    if (r.l == 0.0f) r.l = 0x1p-149f;   // d a power of two: keeps x*l zero or below half an ulp, and inf*l infinite
+    int ed;
+    const uint64_t D0 = (uint64_t)std::ldexp((double)std::frexp(d, &ed), 24);
+    int t = 0;
+    while (!((D0 >> t) & 1)) t++;
+    const uint64_t D = D0 >> t;
+    uint64_t inv = D;   // Newton: inverse of D modulo 2^64
+    for (int k = 0; k < 6; k++) inv *= 2 - D * inv;
+    for (int S = 24; S <= 25 && t <= 3; S++)   // t > 3: |X 2^S - M D| >= 2^t > 8
+        for (int n = -8; n <= 8; n++) {
+            if (n == 0 || n % (1 << t) != 0) continue;
+            const uint64_t mod = 1ull << (S - t);
+            const uint64_t m0 = ((uint64_t)(int64_t)(-(n >> t)) * inv) & (mod - 1);
+            for (uint64_t M = m0; M < (1ull << 25); M += mod) {
+                if (M <= (1ull << 24) || !(M & 1)) continue;
+                const uint64_t X = (uint64_t)((int64_t)(M * D0) + n) >> S;
+                if (X < (1ull << 23) || X >= (1ull << 24) || (X >= D0) != (S == 24)) continue;
+                const float x = (float)X;
+                volatile float q1 = x * r.l, want = x / d;
+                if (std::fma(x, r.h, (float)q1) != want) return r;
+            }
+        }
+    const float lo = d * 0x1p-97f;
+    uint32_t b;
+    std::memcpy(&b, &lo, sizeof b);
+    r.lo = 2 * b - 1;
+    return r;
+}
 
 // Pml<T>::computeABC(sign=1) with Amax=0, Kmax=2, Smax=1200 (lib/pml.cpp:79-126,
 // include/pml.h:14-16).  Output order: A,B,C ltf; A,B,C ltf_stag; A,B,C rbb; A,B,C rbb_stag.

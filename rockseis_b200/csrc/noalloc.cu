@@ -241,7 +241,7 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     a.ntiles = (int)tiles.size();
     a.order = order;
     a.dt = (float)cfg->dt; a.dx = (float)cfg->dx; a.dz = (float)cfg->dz;
-    a.rdx = 1.0f / a.dx; a.rdz = 1.0f / a.dz;
+    a.rdx = divisor(a.dx); a.rdz = divisor(a.dz);
     a.pml = (const float *)(S + o_pml);
     a.lpml = lp;
     int *derr = (int *)(S + o_err);

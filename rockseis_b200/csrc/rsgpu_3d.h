@@ -75,7 +75,7 @@ struct Step3DArgs {
     const Tile3D *tiles;
     int ntiles, order, zc, lpml;
     T dt, dx, dy, dz;
-    T rdx, rdy, rdz;
+    Rcp<T> rdx, rdy, rdz;
     const T *pml;
     const void *maps;          // elastic fast mode: NMAP_E3 CUtensorMaps per shot (null: no TMA kernels)
     int *err;                  // device error word (a bounded wait that gave up)

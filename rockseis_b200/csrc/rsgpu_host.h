@@ -5,12 +5,17 @@
 #include <string>
 #include <vector>
 #include <cuda_runtime.h>
+#include "rsgpu_internal.h"
 #include "rsgpu_kernels.h"
 
 namespace rsgpu {
 
 // thread-local last-error text behind rsgpu_last_error()
 void set_error(const char *fmt, ...);
+
+// The divisor constants of the exact float kernels (rsgpu_internal.h, Rcp).
+Rcp<float> divisor(float d);
+inline Rcp<double> divisor(double) { return {0}; }
 
 void pml_tables_host(int lpml, double dt, int prec, void *out);
 int stagger_host(int physics, int nx, int ny, int nz, int l, int fs, int prec, const void *vp, const void *vs,

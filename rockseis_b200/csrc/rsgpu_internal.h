@@ -121,6 +121,23 @@ enum RecKind {
     REC_E2_PSUM = 7,  // xtri*ytri*(Sxx + Szz) in T: the elastic wavelet gradient (lib/fwi.cpp:2681-2697)
 };
 
+// A divisor d known before the launch, for correctly rounded division by one multiply
+// and one multiply-add (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans. Comput.
+// 53(8), 2004): x/d = RN(x*h + RN(x*l)) with h = RD(1/d) and l = RN(1/d - h).
+// divisor() checks every quotient that could round wrongly for this d; `lo` is 2*bits - 1
+// of the smallest magnitude of x the formula serves (0xffffffff: none, d failed the check).
+template <typename T>
+struct Rcp {
+    unsigned lo;       // double: divided by the hardware routine
+};
+template <>
+struct Rcp<float> {
+    float h, l;
+    unsigned lo;
+    double rd;         // RN(1/d) in double, for the operands below lo
+};
+
 // Arguments of one 2D half-step launch (passed by value).
 template <typename T>
 struct Step2DArgs {
@@ -129,7 +146,7 @@ struct Step2DArgs {
     int ntiles;
     int order;
     T dt, dx, dz;
-    T rdx, rdz;        // RN(1/dx), RN(1/dz): reciprocal-division mode only
+    Rcp<T> rdx, rdz;   // dx and dz as divisors
     const T *pml;      // 12*lpml C-PML tables
     int lpml;
 };
@@ -155,7 +172,7 @@ struct Zm2DArgs {
     const void *maps;             // CUtensorMap [shot][copy][ring field]
     int order;
     T dt, dx, dz;
-    T rdx, rdz;
+    Rcp<T> rdx, rdz;
     const T *pml;                 // 12*lpml C-PML tables
     int lpml;
 };

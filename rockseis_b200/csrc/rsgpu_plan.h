@@ -81,6 +81,9 @@ public:
     cudaStream_t shared_stream = nullptr;  // run on this caller-owned stream
 
     rsgpu_config cfg{};
+    Rcp<float> rcp[3] = {};              // dx, dy, dz as divisors of the exact float kernels
+    Rcp<float> rcp_of(int axis, float) const { return rcp[axis]; }
+    Rcp<double> rcp_of(int, double) const { return {0}; }
     int prec = 0, phys = 0, nshots = 0, tilecfg = 0, ntiles = 0;
     std::vector<ShotLayout> shots;
     std::vector<size_t> rec_pt_offsets;   // [shot*MAXSETS + set]: arena offset of the receiver points (-1 = off grid)

@@ -52,6 +52,9 @@ public:
     cudaStream_t shared_stream = nullptr;      // run on this caller-owned stream
 
     rsgpu_config cfg{};
+    Rcp<float> rcp[3] = {};              // dx, dy, dz as divisors of the exact float kernels
+    Rcp<float> rcp_of(int axis, float) const { return rcp[axis]; }
+    Rcp<double> rcp_of(int, double) const { return {0}; }
     int prec = 0, phys = PHYS_A3D, nshots = 0, es = 4, zc = 64, ntiles = 0;
     int nsets = 1;                             // InjRec3 entries per shot (elastic: MAXSETS)
     std::vector<Layout3D> shots;
