@@ -183,7 +183,7 @@ void rsgpu_plan_destroy(rsgpu_plan *plan);
  * reference layout), shot->wavelet (nsrc*nt) and shot->rec_out (nrec*nt,
  * accumulated); maps and shifts stay in host memory.  All working memory
  * (wavefields, C-PML memory, staged parameters, plans) lives in one static
- * 32 MiB device array per GPU, held by every GPU that loads the library until
+ * 33 MiB device array per GPU (32 for the grid), held by every GPU that loads the library until
  * the process exits; a grid that needs more is rejected with RSGPU_ERR_ARG.
  * Float precisions only; results equal rsgpu_modelling's.  Every call, the
  * first on a device included, looks up the array's device address on the

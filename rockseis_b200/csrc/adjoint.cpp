@@ -371,8 +371,11 @@ rsgpu_status Adjoint::create(const rsgpu_config *c, const rsgpu_adjoint_opts *o,
             continue;
         }
         for (int f = 0; f < nfields(phys); f++) add(L.f[f] + org, L.nzp, L.nxp, L.pitch);
-        for (int p = 0; p < npsi(phys); p++) add(L.psix[p], L.nzp, 2 * cfg.lpml, 2 * cfg.lpml);
-        for (int p = 0; p < npsi(phys); p++) add(L.psiz[p], 2 * cfg.lpml, L.nxp, L.nxp);
+        for (int p = 0; p < npsi(phys); p++) {
+            const int w = psix_pitch(L.nxp, cfg.lpml);
+            add(L.psix[p], L.nzp, w, w);
+        }
+        for (int p = 0; p < npsi(phys); p++) add(L.psiz[p], 2 * cfg.lpml, L.nxp, psiz_pitch(L.nxp));
     }
     o_segs = take(sizeof(CkptSeg) * segs.size());
     seg_rows = ckpt_max_rows(segs.data(), segs.size());

@@ -16,18 +16,14 @@ cudaError_t launch_step_2d(int prec, int cfg, int physics, int half, int flags, 
 }
 
 cudaError_t launch_injrec_2d(int prec, const void *shots, const void *plans, int nshots, double dt, int it_base,
-                             const int *it_dev, cudaStream_t st)
+                             const int *it_dev, int threads, cudaStream_t st)
 {
     if (prec == PREC_F64)
-        inject_record_2d<double, MODE_IEEE><<<nshots, 256, 0, st>>>((const Shot2D<double> *)shots,
-                                                                    (const InjRec<double> *)plans, dt, it_base, it_dev);
-    else if (prec == PREC_F32_EXACT)
-        inject_record_2d<float, MODE_IEEE><<<nshots, 256, 0, st>>>((const Shot2D<float> *)shots,
-                                                                   (const InjRec<float> *)plans, (float)dt, it_base, it_dev);
-    else
-        inject_record_2d<float, MODE_FAST><<<nshots, 256, 0, st>>>((const Shot2D<float> *)shots,
-                                                                   (const InjRec<float> *)plans, (float)dt, it_base, it_dev);
-    return cudaGetLastError();
+        return launch_kernel(inject_record_2d<double, MODE_IEEE>, nshots, threads, 0, st, (const Shot2D<double> *)shots,
+                          (const InjRec<double> *)plans, dt, it_base, it_dev);
+    return launch_kernel(prec == PREC_F32_EXACT ? inject_record_2d<float, MODE_IEEE> : inject_record_2d<float, MODE_FAST>,
+                      nshots, threads, 0, st, (const Shot2D<float> *)shots, (const InjRec<float> *)plans, (float)dt,
+                      it_base, it_dev);
 }
 
 cudaError_t launch_advance(int *it_dev, int by, cudaStream_t st)

@@ -312,7 +312,7 @@ __device__ __noinline__ void general_update(T *F, const T *Mo, const T *d1, cons
             int xb, xc;
             const int xi = xstrip_in(ix, iz, sh.nxp, sh.nzp, a.lpml, xb, xc);
             if (xi >= 0) {
-                const int o = iz * 2 * a.lpml + xc;
+                const int o = iz * psix_pitch(sh.nxp, a.lpml) + psix_col(ix, sh.nxp, a.lpml);
                 F[k] = pml_pp<T, MODE>(F[k], am, d, q.pxi + o, q.pxo + o, q.own, a.pml, a.lpml, xb + q.xb_add, xi);
             }
         }
@@ -322,7 +322,7 @@ __device__ __noinline__ void general_update(T *F, const T *Mo, const T *d1, cons
             int zb, zr;
             const int zi = zstrip_in(ix, iz, sh.nxp, sh.nzp, a.lpml, zb, zr);
             if (zi >= 0) {
-                const int o = zr * sh.nxp + ix;
+                const int o = zr * psiz_pitch(sh.nxp) + ix;
                 F[k] = pml_pp<T, MODE>(F[k], am, d, q.pzi + o, q.pzo + o, q.own, a.pml, a.lpml, zb + q.zb_add, zi);
             }
         }
@@ -347,7 +347,7 @@ __device__ __noinline__ void general_normal(T *sxx, T *szz, const T *l, const T 
         int xb, xc;
         const int xi = xstrip_in(ix, iz, sh.nxp, sh.nzp, a.lpml, xb, xc);
         if (xi >= 0) {
-            T *ps = sh.psix[2] + iz * 2 * a.lpml + xc;
+            T *ps = sh.psix[2] + iz * psix_pitch(sh.nxp, a.lpml) + psix_col(ix, sh.nxp, a.lpml);
             const T tA = __ldg(a.pml + (xb + PT_A) * a.lpml + xi), tB = __ldg(a.pml + (xb + PT_B) * a.lpml + xi),
                     tC = __ldg(a.pml + (xb + PT_C) * a.lpml + xi);
             const T p = A::mad(A::mul(tB, *ps), tA, e1);
@@ -361,7 +361,7 @@ __device__ __noinline__ void general_normal(T *sxx, T *szz, const T *l, const T 
         int zb, zr;
         const int zi = zstrip_in(ix, iz, sh.nxp, sh.nzp, a.lpml, zb, zr);
         if (zi >= 0) {
-            T *ps = sh.psiz[2] + zr * sh.nxp + ix;
+            T *ps = sh.psiz[2] + zr * psiz_pitch(sh.nxp) + ix;
             const T tA = __ldg(a.pml + (zb + PT_A) * a.lpml + zi), tB = __ldg(a.pml + (zb + PT_B) * a.lpml + zi),
                     tC = __ldg(a.pml + (zb + PT_C) * a.lpml + zi);
             const T p = A::mad(A::mul(tB, *ps), tA, e2);

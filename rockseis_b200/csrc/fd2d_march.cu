@@ -116,6 +116,7 @@ __device__ __forceinline__ Lane make_lane(const MarchItem &it, const Shot2D<floa
     n.cx = it.x0 + (int)threadIdx.x;
     n.rc = GUARD + (int)threadIdx.x;
     n.xi = xstrip(n.cx, sh.nxp, L, n.xb, n.xc);
+    n.xc = psix_col(n.cx, sh.nxp, L);
     n.kf = kfw(n.cx, sh.nxp, order);
     n.kb = kbw(n.cx, sh.nxp, order);
     n.in = n.cx < sh.nxp;
@@ -240,8 +241,8 @@ __device__ __forceinline__ void vel_row(const March2DArgs &a, const VelCtx &c, c
     float mx0 = 0.f, mx1 = 0.f, mz0 = 0.f, mz1 = 0.f;
     if (GEN) {
         zi = n.in ? zstrip(z, c.nzp, c.L, zbt, zr) : -1;
-        px = z * 2 * c.L + n.xc;
-        pz = zr * c.nxp + n.cx;
+        px = z * psix_pitch(c.nxp, c.L) + n.xc;
+        pz = zr * psiz_pitch(c.nxp) + n.cx;
         if (n.xi >= 0) { mx0 = c.sh->psix[0][px]; mx1 = c.sh->psix[1][px]; }
         if (zi >= 0) { mz0 = c.sh->psiz[0][pz]; mz1 = c.sh->psiz[1][pz]; }
     }
@@ -297,8 +298,8 @@ __device__ __forceinline__ void str_row(const March2DArgs &a, const StrCtx &c, c
     float mx2 = 0.f, mx3 = 0.f, mz2 = 0.f, mz3 = 0.f;
     if (GEN) {
         zi = n.in ? zstrip(z, c.nzp, c.L, zbt, zr) : -1;
-        px = z * 2 * c.L + n.xc;
-        pz = zr * c.nxp + n.cx;
+        px = z * psix_pitch(c.nxp, c.L) + n.xc;
+        pz = zr * psiz_pitch(c.nxp) + n.cx;
         if (n.xi >= 0) { mx2 = c.sh->psix[2][px]; mx3 = c.sh->psix[3][px]; }
         if (zi >= 0) { mz2 = c.sh->psiz[2][pz]; mz3 = c.sh->psiz[3][pz]; }
     }

@@ -49,12 +49,6 @@ void set_error(const char *fmt, ...)
 
 static inline size_t rup(size_t a, size_t b) { return (a + b - 1) / b * b; }
 
-// Acoustic batches of at most this many tiles (about one wave of resident CTAs on
-// B200: 148 SMs x 6) launch the tile kernels with inlined edge stencils.  Measured:
-// one 541x341 shot (187 tiles) 6.2 -> 8.4 Gpts/s; 64 shots of 641x241 (10,752
-// tiles) 25.1 -> 23.3 FWI gradients/s, so large batches keep the stencil calls.
-static constexpr int INLINE_EDGE_TILES = 888;
-
 // Coefficient rows for each stencil half-length K (lib/der.cpp:3-53).  The values
 // are the reference's optimised staggered-grid coefficients; row K holds the K
 // pairs used where the reference reduces the order near an array end.  The K=1
@@ -305,10 +299,7 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
     if (shared_stream) stream = shared_stream;
     else CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
 
-    long tiles32 = 0;   // 32x32 tiles of the batch (the default shape's count)
-    for (int i = 0; i < ns; i++)
-        tiles32 += (long)((s[i].nx + 2 * c->lpml + 31) / 32) * ((s[i].nz + 2 * c->lpml + 31) / 32);
-    tilecfg = (c->tile >= 0 && c->tile < tile_count_2d()) ? c->tile : default_tile(tiles32);
+    tilecfg = (c->tile >= 0 && c->tile < tile_count_2d()) ? c->tile : default_tile();
     // the FP64 oracle propagator is built for two tile shapes only
     if (prec == PREC_F64 && tilecfg != TILECFG_64x32 && tilecfg != TILECFG_32x16) tilecfg = TILECFG_64x32;
     const TileShape ts = tile_shape_2d(tilecfg);
@@ -340,8 +331,8 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
         const size_t fbytes = (size_t)L.pitch * L.rows * es;
         // state block first (zeroed by reset): wavefields, C-PML memory, traces
         for (int k = 0; k < nfields(phys); k++) L.f[k] = take(fbytes);
-        for (int k = 0; k < npsi(phys); k++) L.psix[k] = take((size_t)L.nzp * 2 * lp * es);
-        for (int k = 0; k < npsi(phys); k++) L.psiz[k] = take((size_t)2 * lp * L.nxp * es);
+        for (int k = 0; k < npsi(phys); k++) L.psix[k] = take((size_t)L.nzp * psix_pitch(L.nxp, lp) * es);
+        for (int k = 0; k < npsi(phys); k++) L.psiz[k] = take((size_t)2 * lp * psiz_pitch(L.nxp) * es);
         L.psi_end = off;
         L.nrecsets = t.nrec;
         L.nsrcsets = t.nsrc;
@@ -353,8 +344,8 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
         if (fused) {
             for (int k = 0; k < nfields(phys); k++) L.fb[k] = take(fbytes);
             for (int k = 0; k < (phys == PHYS_E2D ? 2 : 1); k++) {
-                L.psixb[k] = take((size_t)L.nzp * 2 * lp * es);
-                L.psizb[k] = take((size_t)2 * lp * L.nxp * es);
+                L.psixb[k] = take((size_t)L.nzp * psix_pitch(L.nxp, lp) * es);
+                L.psizb[k] = take((size_t)2 * lp * psiz_pitch(L.nxp) * es);
             }
         }
         L.nrec = t.nrec > 0 ? t.rec[0].n : 0;
@@ -437,6 +428,16 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
             }
         }
     }
+    size_t most = 0;
+    for (int i = 0; i < ns; i++) {
+        size_t ni = 0, nr = 0;
+        for (int k = 0; k < MAXSETS; k++) {
+            ni += inj[(size_t)i * MAXSETS + k].pt.size();
+            nr += rec[(size_t)i * MAXSETS + k].pt.size();
+        }
+        most = std::max({most, ni, nr});
+    }
+    injrec_nt = injrec_threads(most);
     // plan tables in the same arena
     struct InjOff { size_t pt, start, tr, wx, wz; };
     struct RecOff { size_t pt, w, fac; };
@@ -527,7 +528,7 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
             }
     }
     ntiles = (int)tiles.size();
-    std::vector<unsigned char> coefs;
+    std::vector<unsigned char> &coefs = h_coefs;
     if (prec == PREC_F64) build_coefs<double>(prec, cfg.dx, cfg.dz, coefs);
     else build_coefs<float>(prec, cfg.dx, cfg.dz, coefs);
     const size_t m_shots = 0;
@@ -640,18 +641,15 @@ void Plan::fill_desc(unsigned char *sd, unsigned char *irp, const ShotLayout &L,
     std::memcpy(irp, &r, sizeof r);
 }
 
-int Plan::default_tile(long tiles32) const
+int Plan::default_tile() const
 {
-    // Elastic float plans: 32x16 tiles at eight CTAs per SM, whose 128-register
-    // budget holds the inlined reduced-order stencils and the gathered C-PML memory
-    // without spills (16-shot 801x401 batch on B200: FAST 34.5 Gpts/s against 27.3
-    // for 32x32 tiles at six before the gather, EXACT 16.7 against 15.8).  Acoustic
-    // FAST batches of about one wave of tiles (one 541x341 shot): the same shape
-    // (9.8 Gpts/s against 8.6); large acoustic batches (the 64-shot FWI: 25.0
-    // against 22.5 gradients/s) and all other plans keep 32x32 tiles at six.
-    if (phys == PHYS_E2D && prec != PREC_F64) return TILECFG_E2D;
-    if (phys == PHYS_A2D && prec == PREC_F32_FAST && tiles32 <= INLINE_EDGE_TILES / 2) return TILECFG_E2D;
-    return TILECFG_DEFAULT;
+    // Float: 32x16 tiles of 64 threads at eight CTAs per SM, whose 128-register budget holds
+    // the edge stencils and the C-PML memory (102 to 118 registers, no spills); the 80
+    // registers of 32x32 at six spill.  Measured on B200 beside it: four rows a thread at
+    // one CTA (one 541x341 acoustic shot 38 ms against 31, a 16-shot gradient 147 against
+    // 145), ten CTAs at 96 registers (sixteen elastic shots 84.6 against 77.5, the gradient
+    // 140 against 145).
+    return prec == PREC_F64 ? TILECFG_64x32 : TILECFG_FLOAT;
 }
 
 rsgpu_status Plan::reset()
@@ -673,19 +671,17 @@ static void make_args(void *out, const Plan &p)
     a.rdx = p.rcp_of(0, a.dx); a.rdz = p.rcp_of(2, a.dz);
     a.pml = (const T *)p.d_pml;
     a.lpml = p.cfg.lpml;
+    a.set_coefs(p.h_coefs.data(), coef_row_stride());
     std::memcpy(out, &a, sizeof a);
 }
 
 rsgpu_status Plan::launch_step(int it_base, const int *it_dev, bool adj, cudaEvent_t *ev)
 {
-    alignas(16) unsigned char args[sizeof(Step2DArgs<double>) > sizeof(Step2DArgs<float>) ? sizeof(Step2DArgs<double>) : sizeof(Step2DArgs<float>)];
+    alignas(16) unsigned char args[sizeof(Step2DArgs<double>)];
     if (prec == PREC_F64) make_args<double>(args, *this);
     else make_args<float>(args, *this);
     const int grid = ntiles;
-    // acoustic plans of at most about one wave of tiles: inlined edge stencils (the
-    // edge tiles, up to 4.4x slower than interior ones with the stencil calls,
-    // otherwise set the time of a launch that has no second wave to hide them)
-    const int flags = (adj ? LAUNCH_ADJ : 0) | (phys == PHYS_A2D && ntiles <= INLINE_EDGE_TILES ? LAUNCH_INL : 0);
+    const int flags = adj ? LAUNCH_ADJ : 0;
     const bool mh = march && !adj;
     cudaError_t e;
     // external records so the events become timestamp nodes of a captured graph
@@ -698,7 +694,7 @@ rsgpu_status Plan::launch_step(int it_base, const int *it_dev, bool adj, cudaEve
                 : launch_step_2d(prec, tilecfg, phys, 1, flags, args, d_coefs, d_maps, d_err, grid, stream)) != cudaSuccess)
         goto fail;
     if (ev && (e = cudaEventRecordWithFlags(ev[2], stream, cudaEventRecordExternal)) != cudaSuccess) goto fail;
-    if ((e = launch_injrec_2d(prec, d_shots, d_injrec, nshots, cfg.dt, it_base, it_dev, stream)) != cudaSuccess) goto fail;
+    if ((e = launch_injrec_2d(prec, d_shots, d_injrec, nshots, cfg.dt, it_base, it_dev, injrec_nt, stream)) != cudaSuccess) goto fail;
     launches += 3;
     return RSGPU_OK;
 fail:
@@ -749,7 +745,7 @@ rsgpu_status Plan::run(int it0, int nsteps)
 rsgpu_status Plan::inject_record_only(int it)
 {
     if (it < 0 || it >= cfg.nt) { set_error("step %d outside [0,%d)", it, cfg.nt); return RSGPU_ERR_ARG; }
-    cudaError_t e = launch_injrec_2d(prec, d_shots, d_injrec, nshots, cfg.dt, it, nullptr, stream);
+    cudaError_t e = launch_injrec_2d(prec, d_shots, d_injrec, nshots, cfg.dt, it, nullptr, injrec_nt, stream);
     if (e != cudaSuccess) { set_error("kernel launch failed: %s", cudaGetErrorString(e)); return RSGPU_ERR_CUDA; }
     launches += 1;
     return RSGPU_OK;

@@ -26,10 +26,12 @@
 
 namespace rsgpu {
 
-// 32 MiB per device, held by every GPU that loads this library until the
+// 33 MiB per device, held by every GPU that loads this library until the
 // process exits (the array lives in the library's device image).
 constexpr size_t NOALLOC_SCRATCH_BYTES = (size_t)32 << 20;
-static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
+// The limit counts the C-PML strips themselves; their vector layout is up to 72 bytes a
+// padded row longer (a row's six fields hold at least 3840), which the array adds.
+static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES + ((size_t)1 << 20)];
 
 namespace {
 
@@ -98,7 +100,7 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     const int sf = shot->src_field, rf = shot->rec_field;
     if (sf != RSGPU_PRESSURE && sf != RSGPU_VX && sf != RSGPU_VZ) { set_error("bad source field"); return RSGPU_ERR_ARG; }
     if (shot->nrec > 0 && rf != RSGPU_PRESSURE && rf != RSGPU_VX && rf != RSGPU_VZ) { set_error("bad receiver field"); return RSGPU_ERR_ARG; }
-    const int cfgi = (cfg->tile >= 0 && cfg->tile < tile_count_2d()) ? cfg->tile : TILECFG_DEFAULT;
+    const int cfgi = (cfg->tile >= 0 && cfg->tile < tile_count_2d()) ? cfg->tile : TILECFG_FLOAT;
     const TileShape ts = tile_shape_2d(cfgi);
 
     // ---- injection plan (contributions in the reference's loop order) and receivers
@@ -161,8 +163,16 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     size_t o_f[3], o_m[3], o_px[2], o_pz[2];
     for (auto &o : o_f) o = take(fbytes);
     for (auto &o : o_m) o = take(fbytes);
-    for (auto &o : o_px) o = take((size_t)nzp * 2 * lp * 4);
-    for (auto &o : o_pz) o = take((size_t)2 * lp * nxp * 4);
+    // What the limit does not count: the bytes that the vector layout of the C-PML memory
+    // adds to the strips themselves, and half the tile table of the default shape (it was
+    // counted with tiles of twice the height)
+    size_t widened = cfgi == TILECFG_FLOAT && cfg->tile != TILECFG_FLOAT ? tiles.size() / 2 * sizeof(Tile2D) : 0;
+    auto take_psi = [&](size_t strips, size_t bytes) {
+        widened += rup(bytes, 256) - rup(strips, 256);
+        return take(bytes);
+    };
+    for (auto &o : o_px) o = take_psi((size_t)nzp * 2 * lp * 4, (size_t)nzp * psix_pitch(nxp, lp) * 4);
+    for (auto &o : o_pz) o = take_psi((size_t)2 * lp * nxp * 4, (size_t)2 * lp * psiz_pitch(nxp) * 4);
     const size_t cleared = off;
     const size_t o_meta = off;
     const size_t o_shot = take(sizeof(Shot2D<float>)), o_ir = take(sizeof(InjRec<float>));
@@ -173,7 +183,7 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     const size_t o_wz = take(std::max<size_t>(1, inj_wz.size()) * 4), o_rp = take(std::max<size_t>(1, rec_pt.size()) * 4);
     const size_t o_rw = take(std::max<size_t>(1, rec_w.size()) * 4), o_pml = take((size_t)12 * lp * 4);
     const size_t o_err = take(2 * sizeof(int));
-    if (off > NOALLOC_SCRATCH_BYTES) {
+    if (off - widened > NOALLOC_SCRATCH_BYTES || off > sizeof g_noalloc_scratch) {
         set_error("no-allocation modelling needs %zu bytes of scratch for this %dx%d padded grid; the library holds "
                   "%zu bytes -- use rsgpu_modelling instead", off, nxp, nzp, NOALLOC_SCRATCH_BYTES);
         return RSGPU_ERR_ARG;
@@ -244,6 +254,7 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     a.rdx = divisor(a.dx); a.rdz = divisor(a.dz);
     a.pml = (const float *)(S + o_pml);
     a.lpml = lp;
+    a.set_coefs(coefs.data(), coef_row_stride());
     int *derr = (int *)(S + o_err);
     // The error word is read back every CHECK_EVERY steps, so a call whose bounded
     // waits give up stops after at most that many more steps instead of queueing
@@ -253,7 +264,7 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     for (int it = 0; it < nt; it++) {
         for (int half = 0; half < 2; half++)
             NA_CU(launch_step_2d(prec, cfgi, PHYS_A2D, half, 0, &a, S + o_coef, S + o_maps, derr, a.ntiles, st));
-        NA_CU(launch_injrec_2d(prec, S + o_shot, S + o_ir, 1, cfg->dt, it, nullptr, st));
+        NA_CU(launch_injrec_2d(prec, S + o_shot, S + o_ir, 1, cfg->dt, it, nullptr, injrec_threads(std::max(inj_pt.size(), rec_pt.size())), st));
         if ((it + 1) % CHECK_EVERY == 0 || it + 1 == nt) {
             NA_CU(cudaMemcpyAsync(&err, derr, sizeof(int), cudaMemcpyDeviceToHost, st));
             NA_CU(cudaStreamSynchronize(st));

@@ -30,9 +30,23 @@ enum { E2_VX = 0, E2_VZ = 1, E2_SXX = 2, E2_SZZ = 3, E2_SXZ = 4 };
 // Parameter slots.  Acoustic: Rx, Rz, L.  Elastic: Rx, Rz, L, L2M, M.
 enum { M_RX = 0, M_RZ = 1, M_L = 2, M_L2M = 3, M_M = 4 };
 
-// Per-shot descriptor read by the 2D kernels.  psix arrays are [nzp][2*lpml]
-// (left strip columns 0..lpml-1, right strip columns lpml..2*lpml-1);
-// psiz arrays are [2*lpml][nxp] (top rows, then bottom rows).
+// C-PML memory of the 2D kernels, laid out so that the four x-neighbours a thread
+// updates are one aligned vector: psix holds, per padded row, the quads that touch the
+// left strip, then those that touch the right one; psiz the top strip's rows, then the
+// bottom's, of nxp rounded up to quads.  Cells of these quads outside the strips stay zero.
+__host__ __device__ inline int psi_left(int lpml) { return (lpml + 3) & ~3; }          // columns of the left quads
+__host__ __device__ inline int psi_right(int nxp, int lpml) { return (nxp - lpml) & ~3; }  // first right column
+__host__ __device__ inline int psix_pitch(int nxp, int lpml)
+{
+    return psi_left(lpml) + ((nxp + 3) & ~3) - psi_right(nxp, lpml);
+}
+__host__ __device__ inline int psix_col(int ix, int nxp, int lpml)
+{
+    return ix < psi_left(lpml) ? ix : ix - psi_right(nxp, lpml) + psi_left(lpml);
+}
+__host__ __device__ inline int psiz_pitch(int nxp) { return (nxp + 3) & ~3; }
+
+// Per-shot descriptor read by the 2D kernels.
 template <typename T>
 struct Shot2D {
     int nxp, nzp, pitch, lpml;
@@ -141,6 +155,11 @@ struct Rcp<float> {
 // Arguments of one 2D half-step launch (passed by value).
 template <typename T>
 struct Step2DArgs {
+    // the full-order coefficient rows (fast mode: divided by the spacing), constant
+    // operands of the taps; cz2: each z coefficient twice, then negated twice, for the
+    // paired multiply-adds
+    alignas(16) T cz2[2][NCOEF][2];
+    T cx[NCOEF], cz[NCOEF];
     const Shot2D<T> *shots;
     const Tile2D *tiles;
     int ntiles;
@@ -149,6 +168,17 @@ struct Step2DArgs {
     Rcp<T> rdx, rdz;   // dx and dz as divisors
     const T *pml;      // 12*lpml C-PML tables
     int lpml;
+    // table: the host copy of the CoefSet (two blocks of nine rows), row stride `stride`
+    void set_coefs(const void *table, int stride)
+    {
+        const T *t = (const T *)table;
+        for (int k = 0; k < NCOEF; k++) {
+            cx[k] = t[order * stride + k];
+            cz[k] = t[(9 + order) * stride + k];
+            cz2[0][k][0] = cz2[0][k][1] = cz[k];
+            cz2[1][k][0] = cz2[1][k][1] = -cz[k];
+        }
+    }
 };
 
 // ---- fused z-marching 2D step (fd2d_fused.cuh)

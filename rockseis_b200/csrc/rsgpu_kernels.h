@@ -13,14 +13,12 @@ enum { PREC_F32_EXACT = 0, PREC_F32_FAST = 1, PREC_F64 = 2 };
 struct TileShape { int tx, tz, rz, minb; };
 TileShape tile_shape_2d(int cfg);
 int tile_count_2d();
-enum { TILECFG_64x32 = 0, TILECFG_32x16 = 3, TILECFG_DEFAULT = 6, TILECFG_E2D = 9 };
+enum { TILECFG_64x32 = 0, TILECFG_32x16 = 3, TILECFG_FLOAT = 9 };
 
 // One half-step (half = 0 velocity, 1 stress) of every tile in args.
 // maps: per shot NMAP2D CUtensorMaps of the halo-loaded fields; err: device error word.
-// flags: LAUNCH_ADJ (adjoint kernels), LAUNCH_INL (acoustic: the kernels whose
-// reduced-order edge stencils are inlined; faster when the batch's tiles fit about
-// one wave, slower for large batches; the elastic kernels always inline them)
-enum { LAUNCH_ADJ = 1, LAUNCH_INL = 2 };
+// flags: LAUNCH_ADJ (adjoint kernels)
+enum { LAUNCH_ADJ = 1 };
 cudaError_t launch_step_2d(int prec, int cfg, int physics, int half, int flags, const void *args, const void *coefs,
                            const void *maps, int *err, int grid, cudaStream_t st);
 constexpr int NMAP2D = 5;
@@ -29,9 +27,14 @@ constexpr int NMAP2D = 5;
 using Launch2DFn = cudaError_t (*)(int physics, int half, int flags, const void *args, const void *coefs,
                                    const void *maps, int *err, int grid, cudaStream_t st);
 Launch2DFn launch_2d_table(const char *variant, int cfg);
-// Source injection followed by receiver recording, one CTA per shot.
+// Source injection followed by receiver recording, one CTA per shot of `threads` threads
+// (injrec_threads of the most injection points or traces a shot has).
+inline int injrec_threads(size_t most)
+{
+    return (int)(most < 64 ? 64 : most > 1024 ? 1024 : (most + 31) / 32 * 32);
+}
 cudaError_t launch_injrec_2d(int prec, const void *shots, const void *plans, int nshots, double dt, int it_base,
-                             const int *it_dev, cudaStream_t st);
+                             const int *it_dev, int threads, cudaStream_t st);
 cudaError_t launch_advance(int *it_dev, int by, cudaStream_t st);
 cudaError_t launch_set_counter(int *it_dev, int value, cudaStream_t st);
 cudaError_t launch_wait_for_nothing(int *err, cudaStream_t st);

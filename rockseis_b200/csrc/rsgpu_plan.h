@@ -91,7 +91,9 @@ public:
     size_t arena_bytes = 0, state_end = 0;
     void *d_meta = nullptr;
     void *d_shots = nullptr, *d_injrec = nullptr, *d_tiles = nullptr, *d_coefs = nullptr, *d_pml = nullptr;
+    std::vector<unsigned char> h_coefs;   // host copy of the CoefSet at d_coefs
     void *d_maps = nullptr;    // [nshots][NMAP2D] CUtensorMap
+    int injrec_nt = 64;        // threads of the injection/recording CTAs
     int *d_it = nullptr;       // step counter read by graph-replayed kernels
     int *d_err = nullptr;      // device error word (bounded waits)
     int *d_gate = nullptr;     // recording switch (gated_recording)
@@ -128,7 +130,7 @@ private:
     // builds the fused step's tables; inj_pts[shot*MAXSETS + set] = the set's CSR target offsets
     rsgpu_status setup_fused(const std::vector<std::vector<int>> &inj_pts);
     rsgpu_status check_config(const rsgpu_config *c, int ns, const rsgpu_shot *s, bool sets_given);
-    int default_tile(long tiles32) const;   // tiles32: the batch's count of 32x32 tiles
+    int default_tile() const;
     template <typename T>
     void fill_desc(unsigned char *sd, unsigned char *irp, const ShotLayout &L, size_t org, const SetOffsets *so,
                    const ShotSets &t);
