@@ -19,9 +19,9 @@ cudaError_t launch_injrec_2d(int prec, const void *shots, const void *plans, int
                              const int *it_dev, int threads, cudaStream_t st)
 {
     if (prec == PREC_F64)
-        return launch_kernel(inject_record_2d<double, MODE_IEEE>, nshots, threads, 0, st, (const Shot2D<double> *)shots,
+        return launch_pdl(inject_record_2d<double, MODE_IEEE>, nshots, threads, 0, st, (const Shot2D<double> *)shots,
                           (const InjRec<double> *)plans, dt, it_base, it_dev);
-    return launch_kernel(prec == PREC_F32_EXACT ? inject_record_2d<float, MODE_IEEE> : inject_record_2d<float, MODE_FAST>,
+    return launch_pdl(prec == PREC_F32_EXACT ? inject_record_2d<float, MODE_IEEE> : inject_record_2d<float, MODE_FAST>,
                       nshots, threads, 0, st, (const Shot2D<float> *)shots, (const InjRec<float> *)plans, (float)dt,
                       it_base, it_dev);
 }

@@ -240,6 +240,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t phase,
     }
     return true;
 }
+// Programmatic dependent launch: a kernel launched by launch_pdl may start while the one
+// before it in the stream drains.  Before pdl_wait it touches only what no kernel writes
+// (descriptors, tables, coefficients); after it everything earlier in the stream is
+// complete and visible.  pdl_trigger, always after the wait, lets the next kernel start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // 2D tiled TMA load of a box at element coordinates (x, y) into shared memory.
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y)
 {
@@ -387,9 +394,10 @@ __device__ __forceinline__ void stage_words(S &dst, const S *src, int t, int nt)
         reinterpret_cast<int *>(&dst)[i] = reinterpret_cast<const int *>(src)[i];
 }
 
-// The prologue of a tile kernel.  The first thread issues the TMA loads of `nmap` halo'd tiles (maps[m_0..]) into consecutive tiles; meanwhile the
+// The prologue of a tile kernel.  The first thread waits for the kernels before and issues
+// the TMA loads of `nmap` halo'd tiles (maps[m_0..]) into consecutive tiles; meanwhile the
 // other warps bring the shot descriptor and, for edge tiles, the coefficient rows to shared
-// memory.  Ends with a block barrier.
+// memory.  Ends with a block barrier, after which every thread has waited.
 template <typename T, int TX, int TZ, int RZ>
 __device__ __forceinline__ void tile_prologue(unsigned char *sm, uint64_t *bar, const CUtensorMap *maps,
                                               const int *which, int nmap, const Tile2D &tl, Shot2D<T> &sh,
@@ -404,11 +412,14 @@ __device__ __forceinline__ void tile_prologue(unsigned char *sm, uint64_t *bar, 
     }
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
+        pdl_wait();
         mbar_expect_tx(bar, (uint32_t)(nmap * G::TILE_BYTES));
         // element (x0 - GUARD, z0 - GUARD) of the field is element (x0, z0) of the allocation
         for (int m = 0; m < nmap; m++) tma_load_2d(sm + m * G::TILE_STRIDE, maps + which[m], bar, tl.x0, tl.z0);
     }
     __syncthreads();
+    pdl_wait();
+    pdl_trigger();
 }
 
 // ------------------------------------------------------------------ acoustic 2D
@@ -1178,6 +1189,8 @@ __global__ void __launch_bounds__(1024) inject_record_2d(const Shot2D<T> *shots,
     stage_words(sh, shots + blockIdx.x, threadIdx.x, blockDim.x);
     stage_words(pl, plans + blockIdx.x, threadIdx.x, blockDim.x);
     __syncthreads();
+    pdl_wait();
+    pdl_trigger();
     const int it_step = it_base + (it_dev ? *it_dev : 0);
     const int it = pl.rev ? pl.nt - 1 - it_step : it_step;
     const int gate = pl.rec_gate ? *pl.rec_gate : 1;
@@ -1263,11 +1276,21 @@ static cudaError_t set_smem(K k, size_t bytes)
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Launch with programmatic stream serialisation (see pdl_wait; the kernel must call it).
 template <typename... P, typename... V>
-static cudaError_t launch_kernel(void (*k)(P...), int grid, int threads, size_t smem, cudaStream_t st, V... args)
+static cudaError_t launch_pdl(void (*k)(P...), int grid, int threads, size_t smem, cudaStream_t st, V... args)
 {
-    k<<<grid, threads, smem, st>>>(static_cast<P>(args)...);
-    return cudaGetLastError();
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
 }
 
 template <typename T, int MODE, int TX, int TZ, int RZ, int MINB>
@@ -1281,11 +1304,11 @@ cudaError_t launch_2d_cfg(int physics, int half, int flags, const Step2DArgs<T> 
         if (half == 0) {
             static const cudaError_t e = set_smem(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, S::bytes(1));
             if (e != cudaSuccess) return e;
-            return launch_kernel(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, S::bytes(1), st, a, coefs, maps, err);
+            return launch_pdl(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, S::bytes(1), st, a, coefs, maps, err);
         } else {
             static const cudaError_t e = set_smem(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, S::bytes(2));
             if (e != cudaSuccess) return e;
-            return launch_kernel(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
+            return launch_pdl(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
         }
     } else {
         if (half == 0) {
@@ -1293,15 +1316,15 @@ cudaError_t launch_2d_cfg(int physics, int half, int flags, const Step2DArgs<T> 
             static const cudaError_t e1 = set_smem(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, S::bytes(3));
             if (e0 != cudaSuccess) return e0;
             if (e1 != cudaSuccess) return e1;
-            if (adj) return launch_kernel(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, S::bytes(3), st, a, coefs, maps, err);
-            else return launch_kernel(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, S::bytes(3), st, a, coefs, maps, err);
+            if (adj) return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, S::bytes(3), st, a, coefs, maps, err);
+            else return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, S::bytes(3), st, a, coefs, maps, err);
         } else {
             static const cudaError_t e0 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, S::bytes(2));
             static const cudaError_t e1 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, S::bytes(2));
             if (e0 != cudaSuccess) return e0;
             if (e1 != cudaSuccess) return e1;
-            if (adj) return launch_kernel(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
-            else return launch_kernel(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
+            if (adj) return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
+            else return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
         }
     }
 }
