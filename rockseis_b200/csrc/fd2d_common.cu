@@ -4,7 +4,6 @@
 
 namespace rsgpu {
 
-static_assert(NMAP2D == NMAP, "tensor-map slots per shot");
 
 cudaError_t launch_step_2d(int prec, int cfg, int physics, int half, int flags, const void *args, const void *coefs,
                            const void *maps, int *err, int grid, cudaStream_t st)

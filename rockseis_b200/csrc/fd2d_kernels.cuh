@@ -359,20 +359,43 @@ template <typename T, int TX, int TZ, int RZ>
 struct Geo2D {
     static constexpr int NTX = TX / 4, NTZ = TZ / RZ, NT = NTX * NTZ;
     static constexpr int W = TX + 2 * GUARD, H = TZ + 2 * GUARD;
-    static constexpr int TILE_BYTES = (int)sizeof(T) * W * H;
-    static constexpr int TILE_STRIDE = (TILE_BYTES + 127) / 128 * 128;
 };
 
 // Shared-memory prologue shared by all 2D kernels: nfield halo'd tiles (TMA),
 // the coefficient tables and one mbarrier.
-template <typename T, int TX, int TZ, int RZ>
+// HALO: per staged field the axes that carry a halo (halo_2d); a field that is
+// differentiated along one axis only needs none along the other, which leaves that much
+// less to fetch from L2 and more of the SM's memory to the L1 its point-wise loads pass
+// through (B200, 600 steps of sixteen 861 x 461 elastic shots 77 -> 73 ms).
+template <typename T, int TX, int TZ, int... HALO>
 struct Smem2D {
-    using G = Geo2D<T, TX, TZ, RZ>;
-    __host__ __device__ static constexpr size_t coef_off(int nfield) { return (size_t)nfield * G::TILE_STRIDE; }
-    __host__ __device__ static constexpr size_t bar_off(int nfield) { return (coef_off(nfield) + sizeof(CoefSet<T>) + 15) / 16 * 16; }
-    __host__ __device__ static constexpr size_t pml_off(int nfield) { return bar_off(nfield) + 16; }
-    __host__ __device__ static constexpr size_t shot_off(int nfield) { return pml_off(nfield) + 6 * (TX + TZ) * sizeof(T); }
-    __host__ __device__ static constexpr size_t bytes(int nfield) { return shot_off(nfield) + sizeof(Shot2D<T>); }
+    __host__ __device__ static constexpr int tile_bytes(int halo)
+    {
+        return (int)sizeof(T) * (TX + (halo & HALO_X ? 2 * GUARD : 0)) * (TZ + (halo & HALO_Z ? 2 * GUARD : 0));
+    }
+    __host__ __device__ static constexpr int halo(int f)
+    {
+        const int h[] = {HALO...};
+        return h[f];
+    }
+    __host__ __device__ static constexpr int nfield() { return (int)sizeof...(HALO); }
+    __host__ __device__ static constexpr size_t off(int f)
+    {
+        size_t o = 0;
+        for (int k = 0; k < f; k++) o += (tile_bytes(halo(k)) + 127) / 128 * 128;
+        return o;
+    }
+    __host__ __device__ static constexpr size_t bar_off() { return (off(nfield()) + sizeof(CoefSet<T>) + 15) / 16 * 16; }
+    __host__ __device__ static constexpr size_t pml_off() { return bar_off() + 16; }
+    __host__ __device__ static constexpr size_t shot_off() { return pml_off() + 6 * (TX + TZ) * sizeof(T); }
+    __host__ __device__ static constexpr size_t bytes() { return shot_off() + sizeof(Shot2D<T>); }
+    // field f's tile, moved so that [row + GUARD][column + GUARD] is the tile's (row, column)
+    // on the axes it is differentiated along, at its own row length
+    static __device__ __forceinline__ T *tile(unsigned char *sm, int f)
+    {
+        T *t = reinterpret_cast<T *>(sm + off(f));
+        return t - (halo(f) & HALO_Z ? 0 : GUARD * (TX + 2 * GUARD)) - (halo(f) & HALO_X ? 0 : GUARD);
+    }
 };
 
 template <typename T>
@@ -395,27 +418,33 @@ __device__ __forceinline__ void stage_words(S &dst, const S *src, int t, int nt)
 }
 
 // The prologue of a tile kernel.  The first thread waits for the kernels before and issues
-// the TMA loads of `nmap` halo'd tiles (maps[m_0..]) into consecutive tiles; meanwhile the
+// the TMA loads of the fields' tiles into consecutive places; meanwhile the
 // other warps bring the shot descriptor and, for edge tiles, the coefficient rows to shared
 // memory.  Ends with a block barrier, after which every thread has waited.
-template <typename T, int TX, int TZ, int RZ>
+template <typename S, typename T, int NT, int N>
 __device__ __forceinline__ void tile_prologue(unsigned char *sm, uint64_t *bar, const CUtensorMap *maps,
-                                              const int *which, int nmap, const Tile2D &tl, Shot2D<T> &sh,
+                                              const int (&field)[N], const Tile2D &tl, Shot2D<T> &sh,
                                               const Shot2D<T> *shots, CoefSet<T> &cs, const CoefSet<T> *coefs)
 {
-    using G = Geo2D<T, TX, TZ, RZ>;
-    constexpr int FIRST = G::NT > 32 ? 32 : 0;
+    static_assert(N == S::nfield(), "one field a tile");
+    constexpr int FIRST = NT > 32 ? 32 : 0;
     if ((int)threadIdx.x >= FIRST) {
-        const int t = threadIdx.x - FIRST, nt = G::NT - FIRST;
+        const int t = threadIdx.x - FIRST, nt = NT - FIRST;
         stage_words(sh, shots + tl.shot, t, nt);
         if (tl.flags & (TILE_XEDGE | TILE_ZEDGE)) stage_words(cs, coefs, t, nt);
     }
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         pdl_wait();
-        mbar_expect_tx(bar, (uint32_t)(nmap * G::TILE_BYTES));
+        uint32_t total = 0;
+#pragma unroll
+        for (int m = 0; m < N; m++) total += S::tile_bytes(S::halo(m));
+        mbar_expect_tx(bar, total);
         // element (x0 - GUARD, z0 - GUARD) of the field is element (x0, z0) of the allocation
-        for (int m = 0; m < nmap; m++) tma_load_2d(sm + m * G::TILE_STRIDE, maps + which[m], bar, tl.x0, tl.z0);
+#pragma unroll
+        for (int m = 0; m < N; m++)
+            tma_load_2d(sm + S::off(m), maps + tl.shot * NMAP2D + field[m], bar, tl.x0 + (S::halo(m) & HALO_X ? 0 : GUARD),
+                        tl.z0 + (S::halo(m) & HALO_Z ? 0 : GUARD));
     }
     __syncthreads();
     pdl_wait();
@@ -425,7 +454,6 @@ __device__ __forceinline__ void tile_prologue(unsigned char *sm, uint64_t *bar, 
 // ------------------------------------------------------------------ acoustic 2D
 // Field tensor maps per shot: [0] P, [1] Vx, [2] Vz  (acoustic)
 //                             [0] Vx, [1] Vz, [2] Sxx, [3] Szz, [4] Sxz (elastic)
-constexpr int NMAP = 5;
 
 // Reduced-order stencil of K pairs at one point (reference rule near the array
 // ends): taps read from memory at `stride`, K known only at run time.  Used to
@@ -561,26 +589,25 @@ __device__ __forceinline__ void dz_quads(const T *tile, int zr, int xq, const T 
     }
 }
 
-template <typename T, int MODE, int TX, int TZ, int RZ, bool FW>
+template <typename T, int MODE, int W, int RZ, bool FW>
 __device__ __forceinline__ void block_dz(const T *tile, int zr, int xq, const CoefSet<T> &cs, const T (&cu)[NCOEF],
                                          const T (&c2)[2][NCOEF][2], bool zedge, int gz, int nzp, int order, T d,
                                          const Rcp<T> &r, T (&out)[RZ][4])
 {
-    using G = Geo2D<T, TX, TZ, RZ>;
     int K[RZ];
 #pragma unroll
     for (int q = 0; q < RZ; q++) K[q] = FW ? kfw(gz + q, nzp, order) : kbw(gz + q, nzp, order);
     if constexpr (MODE == MODE_FAST && std::is_same<T, float>::value) {
-        dz_stream_f32<G::W, RZ, FW>(tile, zr, xq + GUARD, c2, out);
+        dz_stream_f32<W, RZ, FW>(tile, zr, xq + GUARD, c2, out);
         if (zedge) {
 #pragma unroll
             for (int q = 0; q < RZ; q++)
                 if (K[q] != order)
-                    dz_row_edge<G::W, FW>(tile + (zr + q) * G::W + xq + GUARD, cs.cz + K[q] * CROW, K[q], out[q]);
+                    dz_row_edge<W, FW>(tile + (zr + q) * W + xq + GUARD, cs.cz + K[q] * CROW, K[q], out[q]);
         }
     } else {
-        if (zedge) dz_quads<T, MODE, G::W, RZ, FW, true>(tile, zr, xq, cu, cs.cz, K, out);
-        else dz_quads<T, MODE, G::W, RZ, FW, false>(tile, zr, xq, cu, cs.cz, K, out);
+        if (zedge) dz_quads<T, MODE, W, RZ, FW, true>(tile, zr, xq, cu, cs.cz, K, out);
+        else dz_quads<T, MODE, W, RZ, FW, false>(tile, zr, xq, cu, cs.cz, K, out);
 #pragma unroll
         for (int q = 0; q < RZ; q++) div_by4(out[q], d, r);
     }
@@ -820,7 +847,7 @@ __device__ __forceinline__ void a2d_velocity_tile(const Step2DArgs<T> &a, const 
     for (int q = 0; q < RZ; q++) row_dx<T, MODE, TX, TZ, RZ>(sP, zr + q + GUARD, xq, cs, a.cx, true, xe, gx, sh.nxp, a.order, a.dx, a.rdx, d[q]);
     update_field<T, MODE, TX, TZ, RZ, true, false>(F, M, d, d, ps, pt, 1, 1, fl, gx, gz, xq, zr, sh, a, false);
     store_block<T, RZ>(sh.f[A2_VX], o0, pitch, F);
-    block_dz<T, MODE, TX, TZ, RZ, true>(sP, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d);
+    block_dz<T, MODE, G::W, RZ, true>(sP, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d);
     update_field<T, MODE, TX, TZ, RZ, false, true>(F2, M2, d, d, ps, pt, 1, 1, fl, gx, gz, xq, zr, sh, a, false);
     store_block<T, RZ>(sh.f[A2_VZ], o0, pitch, F2);
     if (pml) ps.template store<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[0], sh.psiz[0]);
@@ -846,7 +873,7 @@ __device__ __forceinline__ void a2d_stress_tile(const Step2DArgs<T> &a, const Sh
     if (!tile_ready(bar, err, pml, pf, pt)) return;
 #pragma unroll
     for (int q = 0; q < RZ; q++) row_dx<T, MODE, TX, TZ, RZ>(sVx, zr + q + GUARD, xq, cs, a.cx, false, xe, gx, sh.nxp, a.order, a.dx, a.rdx, d1[q]);
-    block_dz<T, MODE, TX, TZ, RZ, false>(sVz, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
+    block_dz<T, MODE, TX, RZ, false>(sVz, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
     update_field<T, MODE, TX, TZ, RZ, true, true>(F, M, d1, d2, ps, pt, 0, 0, fl, gx, gz, xq, zr, sh, a, false);
     store_block<T, RZ>(sh.f[A2_P], o0, pitch, F);
     if (pml) ps.template store<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[1], sh.psiz[1]);
@@ -858,7 +885,8 @@ __device__ __forceinline__ void a2d_stress_tile(const Step2DArgs<T> &a, const Sh
 //   Vz += dt*Rz*Dx-Sxz [x psi1]      ; Vz += dt*Rz*Dz+Szz [z stag psi1]
 // Adjoint (lib/waves.cpp:1738-1913): Sxx -> L2M*Sxx + L*Szz, Sxz -> M*Sxz,
 // Szz -> L*Sxx + L2M*Szz (formed in shared memory after the TMA loads).
-template <typename T, int MODE, int TX, int TZ, int RZ>
+// WZZ: row length of the Szz tile (no x halo in the forward step)
+template <typename T, int MODE, int TX, int TZ, int RZ, int WZZ>
 __device__ __forceinline__ void e2d_velocity_tile(const Step2DArgs<T> &a, const Shot2D<T> &sh, const Tile2D &tl,
                                                   const T *sXX, const T *sZZ, const T *sXZ, const CoefSet<T> &cs,
                                                   PmlTile<T, TX, TZ> &pt, uint64_t *bar, int *err)
@@ -877,7 +905,7 @@ __device__ __forceinline__ void e2d_velocity_tile(const Step2DArgs<T> &a, const 
     if (pml) ps.template load<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[0], sh.psiz[0]);
 #pragma unroll
     for (int q = 0; q < RZ; q++) row_dx<T, MODE, TX, TZ, RZ>(sXX, zr + q + GUARD, xq, cs, a.cx, true, xe, gx, sh.nxp, a.order, a.dx, a.rdx, d1[q]);
-    block_dz<T, MODE, TX, TZ, RZ, false>(sXZ, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
+    block_dz<T, MODE, G::W, RZ, false>(sXZ, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
     update_field<T, MODE, TX, TZ, RZ, true, true>(F, M, d1, d2, ps, pt, 1, 0, fl, gx, gz, xq, zr, sh, a, false);
     PsiBlock<T, RZ> p2;
     if (pml) p2.template load<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[1], sh.psiz[1]);
@@ -885,7 +913,7 @@ __device__ __forceinline__ void e2d_velocity_tile(const Step2DArgs<T> &a, const 
     if (pml) ps.template store<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[0], sh.psiz[0]);
 #pragma unroll
     for (int q = 0; q < RZ; q++) row_dx<T, MODE, TX, TZ, RZ>(sXZ, zr + q + GUARD, xq, cs, a.cx, false, xe, gx, sh.nxp, a.order, a.dx, a.rdx, d1[q]);
-    block_dz<T, MODE, TX, TZ, RZ, true>(sZZ, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
+    block_dz<T, MODE, WZZ, RZ, true>(sZZ, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
     update_field<T, MODE, TX, TZ, RZ, true, true>(F2, M2, d1, d2, p2, pt, 0, 1, fl, gx, gz, xq, zr, sh, a, false);
     store_block<T, RZ>(sh.f[E2_VZ], o0, pitch, F2);
     if (pml) p2.template store<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[1], sh.psiz[1]);
@@ -980,7 +1008,7 @@ __device__ __forceinline__ void e2d_stress_tile(const Step2DArgs<T> &a, const Sh
         if (pml) ps.template load<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[2], sh.psiz[2]);
 #pragma unroll
         for (int q = 0; q < RZ; q++) row_dx<T, MODE, TX, TZ, RZ>(sVx, zr + q + GUARD, xq, cs, a.cx, false, xe, gx, sh.nxp, a.order, a.dx, a.rdx, d1[q]);
-        block_dz<T, MODE, TX, TZ, RZ, false>(sVz, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
+        block_dz<T, MODE, G::W, RZ, false>(sVz, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
         update_normal<T, MODE, TX, TZ, RZ, ADJ>(sxx, szz, l, l2m, d1, d2, ps, pt, fl, gx, gz, xq, zr, sh, a);
     }
     {
@@ -997,7 +1025,7 @@ __device__ __forceinline__ void e2d_stress_tile(const Step2DArgs<T> &a, const Sh
         if (pml) ps.template store<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[2], sh.psiz[2]);
 #pragma unroll
         for (int q = 0; q < RZ; q++) row_dx<T, MODE, TX, TZ, RZ>(sVz, zr + q + GUARD, xq, cs, a.cx, true, xe, gx, sh.nxp, a.order, a.dx, a.rdx, d1[q]);
-        block_dz<T, MODE, TX, TZ, RZ, true>(sVx, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
+        block_dz<T, MODE, G::W, RZ, true>(sVx, zr, xq, cs, a.cz, a.cz2, ze, gz, sh.nzp, a.order, a.dz, a.rdz, d2);
         update_field<T, MODE, TX, TZ, RZ, true, true>(F, M, d1, d2, p2, pt, 1, 1, fl, gx, gz, xq, zr, sh, a, ADJ);
         store_block<T, RZ>(sh.f[E2_SXZ], o0, pitch, F);
         if (pml) p2.template store<true, true>(sh, a.lpml, fl, gx, gz, sh.psix[3], sh.psiz[3]);
@@ -1005,21 +1033,29 @@ __device__ __forceinline__ void e2d_stress_tile(const Step2DArgs<T> &a, const Sh
 }
 
 // ------------------------------------------------------------------ kernels
+template <typename T, int TX, int TZ> using SmemA2V = Smem2D<T, TX, TZ, halo_2d(PHYS_A2D, A2_P, false)>;
+template <typename T, int TX, int TZ>
+using SmemA2S = Smem2D<T, TX, TZ, halo_2d(PHYS_A2D, A2_VX, false), halo_2d(PHYS_A2D, A2_VZ, false)>;
+template <typename T, int TX, int TZ, bool ADJ>
+using SmemE2V = Smem2D<T, TX, TZ, halo_2d(PHYS_E2D, E2_SXX, ADJ), halo_2d(PHYS_E2D, E2_SZZ, ADJ), halo_2d(PHYS_E2D, E2_SXZ, ADJ)>;
+template <typename T, int TX, int TZ>
+using SmemE2S = Smem2D<T, TX, TZ, halo_2d(PHYS_E2D, E2_VX, false), halo_2d(PHYS_E2D, E2_VZ, false)>;
 
 template <typename T, int MODE, int TX, int TZ, int RZ, int MINB>
 __global__ void __launch_bounds__(Geo2D<T, TX, TZ, RZ>::NT, MINB)
 a2d_velocity(Step2DArgs<T> a, const CoefSet<T> *coefs, const CUtensorMap *maps, int *err)
 {
-    using S = Smem2D<T, TX, TZ, RZ>;
+    using G = Geo2D<T, TX, TZ, RZ>;
+    using S = SmemA2V<T, TX, TZ>;
     extern __shared__ __align__(128) unsigned char sm[];
-    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::coef_off(1));
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off(1));
-    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off(1));
-    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off(1));
+    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::off(S::nfield()));
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off());
+    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off());
+    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off());
     const Tile2D tl = a.tiles[blockIdx.x];
-    const int which[1] = {tl.shot * NMAP + A2_P};
-    tile_prologue<T, TX, TZ, RZ>(sm, bar, maps, which, 1, tl, sh, a.shots, cs, coefs);
-    const T *sP = reinterpret_cast<const T *>(sm);
+    const int field[] = {A2_P};
+    tile_prologue<S, T, G::NT>(sm, bar, maps, field, tl, sh, a.shots, cs, coefs);
+    const T *sP = S::tile(sm, 0);
     a2d_velocity_tile<T, MODE, TX, TZ, RZ>(a, sh, tl, sP, cs, pt, err, bar);
 }
 
@@ -1028,16 +1064,16 @@ __global__ void __launch_bounds__(Geo2D<T, TX, TZ, RZ>::NT, MINB)
 a2d_stress(Step2DArgs<T> a, const CoefSet<T> *coefs, const CUtensorMap *maps, int *err)
 {
     using G = Geo2D<T, TX, TZ, RZ>;
-    using S = Smem2D<T, TX, TZ, RZ>;
+    using S = SmemA2S<T, TX, TZ>;
     extern __shared__ __align__(128) unsigned char sm[];
-    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::coef_off(2));
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off(2));
-    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off(2));
-    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off(2));
+    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::off(S::nfield()));
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off());
+    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off());
+    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off());
     const Tile2D tl = a.tiles[blockIdx.x];
-    const int which[2] = {tl.shot * NMAP + A2_VX, tl.shot * NMAP + A2_VZ};
-    tile_prologue<T, TX, TZ, RZ>(sm, bar, maps, which, 2, tl, sh, a.shots, cs, coefs);
-    const T *sVx = reinterpret_cast<const T *>(sm), *sVz = reinterpret_cast<const T *>(sm + G::TILE_STRIDE);
+    const int field[] = {A2_VX, A2_VZ};
+    tile_prologue<S, T, G::NT>(sm, bar, maps, field, tl, sh, a.shots, cs, coefs);
+    const T *sVx = S::tile(sm, 0), *sVz = S::tile(sm, 1);
     a2d_stress_tile<T, MODE, TX, TZ, RZ>(a, sh, tl, sVx, sVz, cs, pt, err, bar);
 }
 
@@ -1064,17 +1100,17 @@ __global__ void __launch_bounds__(Geo2D<T, TX, TZ, RZ>::NT, MINB)
 e2d_velocity(Step2DArgs<T> a, const CoefSet<T> *coefs, const CUtensorMap *maps, int *err)
 {
     using G = Geo2D<T, TX, TZ, RZ>;
-    using S = Smem2D<T, TX, TZ, RZ>;
+    using S = SmemE2V<T, TX, TZ, ADJ>;
     extern __shared__ __align__(128) unsigned char sm[];
-    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::coef_off(3));
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off(3));
-    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off(3));
-    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off(3));
+    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::off(S::nfield()));
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off());
+    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off());
+    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off());
     const Tile2D tl = a.tiles[blockIdx.x];
-    const int which[3] = {tl.shot * NMAP + E2_SXX, tl.shot * NMAP + E2_SZZ, tl.shot * NMAP + E2_SXZ};
-    tile_prologue<T, TX, TZ, RZ>(sm, bar, maps, which, 3, tl, sh, a.shots, cs, coefs);
-    T *sXX = reinterpret_cast<T *>(sm), *sZZ = reinterpret_cast<T *>(sm + G::TILE_STRIDE),
-      *sXZ = reinterpret_cast<T *>(sm + 2 * G::TILE_STRIDE);
+    const int field[] = {E2_SXX, E2_SZZ, E2_SXZ};
+    tile_prologue<S, T, G::NT>(sm, bar, maps, field, tl, sh, a.shots, cs, coefs);
+    T *sXX = S::tile(sm, 0), *sZZ = S::tile(sm, 1),
+      *sXZ = S::tile(sm, 2);
     uint64_t *wbar = bar;
     if (ADJ) {
         // every thread reaches the same barriers whether or not the wait succeeded
@@ -1084,7 +1120,7 @@ e2d_velocity(Step2DArgs<T> a, const CoefSet<T> *coefs, const CUtensorMap *maps, 
         __syncthreads();
         wbar = nullptr;
     }
-    e2d_velocity_tile<T, MODE, TX, TZ, RZ>(a, sh, tl, sXX, sZZ, sXZ, cs, pt, wbar, err);
+    e2d_velocity_tile<T, MODE, TX, TZ, RZ, ADJ ? G::W : TX>(a, sh, tl, sXX, sZZ, sXZ, cs, pt, wbar, err);
 }
 
 template <typename T, int MODE, int TX, int TZ, int RZ, int MINB, bool ADJ>
@@ -1092,16 +1128,16 @@ __global__ void __launch_bounds__(Geo2D<T, TX, TZ, RZ>::NT, MINB)
 e2d_stress(Step2DArgs<T> a, const CoefSet<T> *coefs, const CUtensorMap *maps, int *err)
 {
     using G = Geo2D<T, TX, TZ, RZ>;
-    using S = Smem2D<T, TX, TZ, RZ>;
+    using S = SmemE2S<T, TX, TZ>;
     extern __shared__ __align__(128) unsigned char sm[];
-    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::coef_off(2));
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off(2));
-    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off(2));
-    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off(2));
+    CoefSet<T> &cs = *reinterpret_cast<CoefSet<T> *>(sm + S::off(S::nfield()));
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar_off());
+    PmlTile<T, TX, TZ> &pt = *reinterpret_cast<PmlTile<T, TX, TZ> *>(sm + S::pml_off());
+    Shot2D<T> &sh = *reinterpret_cast<Shot2D<T> *>(sm + S::shot_off());
     const Tile2D tl = a.tiles[blockIdx.x];
-    const int which[2] = {tl.shot * NMAP + E2_VX, tl.shot * NMAP + E2_VZ};
-    tile_prologue<T, TX, TZ, RZ>(sm, bar, maps, which, 2, tl, sh, a.shots, cs, coefs);
-    const T *sVx = reinterpret_cast<const T *>(sm), *sVz = reinterpret_cast<const T *>(sm + G::TILE_STRIDE);
+    const int field[] = {E2_VX, E2_VZ};
+    tile_prologue<S, T, G::NT>(sm, bar, maps, field, tl, sh, a.shots, cs, coefs);
+    const T *sVx = S::tile(sm, 0), *sVz = S::tile(sm, 1);
     e2d_stress_tile<T, MODE, TX, TZ, RZ, ADJ>(a, sh, tl, sVx, sVz, cs, pt, bar, err);
 }
 
@@ -1298,33 +1334,32 @@ cudaError_t launch_2d_cfg(int physics, int half, int flags, const Step2DArgs<T> 
                           const CUtensorMap *maps, int *err, int grid, cudaStream_t st)
 {
     using G = Geo2D<T, TX, TZ, RZ>;
-    using S = Smem2D<T, TX, TZ, RZ>;
     const bool adj = (flags & LAUNCH_ADJ) != 0;
     if (physics == PHYS_A2D) {
         if (half == 0) {
-            static const cudaError_t e = set_smem(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, S::bytes(1));
+            static const cudaError_t e = set_smem(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, SmemA2V<T, TX, TZ>::bytes());
             if (e != cudaSuccess) return e;
-            return launch_pdl(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, S::bytes(1), st, a, coefs, maps, err);
+            return launch_pdl(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, SmemA2V<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
         } else {
-            static const cudaError_t e = set_smem(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, S::bytes(2));
+            static const cudaError_t e = set_smem(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, SmemA2S<T, TX, TZ>::bytes());
             if (e != cudaSuccess) return e;
-            return launch_pdl(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
+            return launch_pdl(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, SmemA2S<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
         }
     } else {
         if (half == 0) {
-            static const cudaError_t e0 = set_smem(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, S::bytes(3));
-            static const cudaError_t e1 = set_smem(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, S::bytes(3));
+            static const cudaError_t e0 = set_smem(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, SmemE2V<T, TX, TZ, false>::bytes());
+            static const cudaError_t e1 = set_smem(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, SmemE2V<T, TX, TZ, true>::bytes());
             if (e0 != cudaSuccess) return e0;
             if (e1 != cudaSuccess) return e1;
-            if (adj) return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, S::bytes(3), st, a, coefs, maps, err);
-            else return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, S::bytes(3), st, a, coefs, maps, err);
+            if (adj) return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, SmemE2V<T, TX, TZ, true>::bytes(), st, a, coefs, maps, err);
+            else return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, SmemE2V<T, TX, TZ, false>::bytes(), st, a, coefs, maps, err);
         } else {
-            static const cudaError_t e0 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, S::bytes(2));
-            static const cudaError_t e1 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, S::bytes(2));
+            static const cudaError_t e0 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, SmemE2S<T, TX, TZ>::bytes());
+            static const cudaError_t e1 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, SmemE2S<T, TX, TZ>::bytes());
             if (e0 != cudaSuccess) return e0;
             if (e1 != cudaSuccess) return e1;
-            if (adj) return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
-            else return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, S::bytes(2), st, a, coefs, maps, err);
+            if (adj) return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, SmemE2S<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
+            else return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, SmemE2S<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
         }
     }
 }

@@ -561,7 +561,9 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
         const ShotLayout &L = shots[i];
         for (int k = 0; k < nfields(phys); k++) {
             CUtensorMap *m = reinterpret_cast<CUtensorMap *>(meta.data() + m_maps) + (size_t)i * NMAP2D + k;
-            if (!encode_field_map(m, A + L.f[k], prec, L.pitch, L.rows, ts.tx + 2 * GUARD, ts.tz + 2 * GUARD)) {
+            const int halo = halo_2d(phys, k, adjoint_steps);
+            if (!encode_field_map(m, A + L.f[k], prec, L.pitch, L.rows, ts.tx + (halo & HALO_X ? 2 * GUARD : 0),
+                                  ts.tz + (halo & HALO_Z ? 2 * GUARD : 0))) {
                 set_error("cuTensorMapEncodeTiled failed for shot %d field %d", i, k);
                 return RSGPU_ERR_CUDA;
             }

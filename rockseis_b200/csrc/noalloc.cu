@@ -222,8 +222,9 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     std::memcpy(at(o_tiles), tiles.data(), tiles.size() * sizeof(Tile2D));
     std::memcpy(at(o_coef), coefs.data(), coefs.size());
     for (int k = 0; k < 3; k++)
-        if (!encode_field_map_host(at(o_maps) + k * sizeof(CUtensorMap), S + o_f[k], prec, pitch, rows, ts.tx + 2 * GUARD,
-                                   ts.tz + 2 * GUARD)) {
+        if (const int halo = halo_2d(PHYS_A2D, k, false);
+            !encode_field_map_host(at(o_maps) + k * sizeof(CUtensorMap), S + o_f[k], prec, pitch, rows,
+                                   ts.tx + (halo & HALO_X ? 2 * GUARD : 0), ts.tz + (halo & HALO_Z ? 2 * GUARD : 0))) {
             set_error("cuTensorMapEncodeTiled failed");
             return RSGPU_ERR_CUDA;
         }

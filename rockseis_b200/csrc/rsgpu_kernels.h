@@ -22,6 +22,15 @@ enum { LAUNCH_ADJ = 1 };
 cudaError_t launch_step_2d(int prec, int cfg, int physics, int half, int flags, const void *args, const void *coefs,
                            const void *maps, int *err, int grid, cudaStream_t st);
 constexpr int NMAP2D = 5;
+// Axes along which a tile kernel reads field `f`'s neighbours (slots of rsgpu_internal.h),
+// i.e. the halo of its tensor map's box.  The adjoint velocity step forms work arrays from
+// Sxx and Szz over both halos.
+enum { HALO_X = 1, HALO_Z = 2 };
+constexpr int halo_2d(int phys, int f, bool adj)
+{
+    if (phys == PHYS_A2D) return f == 1 ? HALO_X : f == 2 ? HALO_Z : HALO_X | HALO_Z;   // Vx, Vz, P
+    return f == 2 && !adj ? HALO_X : f == 3 && !adj ? HALO_Z : HALO_X | HALO_Z;         // Sxx, Szz, the others
+}
 // Kernel instantiation table (generated at build time): variant "f32x" (exact),
 // "f32f" (fast), "f64"; nullptr if the tile config is not built for the variant.
 using Launch2DFn = cudaError_t (*)(int physics, int half, int flags, const void *args, const void *coefs,
