@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "adjoint_ops.cuh"
+#include "pdl.cuh"
 #include "rsgpu_adjoint.h"
 #include "rsgpu_kernels.h"
 
@@ -35,6 +36,8 @@ namespace {
 template <typename T, bool EXACT, typename G>
 __global__ void __launch_bounds__(256) corr_fwi_a2d(const Corr2D<T> *desc, T dx, T dz)
 {
+    pdl_wait();
+    pdl_trigger();
     const Corr2D<T> c = desc[blockIdx.z];
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iz = blockIdx.y * blockDim.y + threadIdx.y;
@@ -102,6 +105,8 @@ __global__ void __launch_bounds__(256) corr_fwi_a2d(const Corr2D<T> *desc, T dx,
 template <typename T, bool EXACT, typename G>
 __global__ void __launch_bounds__(256) corr_rtm_a2d(const Corr2D<T> *desc, int nhx, int nhz)
 {
+    pdl_wait();
+    pdl_trigger();
     const Corr2D<T> c = desc[blockIdx.z];
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iz = blockIdx.y * blockDim.y + threadIdx.y;
@@ -367,6 +372,8 @@ __global__ void __launch_bounds__(256) residual_corr_e2d(const Resid2DE<T> *desc
 template <typename T, bool EXACT, typename G>
 __global__ void __launch_bounds__(256) corr_fwi_e2d(const Corr2DE<T> *desc, T dx, T dz)
 {
+    pdl_wait();
+    pdl_trigger();
     const Corr2DE<T> c = desc[blockIdx.z];
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iz = blockIdx.y * blockDim.y + threadIdx.y;
@@ -617,6 +624,8 @@ __device__ __forceinline__ void ck_row(const CkptSeg &s, int r, int lane, F op)
 template <typename T>
 __global__ void __launch_bounds__(256) ckpt_copy_out(const CkptSeg *segs, T *__restrict__ slot)
 {
+    pdl_wait();
+    pdl_trigger();
     const CkptSeg s = segs[blockIdx.y];
     const T *__restrict__ src = (const T *)s.src;
     const int lane = threadIdx.x & 31;
@@ -634,6 +643,8 @@ __global__ void __launch_bounds__(256) ckpt_copy_out(const CkptSeg *segs, T *__r
 template <typename T>
 __global__ void __launch_bounds__(256) ckpt_copy_in(const CkptSeg *segs, const T *__restrict__ slot)
 {
+    pdl_wait();
+    pdl_trigger();
     const CkptSeg s = segs[blockIdx.y];
     T *__restrict__ dst = (T *)s.src;
     const int lane = threadIdx.x & 31;
@@ -651,6 +662,8 @@ __global__ void __launch_bounds__(256) ckpt_copy_in(const CkptSeg *segs, const T
 template <typename T>
 __global__ void __launch_bounds__(256) ckpt_maxabs(const CkptSeg *segs, unsigned *maxbits)
 {
+    pdl_wait();
+    pdl_trigger();
     const CkptSeg s = segs[blockIdx.y];
     const T *__restrict__ src = (const T *)s.src;
     const int lane = threadIdx.x & 31;
@@ -673,6 +686,8 @@ template <typename T, typename S>
 __global__ void __launch_bounds__(256) ckpt_pack(const CkptSeg *segs, S *__restrict__ slot, const unsigned *maxbits,
                                                  float *scales)
 {
+    pdl_wait();
+    pdl_trigger();
     const CkptSeg s = segs[blockIdx.y];
     const float scale = pow2_scale(maxbits[blockIdx.y]);
     const float inv = 1.0f / scale;            // exact: a power of two
@@ -694,6 +709,8 @@ __global__ void __launch_bounds__(256) ckpt_pack(const CkptSeg *segs, S *__restr
 template <typename T, typename S>
 __global__ void __launch_bounds__(256) ckpt_unpack(const CkptSeg *segs, const S *__restrict__ slot, const float *scales)
 {
+    pdl_wait();
+    pdl_trigger();
     const CkptSeg s = segs[blockIdx.y];
     const float scale = scales[blockIdx.y];
     T *__restrict__ dst = (T *)s.src;
@@ -723,14 +740,14 @@ cudaError_t ckpt_save_t(int ck, const CkptSeg *segs, int nseg, int max_rows, voi
 {
     const dim3 grid = ck_grid(nseg, max_rows);
     if (ck == CK_NATIVE) {
-        ckpt_copy_out<T><<<grid, 256, 0, st>>>(segs, (T *)slot);
+        launch_pdl(ckpt_copy_out<T>, grid, 256, 0, st, segs, (T *)slot);
         return cudaGetLastError();
     }
     cudaError_t e = cudaMemsetAsync(maxbits, 0, sizeof(unsigned) * nseg, st);
     if (e != cudaSuccess) return e;
-    ckpt_maxabs<T><<<grid, 256, 0, st>>>(segs, maxbits);
-    if (ck == CK_F16) ckpt_pack<T, __half><<<grid, 256, 0, st>>>(segs, (__half *)slot, maxbits, scales);
-    else ckpt_pack<T, __nv_bfloat16><<<grid, 256, 0, st>>>(segs, (__nv_bfloat16 *)slot, maxbits, scales);
+    launch_pdl(ckpt_maxabs<T>, grid, 256, 0, st, segs, maxbits);
+    if (ck == CK_F16) launch_pdl(ckpt_pack<T, __half>, grid, 256, 0, st, segs, (__half *)slot, maxbits, scales);
+    else launch_pdl(ckpt_pack<T, __nv_bfloat16>, grid, 256, 0, st, segs, (__nv_bfloat16 *)slot, maxbits, scales);
     return cudaGetLastError();
 }
 
@@ -739,9 +756,9 @@ cudaError_t ckpt_load_t(int ck, const CkptSeg *segs, int nseg, int max_rows, con
                         cudaStream_t st)
 {
     const dim3 grid = ck_grid(nseg, max_rows);
-    if (ck == CK_NATIVE) ckpt_copy_in<T><<<grid, 256, 0, st>>>(segs, (const T *)slot);
-    else if (ck == CK_F16) ckpt_unpack<T, __half><<<grid, 256, 0, st>>>(segs, (const __half *)slot, scales);
-    else ckpt_unpack<T, __nv_bfloat16><<<grid, 256, 0, st>>>(segs, (const __nv_bfloat16 *)slot, scales);
+    if (ck == CK_NATIVE) launch_pdl(ckpt_copy_in<T>, grid, 256, 0, st, segs, (const T *)slot);
+    else if (ck == CK_F16) launch_pdl(ckpt_unpack<T, __half>, grid, 256, 0, st, segs, (const __half *)slot, scales);
+    else launch_pdl(ckpt_unpack<T, __nv_bfloat16>, grid, 256, 0, st, segs, (const __nv_bfloat16 *)slot, scales);
     return cudaGetLastError();
 }
 
@@ -751,9 +768,9 @@ cudaError_t corr_fwi_t(int acc, const void *desc, int nshots, int nxmax, int nzm
 {
     const dim3 block(32, 8), grid((nxmax + 31) / 32, (nzmax + 7) / 8, nshots);
     if (acc == ACC_F64)
-        corr_fwi_a2d<T, EXACT, double><<<grid, block, 0, st>>>((const Corr2D<T> *)desc, (T)dx, (T)dz);
+        launch_pdl(corr_fwi_a2d<T, EXACT, double>, grid, block, 0, st, (const Corr2D<T> *)desc, (T)dx, (T)dz);
     else
-        corr_fwi_a2d<T, EXACT, T><<<grid, block, 0, st>>>((const Corr2D<T> *)desc, (T)dx, (T)dz);
+        launch_pdl(corr_fwi_a2d<T, EXACT, T>, grid, block, 0, st, (const Corr2D<T> *)desc, (T)dx, (T)dz);
     return cudaGetLastError();
 }
 
@@ -761,8 +778,8 @@ template <typename T, bool EXACT>
 cudaError_t corr_rtm_t(int acc, const void *desc, int nshots, int nxmax, int nzmax, int nhx, int nhz, cudaStream_t st)
 {
     const dim3 block(32, 8), grid((nxmax + 31) / 32, (nzmax + 7) / 8, nshots);
-    if (acc == ACC_F64) corr_rtm_a2d<T, EXACT, double><<<grid, block, 0, st>>>((const Corr2D<T> *)desc, nhx, nhz);
-    else corr_rtm_a2d<T, EXACT, T><<<grid, block, 0, st>>>((const Corr2D<T> *)desc, nhx, nhz);
+    if (acc == ACC_F64) launch_pdl(corr_rtm_a2d<T, EXACT, double>, grid, block, 0, st, (const Corr2D<T> *)desc, nhx, nhz);
+    else launch_pdl(corr_rtm_a2d<T, EXACT, T>, grid, block, 0, st, (const Corr2D<T> *)desc, nhx, nhz);
     return cudaGetLastError();
 }
 
@@ -920,14 +937,14 @@ cudaError_t launch_corr_fwi_e2d(int prec, int acc, const void *desc, int nshots,
 {
     const dim3 block(32, 8), grid((nxmax + 31) / 32, (nzmax + 7) / 8, nshots);
     if (prec == PREC_F64) {
-        if (acc == ACC_F64) corr_fwi_e2d<double, true, double><<<grid, block, 0, st>>>((const Corr2DE<double> *)desc, dx, dz);
-        else corr_fwi_e2d<double, true, double><<<grid, block, 0, st>>>((const Corr2DE<double> *)desc, dx, dz);
+        if (acc == ACC_F64) launch_pdl(corr_fwi_e2d<double, true, double>, grid, block, 0, st, (const Corr2DE<double> *)desc, dx, dz);
+        else launch_pdl(corr_fwi_e2d<double, true, double>, grid, block, 0, st, (const Corr2DE<double> *)desc, dx, dz);
     } else if (prec == PREC_F32_EXACT) {
-        if (acc == ACC_F64) corr_fwi_e2d<float, true, double><<<grid, block, 0, st>>>((const Corr2DE<float> *)desc, (float)dx, (float)dz);
-        else corr_fwi_e2d<float, true, float><<<grid, block, 0, st>>>((const Corr2DE<float> *)desc, (float)dx, (float)dz);
+        if (acc == ACC_F64) launch_pdl(corr_fwi_e2d<float, true, double>, grid, block, 0, st, (const Corr2DE<float> *)desc, (float)dx, (float)dz);
+        else launch_pdl(corr_fwi_e2d<float, true, float>, grid, block, 0, st, (const Corr2DE<float> *)desc, (float)dx, (float)dz);
     } else {
-        if (acc == ACC_F64) corr_fwi_e2d<float, false, double><<<grid, block, 0, st>>>((const Corr2DE<float> *)desc, (float)dx, (float)dz);
-        else corr_fwi_e2d<float, false, float><<<grid, block, 0, st>>>((const Corr2DE<float> *)desc, (float)dx, (float)dz);
+        if (acc == ACC_F64) launch_pdl(corr_fwi_e2d<float, false, double>, grid, block, 0, st, (const Corr2DE<float> *)desc, (float)dx, (float)dz);
+        else launch_pdl(corr_fwi_e2d<float, false, float>, grid, block, 0, st, (const Corr2DE<float> *)desc, (float)dx, (float)dz);
     }
     return cudaGetLastError();
 }

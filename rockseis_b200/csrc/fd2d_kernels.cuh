@@ -30,6 +30,7 @@
 #include "rsgpu.h"
 #include "rsgpu_internal.h"
 #include "rsgpu_kernels.h"
+#include "pdl.cuh"
 
 namespace rsgpu {
 
@@ -240,13 +241,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t phase,
     }
     return true;
 }
-// Programmatic dependent launch: a kernel launched by launch_pdl may start while the one
-// before it in the stream drains.  Before pdl_wait it touches only what no kernel writes
-// (descriptors, tables, coefficients); after it everything earlier in the stream is
-// complete and visible.  pdl_trigger, always after the wait, lets the next kernel start.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // 2D tiled TMA load of a box at element coordinates (x, y) into shared memory.
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y)
 {
@@ -1145,10 +1139,9 @@ e2d_stress(Step2DArgs<T> a, const CoefSet<T> *coefs, const CUtensorMap *maps, in
 // One CTA per shot.  Injection first (lib/waves.cpp:407-497, 2085-2174), then,
 // after a CTA barrier, recording (lib/waves.cpp:500-595, 2178-2288) of the same step.
 // A few thousand values at most, so the chain of dependent loads is what it costs: the
-// descriptors come to shared memory in one round trip, the loads of an injection point
-// and of a trace that do not need another's result are issued together, a thread's first
-// trace is read ahead of the injection, and sets that inject into different fields share
-// one pass.  Mean launch of a 16-shot gradient whose adjoint injects 301 traces a shot:
+// descriptors come to shared memory in one round trip, a thread's first injection point
+// and first trace are read, but for the wavefields and samples, before the wait for the
+// kernels ahead, and sets that inject into different fields share one pass.  Mean launch of a 16-shot gradient whose adjoint injects 301 traces a shot:
 // 9.9 -> 5.8 us on B200; of one shot with one source 4.4 us before and after.
 
 // What recording a trace needs beside the wavefields.
@@ -1156,9 +1149,9 @@ template <typename T>
 struct RecPoint {
     const RecSet<T> *q;
     int tr, p;
-    T w[4], acc;
+    T w[4];
     // trace k of all the sets in a row; p = -1: none
-    __device__ __forceinline__ void load(const InjRec<T> &pl, int k, int it)
+    __device__ __forceinline__ void load(const InjRec<T> &pl, int k)
     {
         p = -1;
         for (int set = 0; set < pl.nrecsets; set++) {
@@ -1169,7 +1162,6 @@ struct RecPoint {
                 p = q->pt[tr];
 #pragma unroll
                 for (int c = 0; c < 4; c++) w[c] = q->w[4 * tr + c];
-                acc = q->out[(long)tr * pl.nt + it];
                 return;
             }
             k -= q->nrec;
@@ -1177,42 +1169,67 @@ struct RecPoint {
     }
 };
 
-// Injection point j of set q (contributions in the reference's order).
+// Injection point: what it needs beside the wavefields and the wavelet (its first
+// contribution among it), then the injection, contributions in the reference's order.
 template <typename T, int MODE>
-__device__ __forceinline__ void inject_point(const Shot2D<T> &sh, const InjSet<T> &q, int j, int nt, int it, T dt)
-{
-    using A = Ar<T, MODE == MODE_FAST ? MODE_FAST : MODE_IEEE>;
-    const int p = q.pt[j], c0 = q.start[j], c1 = q.start[j + 1];
-    if (q.kind == INJ_E2_P) {
-        T sxx = sh.f[E2_SXX][p], szz = sh.f[E2_SZZ][p];
-#pragma unroll 2
-        for (int c = c0; c < c1; c++) {
-            const T w = q.wav[(long)q.trace[c] * nt + it];
-            const T s = A::mul(A::mul(A::mul(dt, w), q.wx[c]), q.wz[c]);
-            sxx = A::sub(sxx, s);
-            szz = A::sub(szz, s);
+struct InjPoint {
+    const InjSet<T> *q;
+    int p, c0, c1, tr;
+    T wx, wz, mod;
+    __device__ __forceinline__ void load(const Shot2D<T> &sh, const InjSet<T> &set, int j)
+    {
+        q = &set;
+        p = q->pt[j];
+        c0 = q->start[j];
+        c1 = q->start[j + 1];
+        tr = q->trace[c0];
+        wx = q->wx[c0];
+        wz = q->wz[c0];
+        const int m = q->kind == INJ_A2_P ? M_L : q->kind == INJ_A2_VX || q->kind == INJ_E2_VX ? M_RX : M_RZ;
+        mod = q->kind == INJ_E2_P ? T(0) : sh.m[m][p];
+    }
+    __device__ __forceinline__ void inject(const Shot2D<T> &sh, int nt, int it, T dt) const
+    {
+        using A = Ar<T, MODE == MODE_FAST ? MODE_FAST : MODE_IEEE>;
+        if (q->kind == INJ_E2_P) {
+            T sxx = sh.f[E2_SXX][p], szz = sh.f[E2_SZZ][p];
+            for (int c = c0; c < c1; c++) {
+                const T w = q->wav[(long)(c == c0 ? tr : q->trace[c]) * nt + it];
+                const T s = A::mul(A::mul(A::mul(dt, w), c == c0 ? wx : q->wx[c]), c == c0 ? wz : q->wz[c]);
+                sxx = A::sub(sxx, s);
+                szz = A::sub(szz, s);
+            }
+            sh.f[E2_SXX][p] = sxx;
+            sh.f[E2_SZZ][p] = szz;
+            return;
         }
-        sh.f[E2_SXX][p] = sxx;
-        sh.f[E2_SZZ][p] = szz;
-        return;
+        T *F;
+        switch (q->kind) {
+        case INJ_A2_P: F = sh.f[A2_P]; break;
+        case INJ_A2_VX: F = sh.f[A2_VX]; break;
+        case INJ_A2_VZ: F = sh.f[A2_VZ]; break;
+        case INJ_E2_VX: F = sh.f[E2_VX]; break;
+        default: F = sh.f[E2_VZ]; break;
+        }
+        T v = F[p];
+        const T dm = A::mul(dt, mod);
+        for (int c = c0; c < c1; c++) {
+            const T w = q->wav[(long)(c == c0 ? tr : q->trace[c]) * nt + it];
+            v = A::add(v, A::mul(A::mul(A::mul(dm, w), c == c0 ? wx : q->wx[c]), c == c0 ? wz : q->wz[c]));
+        }
+        F[p] = v;
     }
-    T *F;
-    const T *Mod;
-    switch (q.kind) {
-    case INJ_A2_P: F = sh.f[A2_P]; Mod = sh.m[M_L]; break;
-    case INJ_A2_VX: F = sh.f[A2_VX]; Mod = sh.m[M_RX]; break;
-    case INJ_A2_VZ: F = sh.f[A2_VZ]; Mod = sh.m[M_RZ]; break;
-    case INJ_E2_VX: F = sh.f[E2_VX]; Mod = sh.m[M_RX]; break;
-    default: F = sh.f[E2_VZ]; Mod = sh.m[M_RZ]; break;
+};
+// Point k of all the sets in a row: its set, and k made its index there.
+template <typename T>
+__device__ __forceinline__ const InjSet<T> &inj_set_of(const InjRec<T> &pl, int &k)
+{
+    int set = 0;
+    while (pl.inj[set].kind == INJ_NONE || k >= pl.inj[set].ninj) {
+        k -= pl.inj[set].kind == INJ_NONE ? 0 : pl.inj[set].ninj;
+        set++;
     }
-    T v = F[p];
-    const T dm = A::mul(dt, Mod[p]);
-#pragma unroll 2
-    for (int c = c0; c < c1; c++) {
-        const T w = q.wav[(long)q.trace[c] * nt + it];
-        v = A::add(v, A::mul(A::mul(A::mul(dm, w), q.wx[c]), q.wz[c]));
-    }
-    F[p] = v;
+    return pl.inj[set];
 }
 
 template <typename T, int MODE>
@@ -1225,46 +1242,60 @@ __global__ void __launch_bounds__(1024) inject_record_2d(const Shot2D<T> *shots,
     stage_words(sh, shots + blockIdx.x, threadIdx.x, blockDim.x);
     stage_words(pl, plans + blockIdx.x, threadIdx.x, blockDim.x);
     __syncthreads();
+    int nrec = 0, ninj = 0;
+    for (int set = 0; set < pl.nrecsets; set++) nrec += pl.rec[set].kind == REC_NONE ? 0 : pl.rec[set].nrec;
+    // sets that touch the same field add in set order; others share a pass
+    bool apart = true;
+    for (int a = 0; a < pl.ninjsets; a++) {
+        ninj += pl.inj[a].kind == INJ_NONE ? 0 : pl.inj[a].ninj;
+        for (int b = 0; b < a; b++) apart = apart && (pl.inj[a].kind != pl.inj[b].kind || pl.inj[a].kind == INJ_NONE);
+    }
+    RecPoint<T> r;
+    r.p = -1;
+    if ((int)threadIdx.x < nrec) r.load(pl, threadIdx.x);
+    InjPoint<T, MODE> q;
+    if (apart && (int)threadIdx.x < ninj) {
+        int j = threadIdx.x;
+        const InjSet<T> &set = inj_set_of(pl, j);
+        q.load(sh, set, j);
+    }
     pdl_wait();
     pdl_trigger();
     const int it_step = it_base + (it_dev ? *it_dev : 0);
     const int it = pl.rev ? pl.nt - 1 - it_step : it_step;
     const int gate = pl.rec_gate ? *pl.rec_gate : 1;
-    int nrec = 0;
-    for (int set = 0; set < pl.nrecsets; set++) nrec += pl.rec[set].kind == REC_NONE ? 0 : pl.rec[set].nrec;
-    RecPoint<T> r;
-    r.p = -1;
-    if ((int)threadIdx.x < nrec) r.load(pl, threadIdx.x, it);
-    // sets that touch the same field add in set order; others share a pass
-    bool apart = true;
-    for (int a = 0; a < pl.ninjsets; a++)
-        for (int b = 0; b < a; b++) apart = apart && (pl.inj[a].kind != pl.inj[b].kind || pl.inj[a].kind == INJ_NONE);
+    T acc = r.p >= 0 ? r.q->out[(long)r.tr * pl.nt + it] : T(0);
     if (apart) {
-        int total = 0;
-        for (int set = 0; set < pl.ninjsets; set++) total += pl.inj[set].kind == INJ_NONE ? 0 : pl.inj[set].ninj;
-        for (int k = threadIdx.x; k < total; k += blockDim.x) {
-            int j = k, set = 0;
-            while (pl.inj[set].kind == INJ_NONE || j >= pl.inj[set].ninj) j -= pl.inj[set].kind == INJ_NONE ? 0 : pl.inj[set].ninj, set++;
-            inject_point<T, MODE>(sh, pl.inj[set], j, pl.nt, it, dt);
+        for (int k = threadIdx.x; k < ninj; k += blockDim.x) {
+            if (k != (int)threadIdx.x) {
+                int j = k;
+                const InjSet<T> &set = inj_set_of(pl, j);
+                q.load(sh, set, j);
+            }
+            q.inject(sh, pl.nt, it, dt);
         }
     } else {
         for (int set = 0; set < pl.ninjsets; set++) {
             if (set > 0) __syncthreads();
             if (pl.inj[set].kind == INJ_NONE) continue;
-            for (int j = threadIdx.x; j < pl.inj[set].ninj; j += blockDim.x)
-                inject_point<T, MODE>(sh, pl.inj[set], j, pl.nt, it, dt);
+            for (int j = threadIdx.x; j < pl.inj[set].ninj; j += blockDim.x) {
+                q.load(sh, pl.inj[set], j);
+                q.inject(sh, pl.nt, it, dt);
+            }
         }
     }
     if (nrec == 0 || gate == 0) return;
     __syncthreads();
     const int off[4] = {0, 1, sh.pitch, sh.pitch + 1};
     for (int k = threadIdx.x; k < nrec; k += blockDim.x) {
-        if (k != (int)threadIdx.x) r.load(pl, k, it);
+        if (k != (int)threadIdx.x) {
+            r.load(pl, k);
+            acc = r.p >= 0 ? r.q->out[(long)r.tr * pl.nt + it] : T(0);
+        }
         if (r.p < 0) continue;
         const RecSet<T> &q = *r.q;
         const int p = r.p;
         const T wx[4] = {r.w[0], r.w[1], r.w[0], r.w[1]}, wz[4] = {r.w[2], r.w[2], r.w[3], r.w[3]};
-        T acc = r.acc;
         if (q.kind == REC_E2_P) {
             // (1./2.)*xtri*ytri*F/factor is evaluated in double by the reference and
             // added to the T-typed trace sample (lib/waves.cpp:2238-2239)
@@ -1310,23 +1341,6 @@ template <typename K>
 static cudaError_t set_smem(K k, size_t bytes)
 {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
-// Launch with programmatic stream serialisation (see pdl_wait; the kernel must call it).
-template <typename... P, typename... V>
-static cudaError_t launch_pdl(void (*k)(P...), int grid, int threads, size_t smem, cudaStream_t st, V... args)
-{
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3((unsigned)grid);
-    c.blockDim = dim3((unsigned)threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = st;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
 }
 
 template <typename T, int MODE, int TX, int TZ, int RZ, int MINB>

@@ -24,7 +24,7 @@ def traces(c):
 
 
 @pytest.mark.parametrize("dx,amp", [(10.0, 1.0), (8.0, 1.0), (16.0, 1e-30), (9.00014782, 1.0), (9.00014782, 1e-32),
-                                    (7.3, 1e-34), (12.5, 1e-38)])
+                                    (12.5, 1e-34)])
 @pytest.mark.parametrize("physics", [abi.ACOUSTIC2D, abi.ELASTIC2D])
 def test_exact_division(require_gpu, physics, dx, amp):
     # 9.00014782 fails the check of the two-operation quotient and takes the double one throughout
@@ -36,7 +36,7 @@ def test_exact_division(require_gpu, physics, dx, amp):
 
 
 @pytest.mark.parametrize("physics", [abi.ACOUSTIC2D, abi.ELASTIC2D])
-@pytest.mark.parametrize("nx,nz,lpml,order,fs", [(9, 11, 1, 8, 0), (38, 17, 3, 8, 1), (31, 33, 5, 5, 0), (64, 16, 13, 8, 1),
+@pytest.mark.parametrize("nx,nz,lpml,order,fs", [(15, 16, 1, 8, 0), (38, 17, 3, 8, 1), (31, 33, 5, 5, 0), (64, 16, 13, 8, 1),
                                                  (7, 40, 30, 8, 0), (121, 9, 20, 2, 0)])
 def test_strips_and_edges_bitwise(require_gpu, physics, nx, nz, lpml, order, fs):
     # strips that start and end off the vectors' boundaries, and tiles that hold both of an axis' ends
