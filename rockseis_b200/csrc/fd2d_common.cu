@@ -25,6 +25,29 @@ cudaError_t launch_injrec_2d(int prec, const void *shots, const void *plans, int
                       it_base, it_dev);
 }
 
+// Contiguous [d][h][w] rows into a pitched, guarded array (w*h*d values).
+template <typename T>
+static __global__ void __launch_bounds__(256) pad_rows(T *dst, int pitch, long long plane, const T *src, int w, int h,
+                                                       long long n)
+{
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        const long long row = k / w;
+        dst[row / h * plane + row % h * pitch + (k - row * w)] = src[k];
+    }
+}
+
+cudaError_t upload_padded(void *dst, int pitch, long long plane, const void *src, int w, int h, int d, int es,
+                          void *staging, cudaStream_t st)
+{
+    const long long n = (long long)w * h * d;
+    cudaError_t e = cudaMemcpyAsync(staging, src, (size_t)n * es, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return e;
+    const int grid = (int)((n + 255) / 256 < 4736 ? (n + 255) / 256 : 4736);   // 148 SMs x 32
+    if (es == 8) pad_rows<<<grid, 256, 0, st>>>((double *)dst, pitch, plane, (const double *)staging, w, h, n);
+    else pad_rows<<<grid, 256, 0, st>>>((float *)dst, pitch, plane, (const float *)staging, w, h, n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_advance(int *it_dev, int by, cudaStream_t st)
 {
     advance_counter<<<1, 32, 0, st>>>(it_dev, by);

@@ -458,56 +458,52 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
         return RSGPU_ERR_NOMEM;
     }
     CU(cudaMemsetAsync(arena, 0, arena_bytes, stream));
-    // the plan tables below go up with synchronous copies, which do not wait for the
-    // plan's non-blocking stream: let the clearing finish first
-    CU(cudaStreamSynchronize(stream));
     char *A = (char *)arena;
 
-    // ---- uploads
-    std::vector<unsigned char> hb;
-    auto upload_vec_real = [&](size_t o, const std::vector<double> &v) -> rsgpu_status {
-        if (v.empty()) return RSGPU_OK;
-        hb.resize(v.size() * es);
+    // ---- uploads: the parameters through a staging buffer (without one: row by row), and
+    // every table of the plan, contiguous in the arena, in one copy
+    const size_t tab0 = io[0].pt;
+    std::vector<unsigned char> tabs(arena_bytes - tab0, 0);
+    auto put_real = [&](size_t o, const std::vector<double> &v) {
         for (size_t k = 0; k < v.size(); k++) {
-            if (es == 8) ((double *)hb.data())[k] = v[k];
-            else ((float *)hb.data())[k] = (float)v[k];
+            if (es == 8) std::memcpy(&tabs[o - tab0 + 8 * k], &v[k], 8);
+            else { const float f = (float)v[k]; std::memcpy(&tabs[o - tab0 + 4 * k], &f, 4); }
         }
-        CU(cudaMemcpy(A + o, hb.data(), hb.size(), cudaMemcpyHostToDevice));
-        return RSGPU_OK;
     };
-    auto upload_vec_int = [&](size_t o, const std::vector<int> &v) -> rsgpu_status {
-        if (v.empty()) return RSGPU_OK;
-        CU(cudaMemcpy(A + o, v.data(), v.size() * 4, cudaMemcpyHostToDevice));
-        return RSGPU_OK;
+    auto put_int = [&](size_t o, const std::vector<int> &v) {
+        if (!v.empty()) std::memcpy(&tabs[o - tab0], v.data(), v.size() * 4);
     };
+    Staging staging(stream);
+    for (int i = 0; i < ns; i++) staging.want((size_t)shots[i].nxp * shots[i].nzp * es);
+    staging.get();
     for (int i = 0; i < ns; i++) {
         const ShotLayout &L = shots[i];
         const size_t org = ((size_t)GUARD * L.pitch + GUARD) * es;
-        for (int k = 0; k < nparams(phys); k++)
-            CU(cudaMemcpy2DAsync(A + L.m[k] + org, (size_t)L.pitch * es, s[i].model[k], (size_t)L.nxp * es,
-                                 (size_t)L.nxp * es, L.nzp, cudaMemcpyHostToDevice, stream));
+        for (int k = 0; k < nparams(phys); k++) {
+            if (staging.p) CU(upload_padded(A + L.m[k] + org, L.pitch, 0, s[i].model[k], L.nxp, L.nzp, 1, es, staging.p, stream));
+            else
+                CU(cudaMemcpy2DAsync(A + L.m[k] + org, (size_t)L.pitch * es, s[i].model[k], (size_t)L.nxp * es,
+                                     (size_t)L.nxp * es, L.nzp, cudaMemcpyHostToDevice, stream));
+        }
         for (int k = 0; k < sets[i].nsrc; k++)
             if (sets[i].src[k].n > 0)
                 CU(cudaMemcpyAsync(A + L.wavk[k], sets[i].src[k].data, (size_t)sets[i].src[k].n * cfg.nt * es,
                                    cudaMemcpyHostToDevice, stream));
         for (int k = 0; k < MAXSETS; k++) {
             const size_t j = (size_t)i * MAXSETS + k;
-            if ((st = upload_vec_int(io[j].pt, inj[j].pt)) != RSGPU_OK) return st;
-            if ((st = upload_vec_int(io[j].start, inj[j].start)) != RSGPU_OK) return st;
-            if ((st = upload_vec_int(io[j].tr, inj[j].tr)) != RSGPU_OK) return st;
-            if ((st = upload_vec_real(io[j].wx, inj[j].wx)) != RSGPU_OK) return st;
-            if ((st = upload_vec_real(io[j].wz, inj[j].wz)) != RSGPU_OK) return st;
-            if ((st = upload_vec_int(ro[j].pt, rec[j].pt)) != RSGPU_OK) return st;
-            if ((st = upload_vec_real(ro[j].w, rec[j].w)) != RSGPU_OK) return st;
-            if ((st = upload_vec_real(ro[j].fac, rec[j].fac)) != RSGPU_OK) return st;
+            put_int(io[j].pt, inj[j].pt);
+            put_int(io[j].start, inj[j].start);
+            put_int(io[j].tr, inj[j].tr);
+            put_real(io[j].wx, inj[j].wx);
+            put_real(io[j].wz, inj[j].wz);
+            put_int(ro[j].pt, rec[j].pt);
+            put_real(ro[j].w, rec[j].w);
+            put_real(ro[j].fac, rec[j].fac);
         }
     }
-    {
-        std::vector<unsigned char> tab((size_t)12 * lp * es);
-        if (c->pml) std::memcpy(tab.data(), c->pml, tab.size());
-        else pml_tables_host(lp, cfg.dt, prec, tab.data());
-        CU(cudaMemcpy(A + o_pml, tab.data(), tab.size(), cudaMemcpyHostToDevice));
-    }
+    if (c->pml) std::memcpy(&tabs[o_pml - tab0], c->pml, (size_t)12 * lp * es);
+    else pml_tables_host(lp, cfg.dt, prec, &tabs[o_pml - tab0]);
+    CU(cudaMemcpyAsync(A + tab0, tabs.data(), tabs.size(), cudaMemcpyHostToDevice, stream));
     d_pml = A + o_pml;
 
     // ---- device metadata: shot descriptors, injection plans, tiles, coefficients, step counter

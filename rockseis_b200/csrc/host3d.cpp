@@ -306,10 +306,18 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
         return RSGPU_OK;
     };
     rsgpu_status st;
+    Staging staging(stream);
+    for (int i = 0; i < ns && !share_params; i++) staging.want((size_t)shots[i].nxp * shots[i].nyp * shots[i].nzp * es);
+    if (!share_params) staging.get();
     for (int i = 0; i < ns; i++) {
         const Layout3D &L = shots[i];
         const ShotSets &e = eff[i];
         for (int k = 0; k < np3() && !share_params; k++) {
+            if (staging.p) {
+                CU(upload_padded(A + L.m[k] + origin_bytes(L), L.pitch, L.plane, s[i].model[k], L.nxp, L.nyp, L.nzp, es,
+                                 staging.p, stream));
+                continue;
+            }
             cudaMemcpy3DParms p = {};
             p.srcPtr = make_cudaPitchedPtr(const_cast<void *>(s[i].model[k]), (size_t)L.nxp * es, L.nxp, L.nyp);
             p.dstPtr = make_cudaPitchedPtr(A + L.m[k] + origin_bytes(L), (size_t)L.pitch * es, L.pitch, L.rows);

@@ -32,6 +32,25 @@ bool encode_field_map_host(void *map, void *base, int prec, int pitch, int rows,
 // stream and by synchronous copies; dev_free releases it in `st`'s order.
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t st);
 void dev_free(void *p, cudaStream_t st);
+// Device staging memory of an upload: as large as the largest array wanted, or null where
+// that much is not free.  Released in its stream's order.
+struct Staging {
+    void *p = nullptr;
+    size_t bytes = 0;
+    cudaStream_t st;
+    explicit Staging(cudaStream_t s) : st(s) {}
+    Staging(const Staging &) = delete;
+    Staging &operator=(const Staging &) = delete;
+    ~Staging() { dev_free(p, st); }
+    void want(size_t b) { bytes = b > bytes ? b : bytes; }
+    void get()
+    {
+        if (dev_alloc(&p, bytes, st) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+};
 // Return the cached blocks of the current device's pool to the driver.
 cudaError_t dev_trim();
 void make_map_host(int dim, int prec, int ntr, const double *coords, const int *n, const double *o, const double *d,

@@ -44,6 +44,12 @@ inline int injrec_threads(size_t most)
 }
 cudaError_t launch_injrec_2d(int prec, const void *shots, const void *plans, int nshots, double dt, int it_base,
                              const int *it_dev, int threads, cudaStream_t st);
+// Upload a contiguous host array [d][h][w] into a pitched device array through `staging`
+// (device memory for the contiguous values), in st's order.  One contiguous copy and a pass
+// on the device: a pitched copy goes row by row from pageable memory, 3 GB/s (B200 host,
+// the four parameters of a 151 x 141 x 131 window 15 ms of a 27 ms call; 14 ms this way).
+cudaError_t upload_padded(void *dst, int pitch, long long plane, const void *src, int w, int h, int d, int es,
+                          void *staging, cudaStream_t st);
 cudaError_t launch_advance(int *it_dev, int by, cudaStream_t st);
 cudaError_t launch_set_counter(int *it_dev, int value, cudaStream_t st);
 cudaError_t launch_wait_for_nothing(int *err, cudaStream_t st);
