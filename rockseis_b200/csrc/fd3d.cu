@@ -10,52 +10,20 @@
 //     from L2-resident neighbours);
 //   - the C-PML memory-variable update and correction of each face pair are fused
 //     into the same pass.
+// Double runs the plain kernels below, float the TMA-staged ones further down.
 // Arithmetic follows the reference operation by operation (MODE_IEEE: separately
 // rounded ops and IEEE division; MODE_FAST: FMA, coefficients pre-divided).  Near
 // the array ends the reference's reduced-order stencils are evaluated by
 // stencil_k (the same rules as in 2D).  One launch covers all tiles of all shots.
 #include <type_traits>
 
-#include "fd2d_kernels.cuh"
-#include "rsgpu_3d.h"
+#include "fd3d_common.cuh"
 
 namespace rsgpu {
 namespace {
 
 static_assert(TX3 >= 16 && TY3 >= 8, "the halo fetch assigns one x-halo column per thread tx < 16 and two y-halo rows "
                                      "per thread ty < 8");
-
-template <typename T>
-__device__ __forceinline__ void load_coefs3(CoefSet3<T> &s, const CoefSet3<T> *g)
-{
-    const T *src = reinterpret_cast<const T *>(g);
-    T *dst = reinterpret_cast<T *>(&s);
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    for (int i = tid; i < (int)(sizeof(CoefSet3<T>) / sizeof(T)); i += blockDim.x * blockDim.y) dst[i] = src[i];
-}
-
-// Staggered derivative with all NCOEF taps around b[7] (fw: b[0] = f[i-7]) or
-// b[8] (bw: b[0] = f[i-8]); in both cases sum_k (b[8+k*s] - b[7-k*s]) c_k.  The
-// coefficients are read from shared memory (one broadcast per tap), which keeps
-// them out of the register file.
-template <typename T, int MODE>
-__device__ __forceinline__ T taps(const T *b, int s, const T *cu, T d, const Rcp<T> &r)
-{
-    using A = Ar<T, MODE>;
-    T acc = A::mul(A::sub(b[8 * s], b[7 * s]), cu[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A::mad(acc, A::sub(b[(8 + k) * s], b[(7 - k) * s]), cu[k]);
-    return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
-}
-template <typename T, int MODE>
-__device__ __forceinline__ T taps_reg(const T (&q)[16], const T *cu, T d, const Rcp<T> &r)
-{
-    using A = Ar<T, MODE>;
-    T acc = A::mul(A::sub(q[8], q[7]), cu[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A::mad(acc, A::sub(q[8 + k], q[7 - k]), cu[k]);
-    return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
-}
 
 // Velocity half-step (lib/waves.cpp:710-851):
 //   Vx += dt*Rx*Dx+P [x C-PML, staggered tables], Vy likewise in y, Vz in z.
@@ -241,7 +209,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 3) a3d_stress(Step3DArgs<T> a, const
 // Source injection then receiver recording of one step, one CTA per shot
 // (lib/waves.cpp:999-1190).
 template <typename T, int MODE>
-__global__ void inject_record_3d(const Shot3D<T> *shots, const InjRec3<T> *plans, T dt, int it)
+__global__ void __launch_bounds__(1024) inject_record_3d(const Shot3D<T> *shots, const InjRec3<T> *plans, T dt, int it)
 {
     using A = Ar<T, MODE == MODE_FAST ? MODE_FAST : MODE_IEEE>;
     const Shot3D<T> &sh = shots[blockIdx.x];
@@ -252,9 +220,10 @@ __global__ void inject_record_3d(const Shot3D<T> *shots, const InjRec3<T> *plans
         const T *Mod = sh.m[pl.kind_inj == INJ3_P ? M3_L : pl.kind_inj == INJ3_VX ? M3_RX : pl.kind_inj == INJ3_VY ? M3_RY : M3_RZ];
         for (int q = threadIdx.x; q < pl.ninj; q += blockDim.x) {
             const long long p = pl.inj_pt[q];
+            const int c0 = pl.inj_start[q], c1 = pl.inj_start[q + 1];
             T v = F[p];
             const T dm = A::mul(dt, Mod[p]);
-            for (int c = pl.inj_start[q]; c < pl.inj_start[q + 1]; c++) {
+            for (int c = c0; c < c1; c++) {
                 const T w = pl.wav[(long long)pl.inj_trace[c] * pl.nt + it];
                 v = A::add(v, A::mul(A::mul(A::mul(A::mul(dm, w), pl.inj_w[3 * c]), pl.inj_w[3 * c + 1]),
                                      pl.inj_w[3 * c + 2]));
@@ -280,48 +249,127 @@ __global__ void inject_record_3d(const Shot3D<T> *shots, const InjRec3<T> *plans
     }
 }
 
-// ---------------------------------------------------------------- fast mode with TMA-staged planes
-// The two half-steps of RSGPU_F32_FAST with every plane tile brought in by TMA
-// (cp.async.bulk.tensor.2d issued by one thread, completion on an mbarrier per
-// stage) two planes ahead of the plane being computed, so the loads in flight do
-// not depend on registers or resident warps.  The z-derivative still comes from the
-// 16-plane register window, refilled by a plain load eight planes ahead.  Same
-// stencils, C-PML and update order as a3d_velocity / a3d_stress.  Every wait is
-// bounded (2 s): on timeout the CTA records RSGPU_ERR_TIMEOUT and stops.
+// ---------------------------------------------------------------- float: TMA-staged planes
+// The float half-steps (both arithmetics).  A block of 32 x 8 threads owns 32 x 16 columns,
+// two y-adjacent ones a thread, and marches up z with every plane tile brought in by TMA
+// (cp.async.bulk.tensor.2d issued by one thread, completion on an mbarrier per stage) two
+// planes ahead of the plane being computed.  What bounds them is instruction issue and the
+// chain of a plane:
+//   - the two columns run as the lanes of paired f32x2 operations in x and z, and share 17
+//     of 32 shared-memory loads in y;
+//   - the z-derivatives come from 16-plane register windows whose refill is part of the
+//     stage (a plain load, even eight planes ahead, holds the warp at the end of the plane
+//     that issued it);
+//   - the C-PML memory of a plane is requested before the wait for its stage, the factors
+//     of the block's columns and rows sit in shared memory;
+//   - reduced-order z stencils take their taps from the window (from global memory they
+//     cost a chunk at an array end as much as its other planes together), and whole blocks
+//     choose between the full and the reduced x/y stencils;
+//   - one barrier a plane serves both the stage's arrival and its reuse.
+// Measured on B200 (60 steps of four windows to 226 x 199 x 221, fast): one column a thread
+// with everything above but the refill and the pairs 90 ms (95 before), with the refill 75,
+// two planes a barrier 72, two columns a thread 65, and in shorter z-chunks 59.
+// Every wait is bounded (2 s): on timeout the CTA records RSGPU_ERR_TIMEOUT and stops.
 constexpr int NSTG_A3 = 3;
+constexpr int HYA = TYA + 16;   // a block's rows with the y halo
 
 struct A3VelStage {
-    float p[HY3][WX3];         // P with its x and y halos
-    float pv[6][TY3][TX3];     // Vx, Vy, Vz, Rx, Ry, Rz
+    float p[HYA][WX3];         // P with its x and y halos
+    float pv[6][TYA][TX3];     // Vx, Vy, Vz, Rx, Ry, Rz
+    float up[TYA][TX3];        // P nine planes up: the windows' refill
 };
 struct A3StrStage {
-    float vx[TY3][WX3];        // Vx, x halo
-    float vy[HY3][TX3];        // Vy, y halo
-    float pl[2][TY3][TX3];     // P, L
+    float vx[TYA][WX3];        // Vx, x halo
+    float vy[HYA][TX3];        // Vy, y halo
+    float pl[2][TYA][TX3];     // P, L
+    float up[TYA][TX3];        // Vz eight planes up: the windows' refill
 };
 static_assert(sizeof(A3VelStage) % 128 == 0 && sizeof(A3StrStage) % 128 == 0, "TMA destinations stay 128-byte aligned");
-static_assert(sizeof(float) * HY3 * WX3 % 128 == 0 && sizeof(float) * TY3 * WX3 % 128 == 0 &&
-              sizeof(float) * HY3 * TX3 % 128 == 0 && sizeof(float) * TY3 * TX3 % 128 == 0, "tile sizes");
+static_assert(sizeof(float) * HYA * WX3 % 128 == 0 && sizeof(float) * TYA * WX3 % 128 == 0 &&
+              sizeof(float) * HYA * TX3 % 128 == 0 && sizeof(float) * TYA * TX3 % 128 == 0, "tile sizes");
+static_assert(TYA == 2 * TY3, "two rows a thread");
 
 template <typename Stage>
 struct A3Smem {
     Stage st[NSTG_A3];
     uint64_t bar[NSTG_A3];
     CoefSet3<float> cs;
+    PmlBlock3<TYA> pml;
 };
 template <typename Stage>
 constexpr size_t a3_smem_bytes() { return sizeof(A3Smem<Stage>) + 128; }   // + alignment slack
 
-// Allocation row of plane iz, padded row iy_alloc (guards included).
-__device__ __forceinline__ int a3_row(const Shot3D<float> &sh, int iz, int iy_alloc)
+// Two derivatives of full order on the lanes of a pair: `at(k)` the operand pair at tap k of
+// the 16 (7 | 8 around the centre).
+template <int MODE, typename F>
+__device__ __forceinline__ float2 taps_lanes(F at, const float (&c2)[NCOEF][2], float d, const Rcp<float> &r)
 {
-    return (GUARD + iz) * sh.rows + iy_alloc;
+    using A2 = Ar2<float, MODE>;
+    const float2 *cc = reinterpret_cast<const float2 *>(c2);
+    float2 acc = A2::mul(A2::sub(at(8), at(7)), cc[0]);
+#pragma unroll
+    for (int k = 1; k < NCOEF; k++) acc = A2::acc(acc, A2::sub(at(8 + k), at(7 - k)), cc[k]);
+    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
+}
+// The y-derivatives of rows y and y + 1 from 17 shared loads; b at the first row's tap 0.
+template <int MODE>
+__device__ __forceinline__ float2 taps_rows(const float *b, int s, const float *c, float d, const Rcp<float> &r)
+{
+    using A = Ar<float, MODE>;
+    float v[17];
+#pragma unroll
+    for (int k = 0; k < 17; k++) v[k] = b[k * s];
+    float2 acc = make_float2(A::mul(A::sub(v[8], v[7]), c[0]), A::mul(A::sub(v[9], v[8]), c[0]));
+#pragma unroll
+    for (int k = 1; k < NCOEF; k++) {
+        acc.x = A::mad(acc.x, A::sub(v[8 + k], v[7 - k]), c[k]);
+        acc.y = A::mad(acc.y, A::sub(v[9 + k], v[8 - k]), c[k]);
+    }
+    return MODE == MODE_FAST ? acc : make_float2(div_by(acc.x, d, r), div_by(acc.y, d, r));
+}
+// Reduced-order z stencils at a plane near an array end (K the same for the block).
+template <int MODE>
+__device__ __forceinline__ float2 taps_lanes_k(const float2 (&q)[16], int K, const float *c, float d, const Rcp<float> &r)
+{
+    using A2 = Ar2<float, MODE>;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < NCOEF; k++)
+        if (k < K) {
+            const float2 dl = A2::sub(q[8 + k], q[7 - k]), ck = make_float2(c[k], c[k]);
+            acc = k == 0 ? A2::mul(dl, ck) : A2::acc(acc, dl, ck);
+        }
+    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
 }
 
-__global__ void __launch_bounds__(TX3 *TY3, 3) a3d_velocity_tma(Step3DArgs<float> a, const CoefSet3<float> *coefs)
+// What a thread's two columns share in both half-steps.
+struct A3Cols {
+    int ix, iy, col, xc, yc[2], Kx, Ky[2];
+    bool in[2], xe, ye;
+    template <bool FW>
+    __device__ __forceinline__ void set(const Shot3D<float> &sh, const Tile3D &tl, int L, int order)
+    {
+        const int tx = threadIdx.x, ty = threadIdx.y;
+        ix = tl.x0 + tx;
+        iy = tl.y0 + 2 * ty;
+        col = iy * sh.pitch + ix;
+        xe = tl.x0 < order || tl.x0 + TX3 > sh.nxp - order - 1;
+        ye = tl.y0 < order || tl.y0 + TYA > sh.nyp - order - 1;
+        Kx = FW ? kfw(ix, sh.nxp, order) : kbw(ix, sh.nxp, order);
+        xc = strip_col(ix, sh.nxp, L);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            in[r] = ix < sh.nxp && iy + r < sh.nyp;
+            yc[r] = in[r] ? strip_col(iy + r, sh.nyp, L) : -1;
+            Ky[r] = FW ? kfw(iy + r, sh.nyp, order) : kbw(iy + r, sh.nyp, order);
+        }
+    }
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(TX3 *TY3, 2) a3d_velocity_tma(Step3DArgs<float> a, const CoefSet3<float> *coefs)
 {
     using T = float;
-    constexpr int MODE = MODE_FAST;
     using A = Ar<T, MODE>;
     extern __shared__ unsigned char smraw[];
     A3Smem<A3VelStage> &S =
@@ -329,84 +377,118 @@ __global__ void __launch_bounds__(TX3 *TY3, 3) a3d_velocity_tma(Step3DArgs<float
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX3 + tx;
     const Tile3D tl = a.tiles[blockIdx.x];
     const Shot3D<T> &sh = a.shots[tl.shot];
-    load_coefs3(S.cs, coefs);
-    if (tid == 0)
-        for (int k = 0; k < NSTG_A3; k++) mbar_init(&S.bar[k], 1);
-    __syncthreads();
     const CUtensorMap *M = reinterpret_cast<const CUtensorMap *>(a.maps) + (size_t)tl.shot * NMAP_A3;
-    const int x0 = tl.x0, y0 = tl.y0, ix = x0 + tx, iy = y0 + ty;
+    const int x0 = tl.x0, y0 = tl.y0;
     const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch, L = a.lpml, order = a.order;
-    const long long plane = sh.plane;
-    const int col = iy * pitch + ix;
-    const T *P = sh.f[A3_P];
-    T *Vx = sh.f[A3_VX], *Vy = sh.f[A3_VY], *Vz = sh.f[A3_VZ];
-    const bool in_grid = ix < nxp && iy < nyp;
-    const int Kx = kfw(ix, nxp, order), Ky = kfw(iy, nyp, order);
-    int xb = 0, xc = 0, yb = 0, yc = 0;
-    const int xi = in_grid ? xstrip(ix, nxp, L, xb, xc) : -1;
-    const int yi = in_grid ? xstrip(iy, nyp, L, yb, yc) : -1;
+    const int plane = (int)sh.plane;
     const int z0 = tl.z0, ze = min(z0 + a.zc, nzp);
     // stage k <- plane iz; the boxes start on 16-byte boundaries (x0, x0 + 8 multiples of 4)
     auto issue = [&](int iz, int k) {
         A3VelStage &g = S.st[k];
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(&S.bar[k], (uint32_t)sizeof(A3VelStage));
-        tma_load_2d(g.p, M + AM_PH, &S.bar[k], x0, a3_row(sh, iz, y0));
-        for (int q = 0; q < 6; q++) tma_load_2d(g.pv[q], M + AM_VX + q, &S.bar[k], x0 + GUARD, a3_row(sh, iz, GUARD + y0));
+        const int r = alloc_row3(sh, iz, GUARD + y0);
+        tma_load_2d(g.p, M + AM_PH, &S.bar[k], x0, alloc_row3(sh, iz, y0));
+        for (int q = 0; q < 6; q++) tma_load_2d(g.pv[q], M + AM_VX + q, &S.bar[k], x0 + GUARD, r);
+        tma_load_2d(g.up, M + AM_P, &S.bar[k], x0 + GUARD, alloc_row3(sh, iz + 9, GUARD + y0));
     };
-    if (tid == 0)
+    if (tid == 0) {
+        for (int k = 0; k < NSTG_A3; k++) mbar_init(&S.bar[k], 1);
         for (int j = 0; j < NSTG_A3 - 1 && z0 + j < ze; j++) issue(z0 + j, j);
-    T q[16];                                     // P, planes z-7..z+8 (forward z-derivative)
+    }
+    load_coefs3(S.cs, coefs);
+    stage_pml3(S.pml, a.pml, L, x0, y0, nxp, nyp);
+    A3Cols c;
+    c.set<true>(sh, tl, L, order);
+    const T *P = sh.f[A3_P];
+    T *Vx = sh.f[A3_VX], *Vy = sh.f[A3_VY], *Vz = sh.f[A3_VZ];
+    T *psx = sh.psix[0], *psy = sh.psiy[0], *psz = sh.psiz[0];
+    float2 q[16];                                // P, planes z-7..z+8 (forward z-derivative)
 #pragma unroll
-    for (int j = 0; j < 16; j++) q[j] = P[(z0 - 7 + j) * plane + col];
-    const T *cux = S.cs.cx + order * CROW3, *cuy = S.cs.cy + order * CROW3, *cuz = S.cs.cz + order * CROW3;
-    long long o = (long long)z0 * plane + col;
+    for (int j = 0; j < 16; j++) {
+        const T *w = P + (z0 - 7 + j) * plane + c.col;
+        q[j] = make_float2(w[0], w[pitch]);
+    }
+    __syncthreads();
+    int o = z0 * plane + c.col;
     for (int iz = z0; iz < ze; iz++, o += plane) {
         const int j = iz - z0, k = j % NSTG_A3;
-        if (tid == 0 && iz + NSTG_A3 - 1 < ze) issue(iz + NSTG_A3 - 1, (j + NSTG_A3 - 1) % NSTG_A3);
-        const T nq = P[o + 9 * plane];          // window refill, in flight while the stage arrives
+        // the plane's C-PML memory, in flight while the stage arrives
+        const int zc = strip_col(iz, nzp, L);
+        T mx[2], my[2], mz[2];
+        int ox[2], oy[2], oz[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            ox[r] = (iz * nyp + c.iy + r) * 2 * L + c.xc;
+            oy[r] = (iz * 2 * L + c.yc[r]) * nxp + c.ix;
+            oz[r] = (zc * nyp + c.iy + r) * nxp + c.ix;
+            mx[r] = my[r] = mz[r] = 0;
+            if (c.in[r] && c.xc >= 0) mx[r] = psx[ox[r]];
+            if (c.yc[r] >= 0) my[r] = psy[oy[r]];
+            if (c.in[r] && zc >= 0) mz[r] = psz[oz[r]];
+        }
+        // every thread is done with the plane before, whose stage is refilled now
         if (!__syncthreads_and(mbar_wait_bounded(&S.bar[k], (uint32_t)(j / NSTG_A3) & 1u, a.err))) return;
+        if (tid == 0 && iz + NSTG_A3 - 1 < ze) issue(iz + NSTG_A3 - 1, (j + NSTG_A3 - 1) % NSTG_A3);
         const A3VelStage &g = S.st[k];
-        const T *cx = &g.p[ty + 8][tx + 8];
-        const T dfx = (Kx == order) ? taps<T, MODE>(cx - 7, 1, cux, a.dx, a.rdx)
-                                    : stencil_ki<T, MODE>(cx, 1, Kx, S.cs.cx + Kx * CROW3, true, a.dx, a.rdx);
-        const T dfy = (Ky == order) ? taps<T, MODE>(cx - 7 * WX3, WX3, cuy, a.dy, a.rdy)
-                                    : stencil_ki<T, MODE>(cx, WX3, Ky, S.cs.cy + Ky * CROW3, true, a.dy, a.rdy);
+        const T *cx = &g.p[2 * ty + 8][tx + 8];
+        float2 dx, dy, dz;
+        if (!c.xe) {
+            dx = taps_lanes<MODE>([&](int t) { return make_float2(cx[t - 7], cx[WX3 + t - 7]); }, a.cf2[0], a.dx, a.rdx);
+        } else {
+            const T *w = S.cs.cx + c.Kx * CROW3;
+            dx.x = stencil_ki<T, MODE>(cx, 1, c.Kx, w, true, a.dx, a.rdx);
+            dx.y = stencil_ki<T, MODE>(cx + WX3, 1, c.Kx, w, true, a.dx, a.rdx);
+        }
+        if (!c.ye) {
+            dy = taps_rows<MODE>(cx - 7 * WX3, WX3, a.cf[1], a.dy, a.rdy);
+        } else {
+            dy.x = stencil_ki<T, MODE>(cx, WX3, c.Ky[0], S.cs.cy + c.Ky[0] * CROW3, true, a.dy, a.rdy);
+            dy.y = stencil_ki<T, MODE>(cx + WX3, WX3, c.Ky[1], S.cs.cy + c.Ky[1] * CROW3, true, a.dy, a.rdy);
+        }
         const int Kz = kfw(iz, nzp, order);
-        const T dfz = (Kz == order) ? taps_reg<T, MODE>(q, cuz, a.dz, a.rdz)
-                                    : stencil_ki<T, MODE>(P + o, (int)plane, Kz, S.cs.cz + Kz * CROW3, true, a.dz, a.rdz);
-        T vx = g.pv[0][ty][tx], vy = g.pv[1][ty][tx], vz = g.pv[2][ty][tx];
-        T am = A::mul(a.dt, g.pv[3][ty][tx]);
-        vx = A::mad(vx, am, dfx);
-        if (xi >= 0)
-            vx = pml_correct<T, MODE>(vx, am, dfx, sh.psix[0] + ((long long)iz * nyp + iy) * 2 * L + xc, a.pml, L,
-                                      xb + 3, xi);
-        Vx[o] = vx;
-        am = A::mul(a.dt, g.pv[4][ty][tx]);
-        vy = A::mad(vy, am, dfy);
-        if (yi >= 0)
-            vy = pml_correct<T, MODE>(vy, am, dfy, sh.psiy[0] + ((long long)iz * 2 * L + yc) * nxp + ix, a.pml, L,
-                                      yb + 3, yi);
-        Vy[o] = vy;
-        am = A::mul(a.dt, g.pv[5][ty][tx]);
-        vz = A::mad(vz, am, dfz);
-        int zb = 0, zc = 0;
-        const int zi = in_grid ? xstrip(iz, nzp, L, zb, zc) : -1;
-        if (zi >= 0)
-            vz = pml_correct<T, MODE>(vz, am, dfz, sh.psiz[0] + ((long long)zc * nyp + iy) * nxp + ix, a.pml, L,
-                                      zb + 3, zi);
-        Vz[o] = vz;
+        if (Kz == order) dz = taps_lanes<MODE>([&](int t) { return q[t]; }, a.cf2[2], a.dz, a.rdz);
+        else dz = taps_lanes_k<MODE>(q, Kz, S.cs.cz + Kz * CROW3, a.dz, a.rdz);
+        const T *fz = strip_factors(a.pml, L, iz, nzp, 1);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int y = 2 * ty + r, or_ = o + r * pitch;
+            const T dxr = r ? dx.y : dx.x, dyr = r ? dy.y : dy.x, dzr = r ? dz.y : dz.x;
+            T vx = g.pv[0][y][tx], vy = g.pv[1][y][tx], vz = g.pv[2][y][tx];
+            const T ax = A::mul(a.dt, g.pv[3][y][tx]), ay = A::mul(a.dt, g.pv[4][y][tx]), az = A::mul(a.dt, g.pv[5][y][tx]);
+            vx = A::mad(vx, ax, dxr);
+            vy = A::mad(vy, ay, dyr);
+            vz = A::mad(vz, az, dzr);
+            if (c.in[r] && c.xc >= 0) {
+                const T(&f)[3][TX3] = S.pml.x[1];
+                vx = A::msub(vx, ax, pml_term<T, MODE>(mx[r], dxr, f[0][tx], f[1][tx], f[2][tx]));
+                psx[ox[r]] = mx[r];
+            }
+            if (c.yc[r] >= 0) {
+                const T(&f)[3][TYA] = S.pml.y[1];
+                vy = A::msub(vy, ay, pml_term<T, MODE>(my[r], dyr, f[0][y], f[1][y], f[2][y]));
+                psy[oy[r]] = my[r];
+            }
+            if (c.in[r] && zc >= 0) {
+                vz = A::msub(vz, az, pml_term<T, MODE>(mz[r], dzr, __ldg(fz), __ldg(fz + L), __ldg(fz + 2 * L)));
+                psz[oz[r]] = mz[r];
+            }
+            if (c.in[r]) {
+                Vx[or_] = vx;
+                Vy[or_] = vy;
+                Vz[or_] = vz;
+            }
+        }
 #pragma unroll
         for (int jj = 0; jj < 15; jj++) q[jj] = q[jj + 1];
-        q[15] = nq;
-        __syncthreads();   // stage k is refilled next iteration
+        q[15] = make_float2(g.up[2 * ty][tx], g.up[2 * ty + 1][tx]);
     }
 }
 
-__global__ void __launch_bounds__(TX3 *TY3, 3) a3d_stress_tma(Step3DArgs<float> a, const CoefSet3<float> *coefs)
+template <int MODE>
+__global__ void __launch_bounds__(TX3 *TY3, 2) a3d_stress_tma(Step3DArgs<float> a, const CoefSet3<float> *coefs)
 {
     using T = float;
-    constexpr int MODE = MODE_FAST;
     using A = Ar<T, MODE>;
     extern __shared__ unsigned char smraw[];
     A3Smem<A3StrStage> &S =
@@ -414,76 +496,107 @@ __global__ void __launch_bounds__(TX3 *TY3, 3) a3d_stress_tma(Step3DArgs<float> 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX3 + tx;
     const Tile3D tl = a.tiles[blockIdx.x];
     const Shot3D<T> &sh = a.shots[tl.shot];
-    load_coefs3(S.cs, coefs);
-    if (tid == 0)
-        for (int k = 0; k < NSTG_A3; k++) mbar_init(&S.bar[k], 1);
-    __syncthreads();
     const CUtensorMap *M = reinterpret_cast<const CUtensorMap *>(a.maps) + (size_t)tl.shot * NMAP_A3;
-    const int x0 = tl.x0, y0 = tl.y0, ix = x0 + tx, iy = y0 + ty;
+    const int x0 = tl.x0, y0 = tl.y0;
     const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch, L = a.lpml, order = a.order;
-    const long long plane = sh.plane;
-    const int col = iy * pitch + ix;
-    T *P = sh.f[A3_P];
-    const T *Vz = sh.f[A3_VZ];
-    const bool in_grid = ix < nxp && iy < nyp;
-    const int Kx = kbw(ix, nxp, order), Ky = kbw(iy, nyp, order);
-    int xb = 0, xc = 0, yb = 0, yc = 0;
-    const int xi = in_grid ? xstrip(ix, nxp, L, xb, xc) : -1;
-    const int yi = in_grid ? xstrip(iy, nyp, L, yb, yc) : -1;
+    const int plane = (int)sh.plane;
     const int z0 = tl.z0, ze = min(z0 + a.zc, nzp);
     auto issue = [&](int iz, int k) {
         A3StrStage &g = S.st[k];
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(&S.bar[k], (uint32_t)sizeof(A3StrStage));
-        const int rh = a3_row(sh, iz, GUARD + y0);
+        const int rh = alloc_row3(sh, iz, GUARD + y0);
         tma_load_2d(g.vx, M + AM_VXH, &S.bar[k], x0, rh);
-        tma_load_2d(g.vy, M + AM_VYH, &S.bar[k], x0 + GUARD, a3_row(sh, iz, y0));
+        tma_load_2d(g.vy, M + AM_VYH, &S.bar[k], x0 + GUARD, alloc_row3(sh, iz, y0));
         tma_load_2d(g.pl[0], M + AM_P, &S.bar[k], x0 + GUARD, rh);
         tma_load_2d(g.pl[1], M + AM_L, &S.bar[k], x0 + GUARD, rh);
+        tma_load_2d(g.up, M + AM_VZ, &S.bar[k], x0 + GUARD, alloc_row3(sh, iz + 8, GUARD + y0));
     };
-    if (tid == 0)
+    if (tid == 0) {
+        for (int k = 0; k < NSTG_A3; k++) mbar_init(&S.bar[k], 1);
         for (int j = 0; j < NSTG_A3 - 1 && z0 + j < ze; j++) issue(z0 + j, j);
-    T q[16];                                     // Vz, planes z-8..z+7 (backward z-derivative)
+    }
+    load_coefs3(S.cs, coefs);
+    stage_pml3(S.pml, a.pml, L, x0, y0, nxp, nyp);
+    A3Cols c;
+    c.set<false>(sh, tl, L, order);
+    T *P = sh.f[A3_P];
+    const T *Vz = sh.f[A3_VZ];
+    T *psx = sh.psix[1], *psy = sh.psiy[1], *psz = sh.psiz[1];
+    float2 q[16];                                // Vz, planes z-8..z+7 (backward z-derivative)
 #pragma unroll
-    for (int j = 0; j < 16; j++) q[j] = Vz[(z0 - 8 + j) * plane + col];
-    const T *cux = S.cs.cx + order * CROW3, *cuy = S.cs.cy + order * CROW3, *cuz = S.cs.cz + order * CROW3;
-    long long o = (long long)z0 * plane + col;
+    for (int j = 0; j < 16; j++) {
+        const T *w = Vz + (z0 - 8 + j) * plane + c.col;
+        q[j] = make_float2(w[0], w[pitch]);
+    }
+    __syncthreads();
+    int o = z0 * plane + c.col;
     for (int iz = z0; iz < ze; iz++, o += plane) {
         const int j = iz - z0, k = j % NSTG_A3;
-        if (tid == 0 && iz + NSTG_A3 - 1 < ze) issue(iz + NSTG_A3 - 1, (j + NSTG_A3 - 1) % NSTG_A3);
-        const T nq = Vz[o + 8 * plane];
+        const int zc = strip_col(iz, nzp, L);
+        T mx[2], my[2], mz[2];
+        int ox[2], oy[2], oz[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            ox[r] = (iz * nyp + c.iy + r) * 2 * L + c.xc;
+            oy[r] = (iz * 2 * L + c.yc[r]) * nxp + c.ix;
+            oz[r] = (zc * nyp + c.iy + r) * nxp + c.ix;
+            mx[r] = my[r] = mz[r] = 0;
+            if (c.in[r] && c.xc >= 0) mx[r] = psx[ox[r]];
+            if (c.yc[r] >= 0) my[r] = psy[oy[r]];
+            if (c.in[r] && zc >= 0) mz[r] = psz[oz[r]];
+        }
         if (!__syncthreads_and(mbar_wait_bounded(&S.bar[k], (uint32_t)(j / NSTG_A3) & 1u, a.err))) return;
+        if (tid == 0 && iz + NSTG_A3 - 1 < ze) issue(iz + NSTG_A3 - 1, (j + NSTG_A3 - 1) % NSTG_A3);
         const A3StrStage &g = S.st[k];
-        const T *cx = &g.vx[ty][tx + 8];
-        const T *cy = &g.vy[ty + 8][tx];
-        const T d1 = (Kx == order) ? taps<T, MODE>(cx - 8, 1, cux, a.dx, a.rdx)
-                                   : stencil_ki<T, MODE>(cx, 1, Kx, S.cs.cx + Kx * CROW3, false, a.dx, a.rdx);
-        const T d2 = (Ky == order) ? taps<T, MODE>(cy - 8 * TX3, TX3, cuy, a.dy, a.rdy)
-                                   : stencil_ki<T, MODE>(cy, TX3, Ky, S.cs.cy + Ky * CROW3, false, a.dy, a.rdy);
+        const T *cx = &g.vx[2 * ty][tx + 8];
+        const T *cy = &g.vy[2 * ty + 8][tx];
+        float2 d1, d2, d3;
+        if (!c.xe) {
+            d1 = taps_lanes<MODE>([&](int t) { return make_float2(cx[t - 8], cx[WX3 + t - 8]); }, a.cf2[0], a.dx, a.rdx);
+        } else {
+            const T *w = S.cs.cx + c.Kx * CROW3;
+            d1.x = stencil_ki<T, MODE>(cx, 1, c.Kx, w, false, a.dx, a.rdx);
+            d1.y = stencil_ki<T, MODE>(cx + WX3, 1, c.Kx, w, false, a.dx, a.rdx);
+        }
+        if (!c.ye) {
+            d2 = taps_rows<MODE>(cy - 8 * TX3, TX3, a.cf[1], a.dy, a.rdy);
+        } else {
+            d2.x = stencil_ki<T, MODE>(cy, TX3, c.Ky[0], S.cs.cy + c.Ky[0] * CROW3, false, a.dy, a.rdy);
+            d2.y = stencil_ki<T, MODE>(cy + TX3, TX3, c.Ky[1], S.cs.cy + c.Ky[1] * CROW3, false, a.dy, a.rdy);
+        }
         const int Kz = kbw(iz, nzp, order);
-        const T d3 = (Kz == order) ? taps_reg<T, MODE>(q, cuz, a.dz, a.rdz)
-                                   : stencil_ki<T, MODE>(Vz + o, (int)plane, Kz, S.cs.cz + Kz * CROW3, false, a.dz, a.rdz);
-        T p = g.pl[0][ty][tx];
-        const T am = A::mul(a.dt, g.pl[1][ty][tx]);
-        p = A::mad(p, am, d1);
-        if (xi >= 0)
-            p = pml_correct<T, MODE>(p, am, d1, sh.psix[1] + ((long long)iz * nyp + iy) * 2 * L + xc, a.pml, L, xb,
-                                     xi);
-        p = A::mad(p, am, d2);
-        if (yi >= 0)
-            p = pml_correct<T, MODE>(p, am, d2, sh.psiy[1] + ((long long)iz * 2 * L + yc) * nxp + ix, a.pml, L, yb,
-                                     yi);
-        p = A::mad(p, am, d3);
-        int zb = 0, zc = 0;
-        const int zi = in_grid ? xstrip(iz, nzp, L, zb, zc) : -1;
-        if (zi >= 0)
-            p = pml_correct<T, MODE>(p, am, d3, sh.psiz[1] + ((long long)zc * nyp + iy) * nxp + ix, a.pml, L, zb,
-                                     zi);
-        P[o] = p;
+        if (Kz == order) d3 = taps_lanes<MODE>([&](int t) { return q[t]; }, a.cf2[2], a.dz, a.rdz);
+        else d3 = taps_lanes_k<MODE>(q, Kz, S.cs.cz + Kz * CROW3, a.dz, a.rdz);
+        const T *fz = strip_factors(a.pml, L, iz, nzp, 0);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int y = 2 * ty + r;
+            const T dxr = r ? d1.y : d1.x, dyr = r ? d2.y : d2.x, dzr = r ? d3.y : d3.x;
+            T p = g.pl[0][y][tx];
+            const T am = A::mul(a.dt, g.pl[1][y][tx]);
+            p = A::mad(p, am, dxr);
+            if (c.in[r] && c.xc >= 0) {
+                const T(&f)[3][TX3] = S.pml.x[0];
+                p = A::msub(p, am, pml_term<T, MODE>(mx[r], dxr, f[0][tx], f[1][tx], f[2][tx]));
+                psx[ox[r]] = mx[r];
+            }
+            p = A::mad(p, am, dyr);
+            if (c.yc[r] >= 0) {
+                const T(&f)[3][TYA] = S.pml.y[0];
+                p = A::msub(p, am, pml_term<T, MODE>(my[r], dyr, f[0][y], f[1][y], f[2][y]));
+                psy[oy[r]] = my[r];
+            }
+            p = A::mad(p, am, dzr);
+            if (c.in[r] && zc >= 0) {
+                p = A::msub(p, am, pml_term<T, MODE>(mz[r], dzr, __ldg(fz), __ldg(fz + L), __ldg(fz + 2 * L)));
+                psz[oz[r]] = mz[r];
+            }
+            if (c.in[r]) P[o + r * pitch] = p;
+        }
 #pragma unroll
         for (int jj = 0; jj < 15; jj++) q[jj] = q[jj + 1];
-        q[15] = nq;
-        __syncthreads();
+        q[15] = make_float2(g.up[2 * ty][tx], g.up[2 * ty + 1][tx]);
     }
 }
 
@@ -492,27 +605,22 @@ cudaError_t step3(int half, const void *args, const void *coefs, int grid, cudaS
 {
     const Step3DArgs<T> &a = *reinterpret_cast<const Step3DArgs<T> *>(args);
     const dim3 block(TX3, TY3);
-    if constexpr (MODE == MODE_FAST && std::is_same<T, float>::value) {
-        if (a.maps) {
-            // TMA-staged planes (the plan builds the maps in fast mode)
-            if (half == 0) {
-                auto k = a3d_velocity_tma;
-                const size_t sm = a3_smem_bytes<A3VelStage>();
-                cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-                if (e != cudaSuccess) return e;
-                k<<<grid, block, sm, st>>>(a, (const CoefSet3<float> *)coefs);
-            } else {
-                auto k = a3d_stress_tma;
-                const size_t sm = a3_smem_bytes<A3StrStage>();
-                cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-                if (e != cudaSuccess) return e;
-                k<<<grid, block, sm, st>>>(a, (const CoefSet3<float> *)coefs);
-            }
-            return cudaGetLastError();
+    if constexpr (std::is_same<T, float>::value) {
+        if (half == 0) {
+            constexpr size_t sm = a3_smem_bytes<A3VelStage>();
+            static const cudaError_t e = cudaFuncSetAttribute(a3d_velocity_tma<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            if (e != cudaSuccess) return e;
+            a3d_velocity_tma<MODE><<<grid, block, sm, st>>>(a, (const CoefSet3<float> *)coefs);
+        } else {
+            constexpr size_t sm = a3_smem_bytes<A3StrStage>();
+            static const cudaError_t e = cudaFuncSetAttribute(a3d_stress_tma<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            if (e != cudaSuccess) return e;
+            a3d_stress_tma<MODE><<<grid, block, sm, st>>>(a, (const CoefSet3<float> *)coefs);
         }
+    } else {
+        if (half == 0) a3d_velocity<T, MODE><<<grid, block, 0, st>>>(a, (const CoefSet3<T> *)coefs);
+        else a3d_stress<T, MODE><<<grid, block, 0, st>>>(a, (const CoefSet3<T> *)coefs);
     }
-    if (half == 0) a3d_velocity<T, MODE><<<grid, block, 0, st>>>(a, (const CoefSet3<T> *)coefs);
-    else a3d_stress<T, MODE><<<grid, block, 0, st>>>(a, (const CoefSet3<T> *)coefs);
     return cudaGetLastError();
 }
 
@@ -528,16 +636,16 @@ cudaError_t launch_step_3d(int prec, int physics, int half, const void *args, co
 }
 
 cudaError_t launch_injrec_3d(int prec, const void *shots, const void *plans, int nshots, double dt, int it,
-                             cudaStream_t st)
+                             int threads, cudaStream_t st)
 {
     if (prec == PREC_F64)
-        inject_record_3d<double, MODE_IEEE><<<nshots, 256, 0, st>>>((const Shot3D<double> *)shots,
+        inject_record_3d<double, MODE_IEEE><<<nshots, threads, 0, st>>>((const Shot3D<double> *)shots,
                                                                     (const InjRec3<double> *)plans, dt, it);
     else if (prec == PREC_F32_EXACT)
-        inject_record_3d<float, MODE_IEEE><<<nshots, 256, 0, st>>>((const Shot3D<float> *)shots,
+        inject_record_3d<float, MODE_IEEE><<<nshots, threads, 0, st>>>((const Shot3D<float> *)shots,
                                                                    (const InjRec3<float> *)plans, (float)dt, it);
     else
-        inject_record_3d<float, MODE_FAST><<<nshots, 256, 0, st>>>((const Shot3D<float> *)shots,
+        inject_record_3d<float, MODE_FAST><<<nshots, threads, 0, st>>>((const Shot3D<float> *)shots,
                                                                    (const InjRec3<float> *)plans, (float)dt, it);
     return cudaGetLastError();
 }

@@ -25,20 +25,10 @@
 //   psix[3] normal stresses (Vx)   psiy[3] normal (Vy)        psiz[3] normal (Vz)
 //   psix[4] Sxz (Vz, stag.)        psiy[4] Syz (Vz, stag.)    psiz[4] Sxz (Vx, stag.)
 //   psix[5] Sxy (Vy, stag.)        psiy[5] Sxy (Vx, stag.)    psiz[5] Syz (Vy, stag.)
-#include "fd2d_kernels.cuh"
-#include "rsgpu_3d.h"
+#include "fd3d_common.cuh"
 
 namespace rsgpu {
 namespace {
-
-template <typename T>
-__device__ __forceinline__ void load_coefs3e(CoefSet3<T> &s, const CoefSet3<T> *g)
-{
-    const T *src = reinterpret_cast<const T *>(g);
-    T *dst = reinterpret_cast<T *>(&s);
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    for (int i = tid; i < (int)(sizeof(CoefSet3<T>) / sizeof(T)); i += blockDim.x * blockDim.y) dst[i] = src[i];
-}
 
 // Copy the shot descriptor into shared memory: the field pointers are then read
 // from a space that the kernel's global stores cannot alias, so the compiler may
@@ -141,7 +131,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity(Step3DArgs<T> a, con
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
     stage_shot(shs, a.shots + tl.shot);
-    load_coefs3e(S.cs, coefs);
+    load_coefs3(S.cs, coefs);
     __syncthreads();
     const int tx = threadIdx.x, ty = threadIdx.y;
     const Shot3D<T> &sh = shs;
@@ -320,7 +310,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress(Step3DArgs<T> a, const
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
     stage_shot(shs, a.shots + tl.shot);
-    load_coefs3e(S.cs, coefs);
+    load_coefs3(S.cs, coefs);
     __syncthreads();
     const int tx = threadIdx.x, ty = threadIdx.y;
     const Shot3D<T> &sh = shs;
@@ -487,398 +477,21 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress(Step3DArgs<T> a, const
     }
 }
 
-// ---------------------------------------------------------------- fast-mode kernels
-// RSGPU_F32_FAST versions of the two half-steps: the same stencils, C-PML and
-// update order, with derivatives that share an axis and a direction computed in
-// pairs -- one 64-bit shared load and one FADD2/FFMA2 per tap for two fields -- and
-// the full-order coefficients taken from the launch's parameter space.
-//   velocity: x backward (XY, XZ), y backward (XY, YZ), z backward (XZ, YZ);
-//             single: x forward XX, y forward YY, z forward ZZ
-//   stress:   x forward (Vz, Vy), y forward (Vz, Vx), z forward (Vx, Vy);
-//             single: x backward Vx, y backward Vy, z backward Vz
-__device__ __forceinline__ float2 taps_pair(const float2 *b, int s, const float (&c2)[NCOEF][2])
-{
-    using A2 = Ar2<float, MODE_FAST>;
-    const float2 *cc = reinterpret_cast<const float2 *>(c2);
-    float2 acc = A2::mul(A2::sub(b[8 * s], b[7 * s]), cc[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A2::acc(acc, A2::sub(b[(8 + k) * s], b[(7 - k) * s]), cc[k]);
-    return acc;
-}
-__device__ __forceinline__ float2 taps_pair_reg(const float2 (&q)[16], const float (&c2)[NCOEF][2])
-{
-    using A2 = Ar2<float, MODE_FAST>;
-    const float2 *cc = reinterpret_cast<const float2 *>(c2);
-    float2 acc = A2::mul(A2::sub(q[8], q[7]), cc[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A2::acc(acc, A2::sub(q[8 + k], q[7 - k]), cc[k]);
-    return acc;
-}
-
-struct VelSmemF {
-    float xx[2][TY3][WX];      // XX, x halo
-    float2 xq[2][TY3][WX];     // (XY, XZ), x halo
-    float2 yq[2][HY][TX3];     // (XY, YZ), y halo
-    float yy[2][HY][TX3];      // YY, y halo
-    CoefSet3<float> cs;
-};
-
-template <bool ADJ>
-__global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_fast(Step3DArgs<float> a, const CoefSet3<float> *coefs)
-{
-    using T = float;
-    constexpr int MODE = MODE_FAST;
-    using A = Ar<T, MODE>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    VelSmemF &S = *reinterpret_cast<VelSmemF *>(smraw);
-    __shared__ Shot3D<T> shs;
-    const Tile3D tl = a.tiles[blockIdx.x];
-    stage_shot(shs, a.shots + tl.shot);
-    load_coefs3e(S.cs, coefs);
-    __syncthreads();
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const Shot3D<T> &sh = shs;
-    const int ix = tl.x0 + tx, iy = tl.y0 + ty;
-    const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch, L = a.lpml, order = a.order;
-    const int plane = (int)sh.plane;   // a field holds fewer than 2^31 elements
-    const int col = iy * pitch + ix;
-    T *Vx = sh.f[E3_VX], *Vy = sh.f[E3_VY], *Vz = sh.f[E3_VZ];
-    const T *Rx = sh.m[ME_RX], *Ry = sh.m[ME_RY], *Rz = sh.m[ME_RZ];
-    const bool in_grid = ix < nxp && iy < nyp;
-    const int Kxf = kfw(ix, nxp, order), Kxb = kbw(ix, nxp, order);
-    const int Kyf = kfw(iy, nyp, order), Kyb = kbw(iy, nyp, order);
-    int xb = 0, xc = 0, yb = 0, yc = 0;
-    const int xi = in_grid ? xstrip(ix, nxp, L, xb, xc) : -1;
-    const int yi = in_grid ? xstrip(iy, nyp, L, yb, yc) : -1;
-    const int z0 = tl.z0, ze = min(z0 + a.zc, nzp);
-    const int hx = tx < 8 ? -8 : TX3 - 8;
-    // z windows: (XZ, YZ) backward (planes z-8..z+7), ZZ forward (z-7..z+8)
-    float2 qp[16];
-    T qzz[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-        const int oj = (z0 - 8 + j) * plane + col;
-        qp[j] = make_float2(opnd<T, MODE, ADJ>(sh, oj, OP_XZ), opnd<T, MODE, ADJ>(sh, oj, OP_YZ));
-        qzz[j] = opnd<T, MODE, ADJ>(sh, (z0 - 7 + j) * plane + col, OP_ZZ);
-    }
-    int o = z0 * plane + col;
-    T vx = Vx[o], vy = Vy[o], vz = Vz[o], rx = __ldg(Rx + o), ry = __ldg(Ry + o), rz = __ldg(Rz + o);
-    T cxx = opnd<T, MODE, ADJ>(sh, o, OP_XX), cxy = opnd<T, MODE, ADJ>(sh, o, OP_XY), cyy = opnd<T, MODE, ADJ>(sh, o, OP_YY);
-    T hxx = 0, hxy = 0, hxz = 0;
-    if (tx < 16) {
-        hxx = opnd<T, MODE, ADJ>(sh, o + hx, OP_XX);
-        hxy = opnd<T, MODE, ADJ>(sh, o + hx, OP_XY);
-        hxz = opnd<T, MODE, ADJ>(sh, o + hx, OP_XZ);
-    }
-    T vxy0 = opnd<T, MODE, ADJ>(sh, o - 8 * pitch, OP_XY), vxy1 = opnd<T, MODE, ADJ>(sh, o + TY3 * pitch, OP_XY);
-    T vyy0 = opnd<T, MODE, ADJ>(sh, o - 8 * pitch, OP_YY), vyy1 = opnd<T, MODE, ADJ>(sh, o + TY3 * pitch, OP_YY);
-    T vyz0 = opnd<T, MODE, ADJ>(sh, o - 8 * pitch, OP_YZ), vyz1 = opnd<T, MODE, ADJ>(sh, o + TY3 * pitch, OP_YZ);
-    __syncthreads();
-    for (int iz = z0; iz < ze; iz++, o += plane) {
-        const int b = (iz - z0) & 1;
-        S.xx[b][ty][tx + 8] = cxx;
-        S.xq[b][ty][tx + 8] = make_float2(cxy, qp[8].x);
-        S.yq[b][ty + 8][tx] = make_float2(cxy, qp[8].y);
-        S.yy[b][ty + 8][tx] = cyy;
-        if (tx < 16) {
-            const int c = tx < 8 ? tx : tx + TX3;
-            S.xx[b][ty][c] = hxx;
-            S.xq[b][ty][c] = make_float2(hxy, hxz);
-        }
-        S.yq[b][ty][tx] = make_float2(vxy0, vyz0);
-        S.yq[b][ty + TY3 + 8][tx] = make_float2(vxy1, vyz1);
-        S.yy[b][ty][tx] = vyy0;
-        S.yy[b][ty + TY3 + 8][tx] = vyy1;
-        // next plane's inputs (the plane after the chunk lies inside the allocation; unused)
-        const int on = o + plane;
-        const T nvx = Vx[on], nvy = Vy[on], nvz = Vz[on];
-        const T nrx = __ldg(Rx + on), nry = __ldg(Ry + on), nrz = __ldg(Rz + on);
-        const T ncxx = opnd<T, MODE, ADJ>(sh, on, OP_XX), ncxy = opnd<T, MODE, ADJ>(sh, on, OP_XY),
-                ncyy = opnd<T, MODE, ADJ>(sh, on, OP_YY);
-        if (tx < 16) {
-            hxx = opnd<T, MODE, ADJ>(sh, on + hx, OP_XX);
-            hxy = opnd<T, MODE, ADJ>(sh, on + hx, OP_XY);
-            hxz = opnd<T, MODE, ADJ>(sh, on + hx, OP_XZ);
-        }
-        vxy0 = opnd<T, MODE, ADJ>(sh, on - 8 * pitch, OP_XY); vxy1 = opnd<T, MODE, ADJ>(sh, on + TY3 * pitch, OP_XY);
-        vyy0 = opnd<T, MODE, ADJ>(sh, on - 8 * pitch, OP_YY); vyy1 = opnd<T, MODE, ADJ>(sh, on + TY3 * pitch, OP_YY);
-        vyz0 = opnd<T, MODE, ADJ>(sh, on - 8 * pitch, OP_YZ); vyz1 = opnd<T, MODE, ADJ>(sh, on + TY3 * pitch, OP_YZ);
-        __syncthreads();
-        const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
-        int zb = 0, zc = 0;
-        const int zi = in_grid ? xstrip(iz, nzp, L, zb, zc) : -1;
-        const int px = (iz * nyp + iy) * 2 * L + xc;
-        const int py = (iz * 2 * L + yc) * nxp + ix;
-        const int pz = (zc * nyp + iy) * nxp + ix;
-        // full-order derivatives, then the reduced-order ones near the array ends
-        const T *cx1 = &S.xx[b][ty][tx + 8];
-        T dxx = taps3<T, MODE>(cx1 - 7, 1, a.cf[0], a.dx, a.rdx);
-        const float2 *cxq = &S.xq[b][ty][tx + 8];
-        float2 dxq = taps_pair(cxq - 8, 1, a.cf2[0]);
-        const float2 *cyq = &S.yq[b][ty + 8][tx];
-        float2 dyq = taps_pair(cyq - 8 * TX3, TX3, a.cf2[1]);
-        const T *cy1 = &S.yy[b][ty + 8][tx];
-        T dyy = taps3<T, MODE>(cy1 - 7 * TX3, TX3, a.cf[1], a.dy, a.rdy);
-        float2 dzq = taps_pair_reg(qp, a.cf2[2]);
-        T dzz = taps3_reg<T, MODE>(qzz, a.cf[2], a.dz, a.rdz);
-        if (Kxf != order) dxx = stencil_k<T, MODE>(cx1, 1, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
-        if (Kxb != order) {
-            const T *c = reinterpret_cast<const T *>(cxq);
-            dxq.x = stencil_k<T, MODE>(c, 2, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
-            dxq.y = stencil_k<T, MODE>(c + 1, 2, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
-        }
-        if (Kyb != order) {
-            const T *c = reinterpret_cast<const T *>(cyq);
-            dyq.x = stencil_k<T, MODE>(c, 2 * TX3, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-            dyq.y = stencil_k<T, MODE>(c + 1, 2 * TX3, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-        }
-        if (Kyf != order) dyy = stencil_k<T, MODE>(cy1, TX3, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
-        if (Kzb != order) {
-            dzq.x = stencil_z_op<T, MODE, ADJ>(sh, o, plane, Kzb, S.cs.cz + Kzb * CROW3, false, OP_XZ, a.dz, a.rdz);
-            dzq.y = stencil_z_op<T, MODE, ADJ>(sh, o, plane, Kzb, S.cs.cz + Kzb * CROW3, false, OP_YZ, a.dz, a.rdz);
-        }
-        if (Kzf != order)
-            dzz = stencil_z_op<T, MODE, ADJ>(sh, o, plane, Kzf, S.cs.cz + Kzf * CROW3, true, OP_ZZ, a.dz, a.rdz);
-        // ---- Vx: Dx+ XX, Dy- XY, Dz- XZ
-        {
-            const T am = A::mul(a.dt, rx);
-            vx = A::mad(vx, am, dxx);
-            if (xi >= 0) vx = pml_correct<T, MODE>(vx, am, dxx, sh.psix[0] + px, a.pml, L, xb + 3, xi);
-            vx = A::mad(vx, am, dyq.x);
-            if (yi >= 0) vx = pml_correct<T, MODE>(vx, am, dyq.x, sh.psiy[0] + py, a.pml, L, yb, yi);
-            vx = A::mad(vx, am, dzq.x);
-            if (zi >= 0) vx = pml_correct<T, MODE>(vx, am, dzq.x, sh.psiz[0] + pz, a.pml, L, zb, zi);
-            Vx[o] = vx;
-        }
-        // ---- Vy: Dx- XY, Dy+ YY, Dz- YZ
-        {
-            const T am = A::mul(a.dt, ry);
-            vy = A::mad(vy, am, dxq.x);
-            if (xi >= 0) vy = pml_correct<T, MODE>(vy, am, dxq.x, sh.psix[1] + px, a.pml, L, xb, xi);
-            vy = A::mad(vy, am, dyy);
-            if (yi >= 0) vy = pml_correct<T, MODE>(vy, am, dyy, sh.psiy[1] + py, a.pml, L, yb + 3, yi);
-            vy = A::mad(vy, am, dzq.y);
-            if (zi >= 0) vy = pml_correct<T, MODE>(vy, am, dzq.y, sh.psiz[1] + pz, a.pml, L, zb, zi);
-            Vy[o] = vy;
-        }
-        // ---- Vz: Dx- XZ, Dy- YZ, Dz+ ZZ
-        {
-            const T am = A::mul(a.dt, rz);
-            vz = A::mad(vz, am, dxq.y);
-            if (xi >= 0) vz = pml_correct<T, MODE>(vz, am, dxq.y, sh.psix[2] + px, a.pml, L, xb, xi);
-            vz = A::mad(vz, am, dyq.y);
-            if (yi >= 0) vz = pml_correct<T, MODE>(vz, am, dyq.y, sh.psiy[2] + py, a.pml, L, yb, yi);
-            vz = A::mad(vz, am, dzz);
-            if (zi >= 0) vz = pml_correct<T, MODE>(vz, am, dzz, sh.psiz[2] + pz, a.pml, L, zb + 3, zi);
-            Vz[o] = vz;
-        }
-#pragma unroll
-        for (int j = 0; j < 15; j++) { qp[j] = qp[j + 1]; qzz[j] = qzz[j + 1]; }
-        qp[15] = make_float2(opnd<T, MODE, ADJ>(sh, o + 8 * plane, OP_XZ), opnd<T, MODE, ADJ>(sh, o + 8 * plane, OP_YZ));
-        qzz[15] = opnd<T, MODE, ADJ>(sh, o + 9 * plane, OP_ZZ);
-        vx = nvx; vy = nvy; vz = nvz; rx = nrx; ry = nry; rz = nrz;
-        cxx = ncxx; cxy = ncxy; cyy = ncyy;
-    }
-}
-
-struct StrSmemF {
-    float sx[2][TY3][WX];      // Vx, x halo
-    float2 px[2][TY3][WX];     // (Vz, Vy), x halo
-    float sy[2][HY][TX3];      // Vy, y halo
-    float2 py[2][HY][TX3];     // (Vz, Vx), y halo
-    CoefSet3<float> cs;
-};
-
-template <bool ADJ>
-__global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_fast(Step3DArgs<float> a, const CoefSet3<float> *coefs)
-{
-    using T = float;
-    constexpr int MODE = MODE_FAST;
-    using A = Ar<T, MODE>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    StrSmemF &S = *reinterpret_cast<StrSmemF *>(smraw);
-    __shared__ Shot3D<T> shs;
-    const Tile3D tl = a.tiles[blockIdx.x];
-    stage_shot(shs, a.shots + tl.shot);
-    load_coefs3e(S.cs, coefs);
-    __syncthreads();
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const Shot3D<T> &sh = shs;
-    const int ix = tl.x0 + tx, iy = tl.y0 + ty;
-    const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch, L = a.lpml, order = a.order;
-    const int plane = (int)sh.plane;   // a field holds fewer than 2^31 elements
-    const int col = iy * pitch + ix;
-    const T *Vx = sh.f[E3_VX], *Vy = sh.f[E3_VY], *Vz = sh.f[E3_VZ];
-    T *Sxx = sh.f[E3_SXX], *Syy = sh.f[E3_SYY], *Szz = sh.f[E3_SZZ];
-    T *Syz = sh.f[E3_SYZ], *Sxz = sh.f[E3_SXZ], *Sxy = sh.f[E3_SXY];
-    const bool in_grid = ix < nxp && iy < nyp;
-    const int Kxf = kfw(ix, nxp, order), Kxb = kbw(ix, nxp, order);
-    const int Kyf = kfw(iy, nyp, order), Kyb = kbw(iy, nyp, order);
-    int xb = 0, xc = 0, yb = 0, yc = 0;
-    const int xi = in_grid ? xstrip(ix, nxp, L, xb, xc) : -1;
-    const int yi = in_grid ? xstrip(iy, nyp, L, yb, yc) : -1;
-    const int z0 = tl.z0, ze = min(z0 + a.zc, nzp);
-    const int hx = tx < 8 ? -8 : TX3 - 8;
-    // z windows: Vz backward (planes z-8..z+7), (Vx, Vy) forward (z-7..z+8)
-    T qz[16];
-    float2 qv[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-        qz[j] = Vz[(z0 - 8 + j) * plane + col];
-        const int oj = (z0 - 7 + j) * plane + col;
-        qv[j] = make_float2(Vx[oj], Vy[oj]);
-    }
-    int o = z0 * plane + col;
-    T sxx = Sxx[o], syy = Syy[o], szz = Szz[o], syz = Syz[o], sxz = Sxz[o], sxy = Sxy[o];
-    T l = 0, l2m = 0, myz = 0, mxz = 0, mxy = 0;
-    if (!ADJ) {
-        l = __ldg(sh.m[ME_L] + o); l2m = __ldg(sh.m[ME_L2M] + o);
-        myz = __ldg(sh.m[ME_MYZ] + o); mxz = __ldg(sh.m[ME_MXZ] + o); mxy = __ldg(sh.m[ME_MXY] + o);
-    }
-    T hvx = 0, hvy = 0, hvz = 0;
-    if (tx < 16) { hvx = Vx[o + hx]; hvy = Vy[o + hx]; hvz = Vz[o + hx]; }
-    T yx0 = Vx[o - 8 * pitch], yx1 = Vx[o + TY3 * pitch];
-    T yy0 = Vy[o - 8 * pitch], yy1 = Vy[o + TY3 * pitch];
-    T yz0 = Vz[o - 8 * pitch], yz1 = Vz[o + TY3 * pitch];
-    __syncthreads();
-    for (int iz = z0; iz < ze; iz++, o += plane) {
-        const int b = (iz - z0) & 1;
-        const T cvx = qv[7].x, cvy = qv[7].y, cvz = qz[8];
-        S.sx[b][ty][tx + 8] = cvx;
-        S.px[b][ty][tx + 8] = make_float2(cvz, cvy);
-        S.sy[b][ty + 8][tx] = cvy;
-        S.py[b][ty + 8][tx] = make_float2(cvz, cvx);
-        if (tx < 16) {
-            const int c = tx < 8 ? tx : tx + TX3;
-            S.sx[b][ty][c] = hvx;
-            S.px[b][ty][c] = make_float2(hvz, hvy);
-        }
-        S.sy[b][ty][tx] = yy0; S.sy[b][ty + TY3 + 8][tx] = yy1;
-        S.py[b][ty][tx] = make_float2(yz0, yx0); S.py[b][ty + TY3 + 8][tx] = make_float2(yz1, yx1);
-        const int on = o + plane;
-        const T nsxx = Sxx[on], nsyy = Syy[on], nszz = Szz[on], nsyz = Syz[on], nsxz = Sxz[on], nsxy = Sxy[on];
-        T nl = 0, nl2m = 0, nmyz = 0, nmxz = 0, nmxy = 0;
-        if (!ADJ) {
-            nl = __ldg(sh.m[ME_L] + on); nl2m = __ldg(sh.m[ME_L2M] + on);
-            nmyz = __ldg(sh.m[ME_MYZ] + on); nmxz = __ldg(sh.m[ME_MXZ] + on); nmxy = __ldg(sh.m[ME_MXY] + on);
-        }
-        if (tx < 16) { hvx = Vx[on + hx]; hvy = Vy[on + hx]; hvz = Vz[on + hx]; }
-        yx0 = Vx[on - 8 * pitch]; yx1 = Vx[on + TY3 * pitch];
-        yy0 = Vy[on - 8 * pitch]; yy1 = Vy[on + TY3 * pitch];
-        yz0 = Vz[on - 8 * pitch]; yz1 = Vz[on + TY3 * pitch];
-        __syncthreads();
-        const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
-        int zb = 0, zc = 0;
-        const int zi = in_grid ? xstrip(iz, nzp, L, zb, zc) : -1;
-        const int px = (iz * nyp + iy) * 2 * L + xc;
-        const int py = (iz * 2 * L + yc) * nxp + ix;
-        const int pz = (zc * nyp + iy) * nxp + ix;
-        const T *csx = &S.sx[b][ty][tx + 8];
-        T dxx = taps3<T, MODE>(csx - 8, 1, a.cf[0], a.dx, a.rdx);
-        const float2 *cpx = &S.px[b][ty][tx + 8];
-        float2 dxp = taps_pair(cpx - 7, 1, a.cf2[0]);                 // (Dx+ Vz, Dx+ Vy)
-        const T *csy = &S.sy[b][ty + 8][tx];
-        T dyy = taps3<T, MODE>(csy - 8 * TX3, TX3, a.cf[1], a.dy, a.rdy);
-        const float2 *cpy = &S.py[b][ty + 8][tx];
-        float2 dyp = taps_pair(cpy - 7 * TX3, TX3, a.cf2[1]);         // (Dy+ Vz, Dy+ Vx)
-        T dzz = taps3_reg<T, MODE>(qz, a.cf[2], a.dz, a.rdz);
-        float2 dzp = taps_pair_reg(qv, a.cf2[2]);                     // (Dz+ Vx, Dz+ Vy)
-        if (Kxb != order) dxx = stencil_k<T, MODE>(csx, 1, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
-        if (Kxf != order) {
-            const T *c = reinterpret_cast<const T *>(cpx);
-            dxp.x = stencil_k<T, MODE>(c, 2, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
-            dxp.y = stencil_k<T, MODE>(c + 1, 2, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
-        }
-        if (Kyb != order) dyy = stencil_k<T, MODE>(csy, TX3, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-        if (Kyf != order) {
-            const T *c = reinterpret_cast<const T *>(cpy);
-            dyp.x = stencil_k<T, MODE>(c, 2 * TX3, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
-            dyp.y = stencil_k<T, MODE>(c + 1, 2 * TX3, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
-        }
-        if (Kzb != order) dzz = stencil_k<T, MODE>(Vz + o, (int)plane, Kzb, S.cs.cz + Kzb * CROW3, false, a.dz, a.rdz);
-        if (Kzf != order) {
-            dzp.x = stencil_k<T, MODE>(Vx + o, (int)plane, Kzf, S.cs.cz + Kzf * CROW3, true, a.dz, a.rdz);
-            dzp.y = stencil_k<T, MODE>(Vy + o, (int)plane, Kzf, S.cs.cz + Kzf * CROW3, true, a.dz, a.rdz);
-        }
-        // ---- normal stresses
-        {
-            const bool fsrow = sh.fs && iz == L;
-            if (!ADJ) {
-                const T a2 = A::mul(a.dt, l2m), a1 = A::mul(a.dt, l);
-                auto upd3 = [&](T d, T cxx_, T cyy_, T czz_) {
-                    sxx = A::mad(sxx, cxx_, d); syy = A::mad(syy, cyy_, d); szz = A::mad(szz, czz_, d);
-                };
-                auto pml3 = [&](T d, T *psi, int base, int idx, T cxx_, T cyy_, T czz_) {
-                    const T tA = __ldg(a.pml + (base + PT_A) * L + idx), tB = __ldg(a.pml + (base + PT_B) * L + idx),
-                            tC = __ldg(a.pml + (base + PT_C) * L + idx);
-                    const T p = A::mad(A::mul(tB, *psi), tA, d);
-                    *psi = p;
-                    const T cq = A::mad(p, tC, d);
-                    sxx = A::msub(sxx, cxx_, cq); syy = A::msub(syy, cyy_, cq); szz = A::msub(szz, czz_, cq);
-                };
-                upd3(dxx, a2, a1, a1);
-                if (xi >= 0) pml3(dxx, sh.psix[3] + px, xb, xi, a2, a1, a1);
-                upd3(dyy, a1, a2, a1);
-                if (yi >= 0) pml3(dyy, sh.psiy[3] + py, yb, yi, a1, a2, a1);
-                upd3(dzz, a1, a1, a2);
-                if (fsrow) szz = T(0);
-                if (zi >= 0) pml3(dzz, sh.psiz[3] + pz, zb, zi, a1, a1, a2);
-            } else {
-                sxx = A::mad(sxx, a.dt, dxx);
-                if (xi >= 0) sxx = pml_correct<T, MODE>(sxx, a.dt, dxx, sh.psix[3] + px, a.pml, L, xb, xi);
-                syy = A::mad(syy, a.dt, dyy);
-                if (yi >= 0) syy = pml_correct<T, MODE>(syy, a.dt, dyy, sh.psiy[3] + py, a.pml, L, yb, yi);
-                szz = A::mad(szz, a.dt, dzz);
-                if (fsrow) szz = T(0);
-                if (zi >= 0) szz = pml_correct<T, MODE>(szz, a.dt, dzz, sh.psiz[3] + pz, a.pml, L, zb, zi);
-            }
-            Sxx[o] = sxx; Syy[o] = syy; Szz[o] = szz;
-        }
-        // ---- Sxz: Dx+ Vz, Dz+ Vx
-        {
-            const T am = ADJ ? a.dt : A::mul(a.dt, mxz);
-            sxz = A::mad(sxz, am, dxp.x);
-            if (xi >= 0) sxz = pml_correct<T, MODE>(sxz, am, dxp.x, sh.psix[4] + px, a.pml, L, xb + 3, xi);
-            sxz = A::mad(sxz, am, dzp.x);
-            if (zi >= 0) sxz = pml_correct<T, MODE>(sxz, am, dzp.x, sh.psiz[4] + pz, a.pml, L, zb + 3, zi);
-            Sxz[o] = sxz;
-        }
-        // ---- Syz: Dz+ Vy, Dy+ Vz
-        {
-            const T am = ADJ ? a.dt : A::mul(a.dt, myz);
-            syz = A::mad(syz, am, dzp.y);
-            if (zi >= 0) syz = pml_correct<T, MODE>(syz, am, dzp.y, sh.psiz[5] + pz, a.pml, L, zb + 3, zi);
-            syz = A::mad(syz, am, dyp.x);
-            if (yi >= 0) syz = pml_correct<T, MODE>(syz, am, dyp.x, sh.psiy[4] + py, a.pml, L, yb + 3, yi);
-            Syz[o] = syz;
-        }
-        // ---- Sxy: Dy+ Vx, Dx+ Vy
-        {
-            const T am = ADJ ? a.dt : A::mul(a.dt, mxy);
-            sxy = A::mad(sxy, am, dyp.y);
-            if (yi >= 0) sxy = pml_correct<T, MODE>(sxy, am, dyp.y, sh.psiy[5] + py, a.pml, L, yb + 3, yi);
-            sxy = A::mad(sxy, am, dxp.y);
-            if (xi >= 0) sxy = pml_correct<T, MODE>(sxy, am, dxp.y, sh.psix[5] + px, a.pml, L, xb + 3, xi);
-            Sxy[o] = sxy;
-        }
-#pragma unroll
-        for (int j = 0; j < 15; j++) { qz[j] = qz[j + 1]; qv[j] = qv[j + 1]; }
-        qz[15] = Vz[o + 8 * plane];
-        qv[15] = make_float2(Vx[o + 9 * plane], Vy[o + 9 * plane]);
-        sxx = nsxx; syy = nsyy; szz = nszz; syz = nsyz; sxz = nsxz; sxy = nsxy;
-        l = nl; l2m = nl2m; myz = nmyz; mxz = nmxz; mxy = nmxy;
-    }
-}
-
-// ---------------------------------------------------------------- fast mode with TMA-staged planes
-// The forward velocity step and both stress steps of RSGPU_F32_FAST with every
-// plane tile brought in by TMA (cp.async.bulk.tensor.2d, one thread issuing,
-// completion on an mbarrier per stage) NSTG3 - 1 planes ahead of the plane being
-// computed: the loads in flight no longer depend on registers or resident warps.
-// The z-derivatives still come from 16-plane register windows, refilled by plain
-// loads eight planes ahead.  Same stencils, C-PML and update order as
-// e3d_velocity_fast / e3d_stress_fast.  Every wait is bounded (2 s): on timeout the
-// CTA records RSGPU_ERR_TIMEOUT in the error word and stops.
+// ---------------------------------------------------------------- float: TMA-staged planes
+// The forward velocity step and both stress steps in float (the fast adjoint velocity step
+// runs the forward kernel on work arrays; the exact one forms its operands per tap in
+// e3d_velocity) with every plane tile brought in by TMA (cp.async.bulk.tensor.2d, one
+// thread issuing, completion on an mbarrier per stage) NSTG3 - 1 planes ahead of the plane
+// being computed.  Derivatives that share an axis and a direction run in pairs (f32x2).
+// The z-derivatives come from 16-plane register windows, refilled from the stage.  As in the acoustic kernels (fd3d.cu) a plane's chain is what bounds
+// them: its C-PML memory is requested before the wait for its stage, the factors sit in
+// shared memory, reduced-order z stencils read the windows, whole CTAs choose the reduced
+// x/y stencils, one barrier a plane.  The plane loop is unrolled by two (half the moves of
+// the windows; by four is slower).  Measured on B200 (60 steps of two windows to
+// 221 x 201 x 191, fast): 148 ms with a load and a store per C-PML memory in turn and the
+// reduced stencils as calls, 67 like this, 61 in shorter z-chunks.
+// Every wait is bounded (2 s): on timeout the CTA records RSGPU_ERR_TIMEOUT in the error
+// word and stops.
 constexpr int NSTG3 = 3;
 
 struct VelStageT {
@@ -888,9 +501,11 @@ struct VelStageT {
     float yy[HY][TX3];         // Syy, y halo
     float yz[HY][TX3];         // Syz, y halo
     float pv[6][TY3][TX3];     // Vx, Vy, Vz, Rx, Ry, Rz
+    float up[3][TY3][TX3];     // the windows' refills: Sxz and Syz eight planes up, Szz nine
 };
 struct StrStageT {
     float v[3][HY][WX];        // Vx, Vy, Vz, x and y halos
+    float up[3][TY3][TX3];     // the windows' refills: Vx and Vy nine planes up, Vz eight
     float sv[6][TY3][TX3];     // Sxx, Syy, Szz, Syz, Sxz, Sxy
     float mv[5][TY3][TX3];     // L, L2M, M_yz, M_xz, M_xy (forward only)
 };
@@ -906,34 +521,56 @@ struct TmaSmem {
     Stage st[NSTG3];
     uint64_t bar[NSTG3];
     CoefSet3<float> cs;
+    PmlBlock3<TY3> pml;
 };
 template <typename Stage>
 constexpr size_t tma_smem_bytes() { return sizeof(TmaSmem<Stage>) + 128; }   // + alignment slack
 
 // (a - b) pairs of two arrays with the same tap spacing: sum_k c_k (p[(8+k)s] - p[(7-k)s])
+template <int MODE>
 __device__ __forceinline__ float2 taps_pair2(const float *p, const float *q, int sp, int sq,
-                                             const float (&c2)[NCOEF][2])
+                                             const float (&c2)[NCOEF][2], float d, const Rcp<float> &r)
 {
-    using A2 = Ar2<float, MODE_FAST>;
+    using A2 = Ar2<float, MODE>;
     const float2 *cc = reinterpret_cast<const float2 *>(c2);
     float2 acc = A2::mul(A2::sub(make_float2(p[8 * sp], q[8 * sq]), make_float2(p[7 * sp], q[7 * sq])), cc[0]);
 #pragma unroll
     for (int k = 1; k < NCOEF; k++)
         acc = A2::acc(acc, A2::sub(make_float2(p[(8 + k) * sp], q[(8 + k) * sq]),
                                    make_float2(p[(7 - k) * sp], q[(7 - k) * sq])), cc[k]);
-    return acc;
+    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
 }
-
-// Allocation row of plane iz, padded row iy_alloc (guards included).
-__device__ __forceinline__ int alloc_row(const Shot3D<float> &sh, int iz, int iy_alloc)
+template <int MODE>
+__device__ __forceinline__ float2 taps_pair_reg(const float2 (&q)[16], const float (&c2)[NCOEF][2], float d,
+                                                const Rcp<float> &r)
 {
-    return (GUARD + iz) * sh.rows + iy_alloc;
+    using A2 = Ar2<float, MODE>;
+    const float2 *cc = reinterpret_cast<const float2 *>(c2);
+    float2 acc = A2::mul(A2::sub(q[8], q[7]), cc[0]);
+#pragma unroll
+    for (int k = 1; k < NCOEF; k++) acc = A2::acc(acc, A2::sub(q[8 + k], q[7 - k]), cc[k]);
+    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
+}
+// The same at a plane near an array end: K pairs of the row c (the same for the block).
+template <int MODE>
+__device__ __forceinline__ float2 taps_pair_reg_k(const float2 (&q)[16], int K, const float *c, float d,
+                                                  const Rcp<float> &r)
+{
+    using A2 = Ar2<float, MODE>;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < NCOEF; k++)
+        if (k < K) {
+            const float2 dl = A2::sub(q[8 + k], q[7 - k]), ck = make_float2(c[k], c[k]);
+            acc = k == 0 ? A2::mul(dl, ck) : A2::acc(acc, dl, ck);
+        }
+    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
 }
 
+template <int MODE>
 __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float> a, const CoefSet3<float> *coefs)
 {
     using T = float;
-    constexpr int MODE = MODE_FAST;
     using A = Ar<T, MODE>;
     extern __shared__ unsigned char smraw[];
     TmaSmem<VelStageT> &S =
@@ -941,26 +578,18 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
     stage_shot(shs, a.shots + tl.shot);
-    load_coefs3e(S.cs, coefs);
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    load_coefs3(S.cs, coefs);
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX3 + tx;
+    const int x0 = tl.x0, y0 = tl.y0, L = a.lpml, order = a.order;
     if (tid == 0)
         for (int k = 0; k < NSTG3; k++) mbar_init(&S.bar[k], 1);
+    stage_pml3(S.pml, a.pml, L, x0, y0, a.shots[tl.shot].nxp, a.shots[tl.shot].nyp);
     __syncthreads();
     const Shot3D<T> &sh = shs;
     const CUtensorMap *M = reinterpret_cast<const CUtensorMap *>(a.maps) + (size_t)tl.shot * NMAP_E3;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = tl.x0, y0 = tl.y0;
     const int ix = x0 + tx, iy = y0 + ty;
-    const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch, L = a.lpml, order = a.order;
+    const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch;
     const int plane = (int)sh.plane;
-    const int col = iy * pitch + ix;
-    T *Vx = sh.f[E3_VX], *Vy = sh.f[E3_VY], *Vz = sh.f[E3_VZ];
-    const bool in_grid = ix < nxp && iy < nyp;
-    const int Kxf = kfw(ix, nxp, order), Kxb = kbw(ix, nxp, order);
-    const int Kyf = kfw(iy, nyp, order), Kyb = kbw(iy, nyp, order);
-    int xb = 0, xc = 0, yb = 0, yc = 0;
-    const int xi = in_grid ? xstrip(ix, nxp, L, xb, xc) : -1;
-    const int yi = in_grid ? xstrip(iy, nyp, L, yb, yc) : -1;
     const int z0 = tl.z0, ze = min(z0 + a.zc, nzp);
     // stage k <- plane iz: every box starts on a 16-byte boundary (x0 and x0 + 8 are
     // multiples of 4 floats)
@@ -968,7 +597,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
         VelStageT &g = S.st[k];
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(&S.bar[k], VEL_STAGE_BYTES);
-        const int rh = alloc_row(sh, iz, GUARD + y0), ry = alloc_row(sh, iz, y0);
+        const int rh = alloc_row3(sh, iz, GUARD + y0), ry = alloc_row3(sh, iz, y0);
         tma_load_2d(g.xx, M + VM_SXX, &S.bar[k], x0, rh);
         tma_load_2d(g.xz, M + VM_SXZ, &S.bar[k], x0, rh);
         tma_load_2d(g.xy, M + VM_SXY, &S.bar[k], x0, ry);
@@ -976,9 +605,16 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
         tma_load_2d(g.yz, M + VM_SYZ, &S.bar[k], x0 + GUARD, ry);
 #pragma unroll
         for (int q = 0; q < 6; q++) tma_load_2d(g.pv[q], M + VM_VX + q, &S.bar[k], x0 + GUARD, rh);
+        tma_load_2d(g.up[0], M + SM_SXZ, &S.bar[k], x0 + GUARD, alloc_row3(sh, iz + 8, GUARD + y0));
+        tma_load_2d(g.up[1], M + SM_SYZ, &S.bar[k], x0 + GUARD, alloc_row3(sh, iz + 8, GUARD + y0));
+        tma_load_2d(g.up[2], M + SM_SZZ, &S.bar[k], x0 + GUARD, alloc_row3(sh, iz + 9, GUARD + y0));
     };
     if (tid == 0)
         for (int j = 0; j < NSTG3 - 1 && z0 + j < ze; j++) issue(z0 + j, j);
+    const int col = iy * pitch + ix;
+    const bool in_grid = ix < nxp && iy < nyp;
+    const bool xe = x0 < order || x0 + TX3 > nxp - order - 1, ye = y0 < order || y0 + TY3 > nyp - order - 1;
+    const int xc = in_grid ? strip_col(ix, nxp, L) : -1, yc = in_grid ? strip_col(iy, nyp, L) : -1;
     // z windows: (XZ, YZ) backward (planes z-8..z+7), ZZ forward (z-7..z+8)
     const T *Sxz = sh.f[E3_SXZ], *Syz = sh.f[E3_SYZ], *Szz = sh.f[E3_SZZ];
     float2 qp[16];
@@ -990,91 +626,96 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
         qzz[j] = Szz[(z0 - 7 + j) * plane + col];
     }
     int o = z0 * plane + col;
+#pragma unroll 2
     for (int iz = z0; iz < ze; iz++, o += plane) {
         const int j = iz - z0, k = j % NSTG3;
-        if (tid == 0 && iz + NSTG3 - 1 < ze) issue(iz + NSTG3 - 1, (j + NSTG3 - 1) % NSTG3);
-        // window refills of this iteration, in flight while the stage arrives
-        const float2 nq = make_float2(Sxz[o + 8 * plane], Syz[o + 8 * plane]);
-        const T nzz = Szz[o + 9 * plane];
+        // C-PML memory of this iteration, in flight while the stage arrives
+        const int zc = in_grid ? strip_col(iz, nzp, L) : -1;
+        const int px = (iz * nyp + iy) * 2 * L + xc, py = (iz * 2 * L + yc) * nxp + ix, pz = (zc * nyp + iy) * nxp + ix;
+        T mx[3], my[3], mz[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            mx[q] = my[q] = mz[q] = 0;
+            if (xc >= 0) mx[q] = sh.psix[q][px];
+            if (yc >= 0) my[q] = sh.psiy[q][py];
+            if (zc >= 0) mz[q] = sh.psiz[q][pz];
+        }
+        // every thread is done with the plane before, whose stage is refilled now
         if (!__syncthreads_and(mbar_wait_bounded(&S.bar[k], (uint32_t)(j / NSTG3) & 1u, a.err))) return;
+        if (tid == 0 && iz + NSTG3 - 1 < ze) issue(iz + NSTG3 - 1, (j + NSTG3 - 1) % NSTG3);
         const VelStageT &g = S.st[k];
-        const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
-        int zb = 0, zc = 0;
-        const int zi = in_grid ? xstrip(iz, nzp, L, zb, zc) : -1;
-        const int px = (iz * nyp + iy) * 2 * L + xc;
-        const int py = (iz * 2 * L + yc) * nxp + ix;
-        const int pz = (zc * nyp + iy) * nxp + ix;
         const T *cxx = &g.xx[ty][tx + 8], *cxy = &g.xy[ty + 8][tx + 8], *cxz = &g.xz[ty][tx + 8];
         const T *cyy = &g.yy[ty + 8][tx], *cyz = &g.yz[ty + 8][tx];
-        T dxx = taps3<T, MODE>(cxx - 7, 1, a.cf[0], a.dx, a.rdx);
-        float2 dxq = taps_pair2(cxy - 8, cxz - 8, 1, 1, a.cf2[0]);                  // (Dx- XY, Dx- XZ)
-        float2 dyq = taps_pair2(cxy - 8 * WX, cyz - 8 * TX3, WX, TX3, a.cf2[1]);  // (Dy- XY, Dy- YZ)
-        T dyy = taps3<T, MODE>(cyy - 7 * TX3, TX3, a.cf[1], a.dy, a.rdy);
-        float2 dzq = taps_pair_reg(qp, a.cf2[2]);
-        T dzz = taps3_reg<T, MODE>(qzz, a.cf[2], a.dz, a.rdz);
-        if (Kxf != order) dxx = stencil_k<T, MODE>(cxx, 1, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
-        if (Kxb != order) {
-            dxq.x = stencil_k<T, MODE>(cxy, 1, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
-            dxq.y = stencil_k<T, MODE>(cxz, 1, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
+        T dxx, dyy, dzz;
+        float2 dxq, dyq, dzq;      // (Dx- XY, Dx- XZ), (Dy- XY, Dy- YZ), (Dz- XZ, Dz- YZ)
+        if (!xe) {
+            dxx = taps3<T, MODE>(cxx - 7, 1, a.cf[0], a.dx, a.rdx);
+            dxq = taps_pair2<MODE>(cxy - 8, cxz - 8, 1, 1, a.cf2[0], a.dx, a.rdx);
+        } else {
+            const int Kf = kfw(ix, nxp, order), Kb = kbw(ix, nxp, order);
+            const T *cf = S.cs.cx + Kf * CROW3, *cb = S.cs.cx + Kb * CROW3;
+            dxx = stencil_ki<T, MODE>(cxx, 1, Kf, cf, true, a.dx, a.rdx);
+            dxq.x = stencil_ki<T, MODE>(cxy, 1, Kb, cb, false, a.dx, a.rdx);
+            dxq.y = stencil_ki<T, MODE>(cxz, 1, Kb, cb, false, a.dx, a.rdx);
         }
-        if (Kyb != order) {
-            dyq.x = stencil_k<T, MODE>(cxy, WX, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-            dyq.y = stencil_k<T, MODE>(cyz, TX3, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
+        if (!ye) {
+            dyq = taps_pair2<MODE>(cxy - 8 * WX, cyz - 8 * TX3, WX, TX3, a.cf2[1], a.dy, a.rdy);
+            dyy = taps3<T, MODE>(cyy - 7 * TX3, TX3, a.cf[1], a.dy, a.rdy);
+        } else {
+            const int Kf = kfw(iy, nyp, order), Kb = kbw(iy, nyp, order);
+            const T *cf = S.cs.cy + Kf * CROW3, *cb = S.cs.cy + Kb * CROW3;
+            dyq.x = stencil_ki<T, MODE>(cxy, WX, Kb, cb, false, a.dy, a.rdy);
+            dyq.y = stencil_ki<T, MODE>(cyz, TX3, Kb, cb, false, a.dy, a.rdy);
+            dyy = stencil_ki<T, MODE>(cyy, TX3, Kf, cf, true, a.dy, a.rdy);
         }
-        if (Kyf != order) dyy = stencil_k<T, MODE>(cyy, TX3, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
-        if (Kzb != order) {
-            dzq.x = stencil_z_op<T, MODE, false>(sh, o, plane, Kzb, S.cs.cz + Kzb * CROW3, false, OP_XZ, a.dz, a.rdz);
-            dzq.y = stencil_z_op<T, MODE, false>(sh, o, plane, Kzb, S.cs.cz + Kzb * CROW3, false, OP_YZ, a.dz, a.rdz);
+        const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
+        if (Kzf == order && Kzb == order) {
+            dzq = taps_pair_reg<MODE>(qp, a.cf2[2], a.dz, a.rdz);
+            dzz = taps3_reg<T, MODE>(qzz, a.cf[2], a.dz, a.rdz);
+        } else {
+            dzq = taps_pair_reg_k<MODE>(qp, Kzb, S.cs.cz + Kzb * CROW3, a.dz, a.rdz);
+            dzz = taps_reg_k<T, MODE>(qzz, Kzf, S.cs.cz + Kzf * CROW3, a.dz, a.rdz);
         }
-        if (Kzf != order)
-            dzz = stencil_z_op<T, MODE, false>(sh, o, plane, Kzf, S.cs.cz + Kzf * CROW3, true, OP_ZZ, a.dz, a.rdz);
-        T vx = g.pv[0][ty][tx], vy = g.pv[1][ty][tx], vz = g.pv[2][ty][tx];
-        // ---- Vx: Dx+ XX, Dy- XY, Dz- XZ
-        {
-            const T am = A::mul(a.dt, g.pv[3][ty][tx]);
-            vx = A::mad(vx, am, dxx);
-            if (xi >= 0) vx = pml_correct<T, MODE>(vx, am, dxx, sh.psix[0] + px, a.pml, L, xb + 3, xi);
-            vx = A::mad(vx, am, dyq.x);
-            if (yi >= 0) vx = pml_correct<T, MODE>(vx, am, dyq.x, sh.psiy[0] + py, a.pml, L, yb, yi);
-            vx = A::mad(vx, am, dzq.x);
-            if (zi >= 0) vx = pml_correct<T, MODE>(vx, am, dzq.x, sh.psiz[0] + pz, a.pml, L, zb, zi);
-            Vx[o] = vx;
-        }
-        // ---- Vy: Dx- XY, Dy+ YY, Dz- YZ
-        {
-            const T am = A::mul(a.dt, g.pv[4][ty][tx]);
-            vy = A::mad(vy, am, dxq.x);
-            if (xi >= 0) vy = pml_correct<T, MODE>(vy, am, dxq.x, sh.psix[1] + px, a.pml, L, xb, xi);
-            vy = A::mad(vy, am, dyy);
-            if (yi >= 0) vy = pml_correct<T, MODE>(vy, am, dyy, sh.psiy[1] + py, a.pml, L, yb + 3, yi);
-            vy = A::mad(vy, am, dzq.y);
-            if (zi >= 0) vy = pml_correct<T, MODE>(vy, am, dzq.y, sh.psiz[1] + pz, a.pml, L, zb, zi);
-            Vy[o] = vy;
-        }
-        // ---- Vz: Dx- XZ, Dy- YZ, Dz+ ZZ
-        {
-            const T am = A::mul(a.dt, g.pv[5][ty][tx]);
-            vz = A::mad(vz, am, dxq.y);
-            if (xi >= 0) vz = pml_correct<T, MODE>(vz, am, dxq.y, sh.psix[2] + px, a.pml, L, xb, xi);
-            vz = A::mad(vz, am, dyq.y);
-            if (yi >= 0) vz = pml_correct<T, MODE>(vz, am, dyq.y, sh.psiy[2] + py, a.pml, L, yb, yi);
-            vz = A::mad(vz, am, dzz);
-            if (zi >= 0) vz = pml_correct<T, MODE>(vz, am, dzz, sh.psiz[2] + pz, a.pml, L, zb + 3, zi);
-            Vz[o] = vz;
-        }
+        const T *fz = strip_factors(a.pml, L, iz, nzp, 0);
+        // One field: x, y and z part, each with its C-PML correction; stag: the axis whose
+        // derivative is the forward one (staggered factors)
+        auto field = [&](int f, int stag, T *F, T mod, T dx, T dy, T dz) {
+            T v = g.pv[f][ty][tx];
+            const T am = A::mul(a.dt, mod);
+            v = A::mad(v, am, dx);
+            if (xc >= 0) {
+                const T(&w)[3][TX3] = S.pml.x[stag == 0];
+                v = A::msub(v, am, pml_term<T, MODE>(mx[f], dx, w[0][tx], w[1][tx], w[2][tx]));
+                sh.psix[f][px] = mx[f];
+            }
+            v = A::mad(v, am, dy);
+            if (yc >= 0) {
+                const T(&w)[3][TY3] = S.pml.y[stag == 1];
+                v = A::msub(v, am, pml_term<T, MODE>(my[f], dy, w[0][ty], w[1][ty], w[2][ty]));
+                sh.psiy[f][py] = my[f];
+            }
+            v = A::mad(v, am, dz);
+            if (zc >= 0) {
+                const T *w = fz + (stag == 2) * 3 * L;
+                v = A::msub(v, am, pml_term<T, MODE>(mz[f], dz, __ldg(w), __ldg(w + L), __ldg(w + 2 * L)));
+                sh.psiz[f][pz] = mz[f];
+            }
+            F[o] = v;
+        };
+        field(0, 0, sh.f[E3_VX], g.pv[3][ty][tx], dxx, dyq.x, dzq.x);     // Dx+ XX, Dy- XY, Dz- XZ
+        field(1, 1, sh.f[E3_VY], g.pv[4][ty][tx], dxq.x, dyy, dzq.y);     // Dx- XY, Dy+ YY, Dz- YZ
+        field(2, 2, sh.f[E3_VZ], g.pv[5][ty][tx], dxq.y, dyq.y, dzz);     // Dx- XZ, Dy- YZ, Dz+ ZZ
 #pragma unroll
         for (int q = 0; q < 15; q++) { qp[q] = qp[q + 1]; qzz[q] = qzz[q + 1]; }
-        qp[15] = nq;
-        qzz[15] = nzz;
-        __syncthreads();   // stage k is refilled next iteration
+        qp[15] = make_float2(g.up[0][ty][tx], g.up[1][ty][tx]);
+        qzz[15] = g.up[2][ty][tx];
     }
 }
 
-template <bool ADJ>
+template <int MODE, bool ADJ>
 __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> a, const CoefSet3<float> *coefs)
 {
     using T = float;
-    constexpr int MODE = MODE_FAST;
     using A = Ar<T, MODE>;
     extern __shared__ unsigned char smraw[];
     TmaSmem<StrStageT> &S =
@@ -1082,36 +723,29 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> 
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
     stage_shot(shs, a.shots + tl.shot);
-    load_coefs3e(S.cs, coefs);
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    load_coefs3(S.cs, coefs);
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX3 + tx;
+    const int x0 = tl.x0, y0 = tl.y0, L = a.lpml, order = a.order;
     if (tid == 0)
         for (int k = 0; k < NSTG3; k++) mbar_init(&S.bar[k], 1);
+    stage_pml3(S.pml, a.pml, L, x0, y0, a.shots[tl.shot].nxp, a.shots[tl.shot].nyp);
     __syncthreads();
     const Shot3D<T> &sh = shs;
     const CUtensorMap *M = reinterpret_cast<const CUtensorMap *>(a.maps) + (size_t)tl.shot * NMAP_E3;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = tl.x0, y0 = tl.y0;
     const int ix = x0 + tx, iy = y0 + ty;
-    const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch, L = a.lpml, order = a.order;
+    const int nxp = sh.nxp, nyp = sh.nyp, nzp = sh.nzp, pitch = sh.pitch;
     const int plane = (int)sh.plane;
-    const int col = iy * pitch + ix;
-    const T *Vx = sh.f[E3_VX], *Vy = sh.f[E3_VY], *Vz = sh.f[E3_VZ];
-    T *Sxx = sh.f[E3_SXX], *Syy = sh.f[E3_SYY], *Szz = sh.f[E3_SZZ];
-    T *Syz = sh.f[E3_SYZ], *Sxz = sh.f[E3_SXZ], *Sxy = sh.f[E3_SXY];
-    const bool in_grid = ix < nxp && iy < nyp;
-    const int Kxf = kfw(ix, nxp, order), Kxb = kbw(ix, nxp, order);
-    const int Kyf = kfw(iy, nyp, order), Kyb = kbw(iy, nyp, order);
-    int xb = 0, xc = 0, yb = 0, yc = 0;
-    const int xi = in_grid ? xstrip(ix, nxp, L, xb, xc) : -1;
-    const int yi = in_grid ? xstrip(iy, nyp, L, yb, yc) : -1;
     const int z0 = tl.z0, ze = min(z0 + a.zc, nzp);
     auto issue = [&](int iz, int k) {
         StrStageT &g = S.st[k];
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(&S.bar[k], ADJ ? STR_STAGE_BYTES_ADJ : STR_STAGE_BYTES_FW);
-        const int rh = alloc_row(sh, iz, GUARD + y0), ry = alloc_row(sh, iz, y0);
+        const int rh = alloc_row3(sh, iz, GUARD + y0), ry = alloc_row3(sh, iz, y0);
 #pragma unroll
-        for (int q = 0; q < 3; q++) tma_load_2d(g.v[q], M + SM_VX + q, &S.bar[k], x0, ry);
+        for (int q = 0; q < 3; q++) {
+            tma_load_2d(g.v[q], M + SM_VX + q, &S.bar[k], x0, ry);
+            tma_load_2d(g.up[q], M + VM_VX + q, &S.bar[k], x0 + GUARD, alloc_row3(sh, iz + (q == 2 ? 8 : 9), GUARD + y0));
+        }
 #pragma unroll
         for (int q = 0; q < 6; q++) tma_load_2d(g.sv[q], M + SM_SXX + q, &S.bar[k], x0 + GUARD, rh);
         if (!ADJ) {
@@ -1121,7 +755,12 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> 
     };
     if (tid == 0)
         for (int j = 0; j < NSTG3 - 1 && z0 + j < ze; j++) issue(z0 + j, j);
+    const int col = iy * pitch + ix;
+    const bool in_grid = ix < nxp && iy < nyp;
+    const bool xe = x0 < order || x0 + TX3 > nxp - order - 1, ye = y0 < order || y0 + TY3 > nyp - order - 1;
+    const int xc = in_grid ? strip_col(ix, nxp, L) : -1, yc = in_grid ? strip_col(iy, nyp, L) : -1;
     // z windows: Vz backward (planes z-8..z+7), (Vx, Vy) forward (z-7..z+8)
+    const T *Vx = sh.f[E3_VX], *Vy = sh.f[E3_VY], *Vz = sh.f[E3_VZ];
     T qz[16];
     float2 qv[16];
 #pragma unroll
@@ -1131,110 +770,137 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> 
         qv[j] = make_float2(Vx[oj], Vy[oj]);
     }
     int o = z0 * plane + col;
+#pragma unroll 2
     for (int iz = z0; iz < ze; iz++, o += plane) {
         const int j = iz - z0, k = j % NSTG3;
-        if (tid == 0 && iz + NSTG3 - 1 < ze) issue(iz + NSTG3 - 1, (j + NSTG3 - 1) % NSTG3);
-        const T nz = Vz[o + 8 * plane];
-        const float2 nv = make_float2(Vx[o + 9 * plane], Vy[o + 9 * plane]);
+        const int zc = in_grid ? strip_col(iz, nzp, L) : -1;
+        const int px = (iz * nyp + iy) * 2 * L + xc, py = (iz * 2 * L + yc) * nxp + ix, pz = (zc * nyp + iy) * nxp + ix;
+        T mx[3], my[3], mz[3];     // memory arrays 3, 4 and 5 of each face pair
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            mx[q] = my[q] = mz[q] = 0;
+            if (xc >= 0) mx[q] = sh.psix[3 + q][px];
+            if (yc >= 0) my[q] = sh.psiy[3 + q][py];
+            if (zc >= 0) mz[q] = sh.psiz[3 + q][pz];
+        }
         if (!__syncthreads_and(mbar_wait_bounded(&S.bar[k], (uint32_t)(j / NSTG3) & 1u, a.err))) return;
+        if (tid == 0 && iz + NSTG3 - 1 < ze) issue(iz + NSTG3 - 1, (j + NSTG3 - 1) % NSTG3);
         const StrStageT &g = S.st[k];
-        const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
-        int zb = 0, zc = 0;
-        const int zi = in_grid ? xstrip(iz, nzp, L, zb, zc) : -1;
-        const int px = (iz * nyp + iy) * 2 * L + xc;
-        const int py = (iz * 2 * L + yc) * nxp + ix;
-        const int pz = (zc * nyp + iy) * nxp + ix;
         const T *cvx = &g.v[0][ty + 8][tx + 8], *cvy = &g.v[1][ty + 8][tx + 8], *cvz = &g.v[2][ty + 8][tx + 8];
-        T dxx = taps3<T, MODE>(cvx - 8, 1, a.cf[0], a.dx, a.rdx);
-        float2 dxp = taps_pair2(cvz - 7, cvy - 7, 1, 1, a.cf2[0]);                  // (Dx+ Vz, Dx+ Vy)
-        T dyy = taps3<T, MODE>(cvy - 8 * WX, WX, a.cf[1], a.dy, a.rdy);
-        float2 dyp = taps_pair2(cvz - 7 * WX, cvx - 7 * WX, WX, WX, a.cf2[1]);     // (Dy+ Vz, Dy+ Vx)
-        T dzz = taps3_reg<T, MODE>(qz, a.cf[2], a.dz, a.rdz);
-        float2 dzp = taps_pair_reg(qv, a.cf2[2]);                                   // (Dz+ Vx, Dz+ Vy)
-        if (Kxb != order) dxx = stencil_k<T, MODE>(cvx, 1, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
-        if (Kxf != order) {
-            dxp.x = stencil_k<T, MODE>(cvz, 1, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
-            dxp.y = stencil_k<T, MODE>(cvy, 1, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
+        T dxx, dyy, dzz;
+        float2 dxp, dyp, dzp;      // (Dx+ Vz, Dx+ Vy), (Dy+ Vz, Dy+ Vx), (Dz+ Vx, Dz+ Vy)
+        if (!xe) {
+            dxx = taps3<T, MODE>(cvx - 8, 1, a.cf[0], a.dx, a.rdx);
+            dxp = taps_pair2<MODE>(cvz - 7, cvy - 7, 1, 1, a.cf2[0], a.dx, a.rdx);
+        } else {
+            const int Kf = kfw(ix, nxp, order), Kb = kbw(ix, nxp, order);
+            const T *cf = S.cs.cx + Kf * CROW3, *cb = S.cs.cx + Kb * CROW3;
+            dxx = stencil_ki<T, MODE>(cvx, 1, Kb, cb, false, a.dx, a.rdx);
+            dxp.x = stencil_ki<T, MODE>(cvz, 1, Kf, cf, true, a.dx, a.rdx);
+            dxp.y = stencil_ki<T, MODE>(cvy, 1, Kf, cf, true, a.dx, a.rdx);
         }
-        if (Kyb != order) dyy = stencil_k<T, MODE>(cvy, WX, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-        if (Kyf != order) {
-            dyp.x = stencil_k<T, MODE>(cvz, WX, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
-            dyp.y = stencil_k<T, MODE>(cvx, WX, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
+        if (!ye) {
+            dyy = taps3<T, MODE>(cvy - 8 * WX, WX, a.cf[1], a.dy, a.rdy);
+            dyp = taps_pair2<MODE>(cvz - 7 * WX, cvx - 7 * WX, WX, WX, a.cf2[1], a.dy, a.rdy);
+        } else {
+            const int Kf = kfw(iy, nyp, order), Kb = kbw(iy, nyp, order);
+            const T *cf = S.cs.cy + Kf * CROW3, *cb = S.cs.cy + Kb * CROW3;
+            dyy = stencil_ki<T, MODE>(cvy, WX, Kb, cb, false, a.dy, a.rdy);
+            dyp.x = stencil_ki<T, MODE>(cvz, WX, Kf, cf, true, a.dy, a.rdy);
+            dyp.y = stencil_ki<T, MODE>(cvx, WX, Kf, cf, true, a.dy, a.rdy);
         }
-        if (Kzb != order) dzz = stencil_k<T, MODE>(Vz + o, plane, Kzb, S.cs.cz + Kzb * CROW3, false, a.dz, a.rdz);
-        if (Kzf != order) {
-            dzp.x = stencil_k<T, MODE>(Vx + o, plane, Kzf, S.cs.cz + Kzf * CROW3, true, a.dz, a.rdz);
-            dzp.y = stencil_k<T, MODE>(Vy + o, plane, Kzf, S.cs.cz + Kzf * CROW3, true, a.dz, a.rdz);
+        const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
+        if (Kzf == order && Kzb == order) {
+            dzz = taps3_reg<T, MODE>(qz, a.cf[2], a.dz, a.rdz);
+            dzp = taps_pair_reg<MODE>(qv, a.cf2[2], a.dz, a.rdz);
+        } else {
+            dzz = taps_reg_k<T, MODE>(qz, Kzb, S.cs.cz + Kzb * CROW3, a.dz, a.rdz);
+            dzp = taps_pair_reg_k<MODE>(qv, Kzf, S.cs.cz + Kzf * CROW3, a.dz, a.rdz);
         }
-        T sxx = g.sv[0][ty][tx], syy = g.sv[1][ty][tx], szz = g.sv[2][ty][tx];
-        T syz = g.sv[3][ty][tx], sxz = g.sv[4][ty][tx], sxy = g.sv[5][ty][tx];
+        const T *fz0 = strip_factors(a.pml, L, iz, nzp, 0);
+        // the derivative term of memory array 3 + f along an axis, its memory updated
+        auto term_x = [&](int f, T d) {
+            const T(&w)[3][TX3] = S.pml.x[f != 0];
+            const T c = pml_term<T, MODE>(mx[f], d, w[0][tx], w[1][tx], w[2][tx]);
+            sh.psix[3 + f][px] = mx[f];
+            return c;
+        };
+        auto term_y = [&](int f, T d) {
+            const T(&w)[3][TY3] = S.pml.y[f != 0];
+            const T c = pml_term<T, MODE>(my[f], d, w[0][ty], w[1][ty], w[2][ty]);
+            sh.psiy[3 + f][py] = my[f];
+            return c;
+        };
+        auto term_z = [&](int f, T d) {
+            const T *w = fz0 + (f != 0) * 3 * L;
+            const T c = pml_term<T, MODE>(mz[f], d, __ldg(w), __ldg(w + L), __ldg(w + 2 * L));
+            sh.psiz[3 + f][pz] = mz[f];
+            return c;
+        };
         // ---- normal stresses
         {
+            T sxx = g.sv[0][ty][tx], syy = g.sv[1][ty][tx], szz = g.sv[2][ty][tx];
             const bool fsrow = sh.fs && iz == L;
-            if (!ADJ) {
-                const T l = g.mv[0][ty][tx], l2m = g.mv[1][ty][tx];
-                const T a2 = A::mul(a.dt, l2m), a1 = A::mul(a.dt, l);
-                auto upd3 = [&](T d, T cxx_, T cyy_, T czz_) {
-                    sxx = A::mad(sxx, cxx_, d); syy = A::mad(syy, cyy_, d); szz = A::mad(szz, czz_, d);
-                };
-                auto pml3 = [&](T d, T *psi, int base, int idx, T cxx_, T cyy_, T czz_) {
-                    const T tA = __ldg(a.pml + (base + PT_A) * L + idx), tB = __ldg(a.pml + (base + PT_B) * L + idx),
-                            tC = __ldg(a.pml + (base + PT_C) * L + idx);
-                    const T p = A::mad(A::mul(tB, *psi), tA, d);
-                    *psi = p;
-                    const T cq = A::mad(p, tC, d);
-                    sxx = A::msub(sxx, cxx_, cq); syy = A::msub(syy, cyy_, cq); szz = A::msub(szz, czz_, cq);
-                };
-                upd3(dxx, a2, a1, a1);
-                if (xi >= 0) pml3(dxx, sh.psix[3] + px, xb, xi, a2, a1, a1);
-                upd3(dyy, a1, a2, a1);
-                if (yi >= 0) pml3(dyy, sh.psiy[3] + py, yb, yi, a1, a2, a1);
-                upd3(dzz, a1, a1, a2);
-                if (fsrow) szz = T(0);
-                if (zi >= 0) pml3(dzz, sh.psiz[3] + pz, zb, zi, a1, a1, a2);
-            } else {
-                sxx = A::mad(sxx, a.dt, dxx);
-                if (xi >= 0) sxx = pml_correct<T, MODE>(sxx, a.dt, dxx, sh.psix[3] + px, a.pml, L, xb, xi);
-                syy = A::mad(syy, a.dt, dyy);
-                if (yi >= 0) syy = pml_correct<T, MODE>(syy, a.dt, dyy, sh.psiy[3] + py, a.pml, L, yb, yi);
-                szz = A::mad(szz, a.dt, dzz);
-                if (fsrow) szz = T(0);
-                if (zi >= 0) szz = pml_correct<T, MODE>(szz, a.dt, dzz, sh.psiz[3] + pz, a.pml, L, zb, zi);
+            // adjoint: each normal stress takes its own derivative, without the moduli
+            const T a1 = ADJ ? a.dt : A::mul(a.dt, g.mv[0][ty][tx]), a2 = ADJ ? a.dt : A::mul(a.dt, g.mv[1][ty][tx]);
+            sxx = A::mad(sxx, a2, dxx);
+            if (!ADJ) { syy = A::mad(syy, a1, dxx); szz = A::mad(szz, a1, dxx); }
+            if (xc >= 0) {
+                const T c = term_x(0, dxx);
+                sxx = A::msub(sxx, a2, c);
+                if (!ADJ) { syy = A::msub(syy, a1, c); szz = A::msub(szz, a1, c); }
             }
-            Sxx[o] = sxx; Syy[o] = syy; Szz[o] = szz;
+            syy = A::mad(syy, a2, dyy);
+            if (!ADJ) { sxx = A::mad(sxx, a1, dyy); szz = A::mad(szz, a1, dyy); }
+            if (yc >= 0) {
+                const T c = term_y(0, dyy);
+                syy = A::msub(syy, a2, c);
+                if (!ADJ) { sxx = A::msub(sxx, a1, c); szz = A::msub(szz, a1, c); }
+            }
+            szz = A::mad(szz, a2, dzz);
+            if (!ADJ) { sxx = A::mad(sxx, a1, dzz); syy = A::mad(syy, a1, dzz); }
+            if (fsrow) szz = T(0);
+            if (zc >= 0) {
+                const T c = term_z(0, dzz);
+                szz = A::msub(szz, a2, c);
+                if (!ADJ) { sxx = A::msub(sxx, a1, c); syy = A::msub(syy, a1, c); }
+            }
+            sh.f[E3_SXX][o] = sxx; sh.f[E3_SYY][o] = syy; sh.f[E3_SZZ][o] = szz;
         }
         // ---- Sxz: Dx+ Vz, Dz+ Vx
         {
+            T v = g.sv[4][ty][tx];
             const T am = ADJ ? a.dt : A::mul(a.dt, g.mv[3][ty][tx]);
-            sxz = A::mad(sxz, am, dxp.x);
-            if (xi >= 0) sxz = pml_correct<T, MODE>(sxz, am, dxp.x, sh.psix[4] + px, a.pml, L, xb + 3, xi);
-            sxz = A::mad(sxz, am, dzp.x);
-            if (zi >= 0) sxz = pml_correct<T, MODE>(sxz, am, dzp.x, sh.psiz[4] + pz, a.pml, L, zb + 3, zi);
-            Sxz[o] = sxz;
+            v = A::mad(v, am, dxp.x);
+            if (xc >= 0) v = A::msub(v, am, term_x(1, dxp.x));
+            v = A::mad(v, am, dzp.x);
+            if (zc >= 0) v = A::msub(v, am, term_z(1, dzp.x));
+            sh.f[E3_SXZ][o] = v;
         }
         // ---- Syz: Dz+ Vy, Dy+ Vz
         {
+            T v = g.sv[3][ty][tx];
             const T am = ADJ ? a.dt : A::mul(a.dt, g.mv[2][ty][tx]);
-            syz = A::mad(syz, am, dzp.y);
-            if (zi >= 0) syz = pml_correct<T, MODE>(syz, am, dzp.y, sh.psiz[5] + pz, a.pml, L, zb + 3, zi);
-            syz = A::mad(syz, am, dyp.x);
-            if (yi >= 0) syz = pml_correct<T, MODE>(syz, am, dyp.x, sh.psiy[4] + py, a.pml, L, yb + 3, yi);
-            Syz[o] = syz;
+            v = A::mad(v, am, dzp.y);
+            if (zc >= 0) v = A::msub(v, am, term_z(2, dzp.y));
+            v = A::mad(v, am, dyp.x);
+            if (yc >= 0) v = A::msub(v, am, term_y(1, dyp.x));
+            sh.f[E3_SYZ][o] = v;
         }
         // ---- Sxy: Dy+ Vx, Dx+ Vy
         {
+            T v = g.sv[5][ty][tx];
             const T am = ADJ ? a.dt : A::mul(a.dt, g.mv[4][ty][tx]);
-            sxy = A::mad(sxy, am, dyp.y);
-            if (yi >= 0) sxy = pml_correct<T, MODE>(sxy, am, dyp.y, sh.psiy[5] + py, a.pml, L, yb + 3, yi);
-            sxy = A::mad(sxy, am, dxp.y);
-            if (xi >= 0) sxy = pml_correct<T, MODE>(sxy, am, dxp.y, sh.psix[5] + px, a.pml, L, xb + 3, xi);
-            Sxy[o] = sxy;
+            v = A::mad(v, am, dyp.y);
+            if (yc >= 0) v = A::msub(v, am, term_y(2, dyp.y));
+            v = A::mad(v, am, dxp.y);
+            if (xc >= 0) v = A::msub(v, am, term_x(2, dxp.y));
+            sh.f[E3_SXY][o] = v;
         }
 #pragma unroll
         for (int q = 0; q < 15; q++) { qz[q] = qz[q + 1]; qv[q] = qv[q + 1]; }
-        qz[15] = nz;
-        qv[15] = nv;
-        __syncthreads();   // stage k is refilled next iteration
+        qz[15] = g.up[2][ty][tx];
+        qv[15] = make_float2(g.up[0][ty][tx], g.up[1][ty][tx]);
     }
 }
 
@@ -1265,9 +931,10 @@ __device__ void inject_set(const Shot3D<T> &sh, const InjRec3<T> &pl, T dt, int 
         const T *Mod = sh.m[ME_RX + k];
         for (int q = threadIdx.x; q < pl.ninj; q += blockDim.x) {
             const long long p = pl.inj_pt[q];
+            const int c0 = pl.inj_start[q], c1 = pl.inj_start[q + 1];
             T v = F[p];
             const T dm = A::mul(dt, Mod[p]);
-            for (int c = pl.inj_start[q]; c < pl.inj_start[q + 1]; c++) {
+            for (int c = c0; c < c1; c++) {
                 const T w = pl.wav[(long long)pl.inj_trace[c] * pl.nt + it];
                 v = A::add(v, A::mul(A::mul(A::mul(A::mul(dm, w), pl.inj_w[3 * c]), pl.inj_w[3 * c + 1]),
                                      pl.inj_w[3 * c + 2]));
@@ -1327,54 +994,39 @@ __device__ void record_set(const Shot3D<T> &sh, const InjRec3<T> &pl, int it)
 }
 
 template <typename T, int MODE>
-__global__ void inject_record_e3d(const Shot3D<T> *shots, const InjRec3<T> *plans, int nsets, T dt, int it0)
+__global__ void __launch_bounds__(1024) inject_record_e3d(const Shot3D<T> *shots, const InjRec3<T> *plans, int nsets, T dt, int it0)
 {
     const Shot3D<T> &sh = shots[blockIdx.x];
     const InjRec3<T> *pl = plans + (long long)blockIdx.x * nsets;
     const int it = pl[0].rev ? pl[0].nt - 1 - it0 : it0;
     for (int k = 0; k < nsets; k++) {
-        if (k) __syncthreads();
+        // sets that inject into the same field add in set order
+        bool same = false;
+        for (int q = 0; q < k; q++) same = same || pl[q].kind_inj == pl[k].kind_inj;
+        if (same) __syncthreads();
         inject_set<T, MODE>(sh, pl[k], dt, it);
     }
     __syncthreads();
     for (int k = 0; k < nsets; k++) record_set<T, MODE>(sh, pl[k], it);
 }
 
-template <bool ADJ>
-cudaError_t step_e3_fast(int half, const void *args, const void *coefs, int grid, cudaStream_t st)
+// The float half-steps on TMA-staged planes.
+template <int MODE, bool ADJ>
+cudaError_t step_e3_tma(int half, const Step3DArgs<float> &a, const CoefSet3<float> *coefs, int grid, cudaStream_t st)
 {
-    const Step3DArgs<float> &a = *reinterpret_cast<const Step3DArgs<float> *>(args);
     const dim3 block(TX3, TY3);
-    if (a.maps && !(half == 0 && ADJ)) {
-        // TMA-staged planes (the adjoint velocity step differentiates work arrays formed
-        // from five fields and keeps the register-staged kernel)
-        if (half == 0) {
-            auto k = e3d_velocity_tma;
-            static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                              (int)tma_smem_bytes<VelStageT>());
-            if (e != cudaSuccess) return e;
-            k<<<grid, block, tma_smem_bytes<VelStageT>(), st>>>(a, (const CoefSet3<float> *)coefs);
-        } else {
-            auto k = e3d_stress_tma<ADJ>;
-            static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                              (int)tma_smem_bytes<StrStageT>());
-            if (e != cudaSuccess) return e;
-            k<<<grid, block, tma_smem_bytes<StrStageT>(), st>>>(a, (const CoefSet3<float> *)coefs);
-        }
-        return cudaGetLastError();
-    }
     if (half == 0) {
-        auto k = e3d_velocity_fast<ADJ>;
+        auto k = e3d_velocity_tma<MODE>;
         static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          (int)sizeof(VelSmemF));
+                                                          (int)tma_smem_bytes<VelStageT>());
         if (e != cudaSuccess) return e;
-        k<<<grid, block, sizeof(VelSmemF), st>>>(a, (const CoefSet3<float> *)coefs);
+        k<<<grid, block, tma_smem_bytes<VelStageT>(), st>>>(a, coefs);
     } else {
-        auto k = e3d_stress_fast<ADJ>;
+        auto k = e3d_stress_tma<MODE, ADJ>;
         static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          (int)sizeof(StrSmemF));
+                                                          (int)tma_smem_bytes<StrStageT>());
         if (e != cudaSuccess) return e;
-        k<<<grid, block, sizeof(StrSmemF), st>>>(a, (const CoefSet3<float> *)coefs);
+        k<<<grid, block, tma_smem_bytes<StrStageT>(), st>>>(a, coefs);
     }
     return cudaGetLastError();
 }
@@ -1383,21 +1035,32 @@ template <typename T, int MODE, bool ADJ>
 cudaError_t step_e3(int half, const void *args, const void *coefs, int grid, cudaStream_t st)
 {
     const Step3DArgs<T> &a = *reinterpret_cast<const Step3DArgs<T> *>(args);
+    const CoefSet3<T> *cs = (const CoefSet3<T> *)coefs;
     const dim3 block(TX3, TY3);
-    if (half == 0) {
-        auto k = e3d_velocity<T, MODE, ADJ>;
-        static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          (int)sizeof(VelSmem<T>));
-        if (e != cudaSuccess) return e;
-        k<<<grid, block, sizeof(VelSmem<T>), st>>>(a, (const CoefSet3<T> *)coefs);
-    } else {
-        auto k = e3d_stress<T, MODE, ADJ>;
-        static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          (int)sizeof(StrSmem<T>));
-        if (e != cudaSuccess) return e;
-        k<<<grid, block, sizeof(StrSmem<T>), st>>>(a, (const CoefSet3<T> *)coefs);
+    if constexpr (std::is_same<T, float>::value) {
+        // the exact adjoint velocity step forms its operands per tap (the fast one is a
+        // forward step on work arrays, which the exact one's memory budget does not hold)
+        if (!(half == 0 && ADJ)) return step_e3_tma<MODE, ADJ>(half, a, cs, grid, st);
     }
-    return cudaGetLastError();
+    if constexpr (!(std::is_same<T, float>::value && MODE == MODE_FAST)) {
+        if (half == 0) {
+            if constexpr (ADJ || !std::is_same<T, float>::value) {
+                auto k = e3d_velocity<T, MODE, ADJ>;
+                static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                                  (int)sizeof(VelSmem<T>));
+                if (e != cudaSuccess) return e;
+                k<<<grid, block, sizeof(VelSmem<T>), st>>>(a, cs);
+            }
+        } else if constexpr (!std::is_same<T, float>::value) {
+            auto k = e3d_stress<T, MODE, ADJ>;
+            static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                              (int)sizeof(StrSmem<T>));
+            if (e != cudaSuccess) return e;
+            k<<<grid, block, sizeof(StrSmem<T>), st>>>(a, cs);
+        }
+        return cudaGetLastError();
+    }
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace
@@ -1411,7 +1074,8 @@ cudaError_t launch_step_e3d(int prec, int half, int adj, const void *args, const
     if (prec == PREC_F32_EXACT)
         return adj ? step_e3<float, MODE_IEEE, true>(half, args, coefs, grid, st)
                    : step_e3<float, MODE_IEEE, false>(half, args, coefs, grid, st);
-    return adj ? step_e3_fast<true>(half, args, coefs, grid, st) : step_e3_fast<false>(half, args, coefs, grid, st);
+    return adj ? step_e3<float, MODE_FAST, true>(half, args, coefs, grid, st)
+               : step_e3<float, MODE_FAST, false>(half, args, coefs, grid, st);
 }
 
 // Work arrays of the adjoint velocity step (FAST arithmetic), the operands that
@@ -1458,17 +1122,17 @@ cudaError_t launch_work_e3d(const void *desc, int nshots, cudaStream_t st)
 }
 
 cudaError_t launch_injrec_e3d(int prec, const void *shots, const void *plans, int nshots, int nsets, double dt,
-                              int it, cudaStream_t st)
+                              int it, int threads, cudaStream_t st)
 {
     if (prec == PREC_F64)
-        inject_record_e3d<double, MODE_IEEE><<<nshots, 256, 0, st>>>((const Shot3D<double> *)shots,
+        inject_record_e3d<double, MODE_IEEE><<<nshots, threads, 0, st>>>((const Shot3D<double> *)shots,
                                                                      (const InjRec3<double> *)plans, nsets, dt, it);
     else if (prec == PREC_F32_EXACT)
-        inject_record_e3d<float, MODE_IEEE><<<nshots, 256, 0, st>>>((const Shot3D<float> *)shots,
+        inject_record_e3d<float, MODE_IEEE><<<nshots, threads, 0, st>>>((const Shot3D<float> *)shots,
                                                                     (const InjRec3<float> *)plans, nsets, (float)dt,
                                                                     it);
     else
-        inject_record_e3d<float, MODE_FAST><<<nshots, 256, 0, st>>>((const Shot3D<float> *)shots,
+        inject_record_e3d<float, MODE_FAST><<<nshots, threads, 0, st>>>((const Shot3D<float> *)shots,
                                                                     (const InjRec3<float> *)plans, nsets, (float)dt,
                                                                     it);
     return cudaGetLastError();

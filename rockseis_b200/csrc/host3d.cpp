@@ -58,6 +58,43 @@ Plan3D::~Plan3D()
     if (stream && stream != shared_stream) cudaStreamDestroy(stream);
 }
 
+// Planes per z-chunk: the division of the tallest window into chunks of 20 to 40 planes that
+// the model below gives the least time.  A chunk costs its planes plus the fill of the
+// register windows (about CHUNK_FILL planes), a launch as many chunks as fall on one SM and
+// about CHUNK_TAIL more, for the ragged end (blocks at the array ends and in the strips take
+// longer).  Measured on B200: two elastic windows to 192x196x191 67.3 ms whole, 62.6 in 48
+// planes, 61.4 in 32; four acoustic ones to 226x235x221 59.6 in 56, 58.7 in 37; a gradient of
+// one 161x151x141 window 100 ms in 71, 94 in 36, 85 in 29, 92 in 24; one exact 151x141x131
+// window 20 ms a call in 64, 17 in 33, 15 in 27, 14 in 22.
+int Plan3D::pick_zchunk(const rsgpu_shot *s) const
+{
+    constexpr int CHUNK_FILL = 8, CHUNK_TAIL = 2, ZC_MIN = 20, ZC_MAX = 40;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+        cudaGetLastError();
+        return 64;
+    }
+    int nz = 0;
+    for (int i = 0; i < nshots; i++) nz = std::max(nz, s[i].nz + 2 * cfg.lpml);
+    int best = nz;
+    double best_cost = -1;
+    for (int n = 1; (nz + n - 1) / n >= std::min(ZC_MIN, nz); n++) {
+        const int z = (nz + n - 1) / n;
+        if (z > ZC_MAX) continue;
+        long long blocks = 0;
+        for (int i = 0; i < nshots; i++) {
+            const long long bx = (s[i].nx + 2 * cfg.lpml + TX3 - 1) / TX3;
+            const long long by = (s[i].ny + 2 * cfg.lpml + rows_per_block() - 1) / rows_per_block();
+            blocks += bx * by * ((s[i].nz + 2 * cfg.lpml + z - 1) / z);
+        }
+        const double cost = (double)((blocks + sms - 1) / sms + CHUNK_TAIL) * (z + CHUNK_FILL);
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = z; }
+        if (z == 1) break;
+    }
+    return best;
+}
+
 rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, const ShotSets *sets)
 {
     if (!c || !s || ns < 1) { set_error("null config/shots or nshots < 1"); return RSGPU_ERR_ARG; }
@@ -140,7 +177,7 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
     prec = c->precision;
     nshots = ns;
     es = prec == PREC_F64 ? 8 : 4;
-    zc = c->zchunk > 0 ? c->zchunk : 64;      // planes per z-chunk
+    zc = c->zchunk > 0 ? c->zchunk : pick_zchunk(s);
     if (shared_stream) stream = shared_stream;
     else CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     const int lp = cfg.lpml;
@@ -265,6 +302,9 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
         }
     }
     std::vector<SetTables> tabs(nps);
+    size_t most = 0;
+    for (int j = 0; j < nps; j++) most = std::max({most, inj_pt[j].size(), rec_pt[j].size()});
+    injrec_nt = injrec_threads(most);
     for (int j = 0; j < nps; j++) {
         SetTables &t = tabs[j];
         t.ip = take(inj_pt[j].size() * 8);
@@ -359,7 +399,7 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
     for (int i = 0; i < ns; i++) {
         const Layout3D &L = shots[i];
         for (int z0 = 0; z0 < L.nzp; z0 += zc)
-            for (int y0 = 0; y0 < L.nyp; y0 += TY3)
+            for (int y0 = 0; y0 < L.nyp; y0 += rows_per_block())
                 for (int x0 = 0; x0 < L.nxp; x0 += TX3) tiles.push_back({i, x0, y0, z0});
     }
     ntiles = (int)tiles.size();
@@ -374,12 +414,12 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
     const size_t ir_bytes = prec == PREC_F64 ? sizeof(InjRec3<double>) : sizeof(InjRec3<float>);
     const size_t m_shots = 0, m_ir = rup3(ns * shot_bytes, 256), m_tiles = rup3(m_ir + (size_t)nps * ir_bytes, 256);
     const size_t m_coef = rup3(m_tiles + tiles.size() * sizeof(Tile3D), 256);
-    // fast mode: the tensor maps of the TMA-staged kernels
-    const bool tma = prec == PREC_F32_FAST;
+    // float: the tensor maps of the TMA-staged kernels
+    const bool tma = prec != PREC_F64;
     const int nmap = phys == PHYS_E3D ? NMAP_E3 : NMAP_A3;
     const size_t m_maps = rup3(m_coef + coefs.size(), 256);
     // adjoint velocity through work arrays: a second set of shot descriptors and maps
-    const bool wpass = tma && adjoint_steps && phys == PHYS_E3D;
+    const bool wpass = prec == PREC_F32_FAST && adjoint_steps && phys == PHYS_E3D;
     const size_t m_maps_w = rup3(m_maps + (tma ? (size_t)ns * nmap * sizeof(CUtensorMap) : 0), 256);
     const size_t m_shots_w = rup3(m_maps_w + (wpass ? (size_t)ns * NMAP_E3 * sizeof(CUtensorMap) : 0), 256);
     const size_t m_wdesc = rup3(m_shots_w + (wpass ? ns * shot_bytes : 0), 256);
@@ -405,9 +445,9 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
         // VM_* then SM_* (rsgpu_3d.h)
         // acoustic: AM_* (rsgpu_3d.h)
         const Spec spec_a[NMAP_A3] = {
-            {A3_P, false, WX3, HY3}, {A3_VX, false, TX3, TY3}, {A3_VY, false, TX3, TY3}, {A3_VZ, false, TX3, TY3},
-            {M3_RX, true, TX3, TY3}, {M3_RY, true, TX3, TY3}, {M3_RZ, true, TX3, TY3},
-            {A3_VX, false, WX3, TY3}, {A3_VY, false, TX3, HY3}, {A3_P, false, TX3, TY3}, {M3_L, true, TX3, TY3}};
+            {A3_P, false, WX3, TYA + 16}, {A3_VX, false, TX3, TYA}, {A3_VY, false, TX3, TYA}, {A3_VZ, false, TX3, TYA},
+            {M3_RX, true, TX3, TYA}, {M3_RY, true, TX3, TYA}, {M3_RZ, true, TX3, TYA},
+            {A3_VX, false, WX3, TYA}, {A3_VY, false, TX3, TYA + 16}, {A3_P, false, TX3, TYA}, {M3_L, true, TX3, TYA}};
         const Spec spec_e[NMAP_E3] = {
             {E3_SXX, false, WX3, TY3}, {E3_SXZ, false, WX3, TY3}, {E3_SXY, false, WX3, HY3},
             {E3_SYY, false, TX3, HY3}, {E3_SYZ, false, TX3, HY3},
@@ -590,20 +630,20 @@ rsgpu_status Plan3D::step(int it)
         if ((e = launch_work_e3d(d_wdesc, nshots, stream)) != cudaSuccess) goto fail;
         if ((e = launch_step_e3d(prec, 0, 0, wargs, d_coefs, ntiles, stream)) != cudaSuccess) goto fail;
         if ((e = launch_step_e3d(prec, 1, 1, args, d_coefs, ntiles, stream)) != cudaSuccess) goto fail;
-        if ((e = launch_injrec_e3d(prec, d_shots, d_injrec, nshots, nsets, cfg.dt, it, stream)) != cudaSuccess) goto fail;
+        if ((e = launch_injrec_e3d(prec, d_shots, d_injrec, nshots, nsets, cfg.dt, it, injrec_nt, stream)) != cudaSuccess) goto fail;
         launches += 4;
         return RSGPU_OK;
     }
     if (phys == PHYS_E3D) {
         if ((e = launch_step_e3d(prec, 0, adjoint_steps, args, d_coefs, ntiles, stream)) != cudaSuccess) goto fail;
         if ((e = launch_step_e3d(prec, 1, adjoint_steps, args, d_coefs, ntiles, stream)) != cudaSuccess) goto fail;
-        if ((e = launch_injrec_e3d(prec, d_shots, d_injrec, nshots, nsets, cfg.dt, it, stream)) != cudaSuccess) goto fail;
+        if ((e = launch_injrec_e3d(prec, d_shots, d_injrec, nshots, nsets, cfg.dt, it, injrec_nt, stream)) != cudaSuccess) goto fail;
         launches += 3;
         return RSGPU_OK;
     }
     if ((e = launch_step_3d(prec, PHYS_A3D, 0, args, d_coefs, ntiles, stream)) != cudaSuccess) goto fail;
     if ((e = launch_step_3d(prec, PHYS_A3D, 1, args, d_coefs, ntiles, stream)) != cudaSuccess) goto fail;
-    if ((e = launch_injrec_3d(prec, d_shots, d_injrec, nshots, cfg.dt, it, stream)) != cudaSuccess) goto fail;
+    if ((e = launch_injrec_3d(prec, d_shots, d_injrec, nshots, cfg.dt, it, injrec_nt, stream)) != cudaSuccess) goto fail;
     launches += 3;
     return RSGPU_OK;
 fail:
@@ -634,8 +674,8 @@ rsgpu_status Plan3D::set_recording(bool on)
 rsgpu_status Plan3D::inject_record_only(int it)
 {
     if (it < 0 || it >= cfg.nt) { set_error("step %d outside [0,%d)", it, cfg.nt); return RSGPU_ERR_ARG; }
-    cudaError_t e = phys == PHYS_E3D ? launch_injrec_e3d(prec, d_shots, d_injrec, nshots, nsets, cfg.dt, it, stream)
-                                     : launch_injrec_3d(prec, d_shots, d_injrec, nshots, cfg.dt, it, stream);
+    cudaError_t e = phys == PHYS_E3D ? launch_injrec_e3d(prec, d_shots, d_injrec, nshots, nsets, cfg.dt, it, injrec_nt, stream)
+                                     : launch_injrec_3d(prec, d_shots, d_injrec, nshots, cfg.dt, it, injrec_nt, stream);
     if (e != cudaSuccess) { set_error("3D kernel launch failed: %s", cudaGetErrorString(e)); return RSGPU_ERR_CUDA; }
     launches += 1;
     return RSGPU_OK;

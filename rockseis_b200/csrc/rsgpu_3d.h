@@ -14,6 +14,7 @@ namespace rsgpu {
 
 constexpr int TX3 = 32;   // x columns per CTA (one warp row)
 constexpr int TY3 = 8;    // y rows per CTA
+constexpr int TYA = 16;   // y rows per CTA of the acoustic float kernels (two a thread)
 constexpr int WX3 = TX3 + 16, HY3 = TY3 + 16;   // a tile with its 8-cell x or y halos
 
 enum { A3_P = 0, A3_VX = 1, A3_VY = 2, A3_VZ = 3 };
@@ -39,8 +40,8 @@ struct Shot3D {
 
 // Tensor maps of the acoustic 3D TMA kernels (FAST), per shot, over whole pitched
 // arrays like the elastic ones:
-//   velocity: P {48 x 24} (x and y halos); Vx, Vy, Vz, Rx, Ry, Rz {32 x 8}
-//   stress:   Vx {48 x 8} (x halo); Vy {32 x 24} (y halo); P, L {32 x 8}
+//   velocity: P {48 x 32} (x and y halos); Vx, Vy, Vz, Rx, Ry, Rz {32 x 16}
+//   stress:   Vx {48 x 16} (x halo); Vy {32 x 32} (y halo); P, L {32 x 16}
 enum {
     AM_PH = 0, AM_VX, AM_VY, AM_VZ, AM_RX, AM_RY, AM_RZ, AM_VXH, AM_VYH, AM_P, AM_L,
     NMAP_A3
@@ -135,8 +136,8 @@ cudaError_t launch_step_e3d(int prec, int half, int adj, const void *args, const
 // holds source set k and receiver set k; every set is injected, then every set
 // recorded.
 cudaError_t launch_injrec_e3d(int prec, const void *shots, const void *plans, int nshots, int nsets, double dt,
-                              int it, cudaStream_t st);
+                              int it, int threads, cudaStream_t st);
 cudaError_t launch_injrec_3d(int prec, const void *shots, const void *plans, int nshots, double dt, int it,
-                             cudaStream_t st);
+                             int threads, cudaStream_t st);
 
 }  // namespace rsgpu

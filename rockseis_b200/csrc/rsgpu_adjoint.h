@@ -180,8 +180,9 @@ cudaError_t launch_residual_e2d(int prec, int acc, const void *desc, int nshots,
 // The 3D correlations: one thread per (x, y) column and CORR_ZC planes, blockIdx.z the
 // shot and the chunk.  A column's planes are independent but for a few values carried from
 // plane to plane; whole columns left most of the chip idle (one 121 x 111 x 101 elastic
-// window: 60 blocks, 620 us a launch, against 137 us in chunks).
-constexpr int CORR_ZC = 16;
+// window: 60 blocks, 620 us a launch; 137 us in chunks of 16, and with 8 the whole
+// gradient of two such windows takes 85 ms against 87).
+constexpr int CORR_ZC = 8;
 inline int corr_chunks(int nzmax) { return (nzmax + CORR_ZC - 1) / CORR_ZC; }
 cudaError_t launch_corr_rtm_a3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, int nzmax, int nhx,
                                 int nhy, int nhz, cudaStream_t st);

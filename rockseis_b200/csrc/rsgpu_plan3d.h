@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include "rsgpu.h"
 #include "rsgpu_kernels.h"
+#include "rsgpu_3d.h"
 #include "rsgpu_plan.h"
 
 namespace rsgpu {
@@ -56,6 +57,7 @@ public:
     Rcp<float> rcp_of(int axis, float) const { return rcp[axis]; }
     Rcp<double> rcp_of(int, double) const { return {0}; }
     int prec = 0, phys = PHYS_A3D, nshots = 0, es = 4, zc = 64, ntiles = 0;
+    int injrec_nt = 64;                  // threads of the injection/recording CTAs
     int nsets = 1;                             // InjRec3 entries per shot (elastic: MAXSETS)
     std::vector<Layout3D> shots;
     std::vector<size_t> rec_pt_offsets;        // [shot*nsets + set]: arena offset of the receiver points (long long, -1 off grid)
@@ -76,6 +78,8 @@ public:
     const char *param_base(int i, int k) const;
 
 private:
+    int rows_per_block() const { return phys == PHYS_A3D && prec != PREC_F64 ? TYA : TY3; }
+    int pick_zchunk(const rsgpu_shot *s) const;   // planes per z-chunk for this batch
     struct SetTables {
         size_t ip, is, it, iw, rp, rw;
         int ninj, nrec;

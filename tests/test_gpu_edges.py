@@ -3,14 +3,16 @@
 EXACT float must equal the oracle bit for bit: divisors of every kind (a power of two,
 one whose reciprocal formula fails its check) at amplitudes down to subnormals, C-PML
 strips and array ends off every vector and tile boundary, more sources and receivers than
-threads.
+threads, z-chunks of every remainder.  The elastic 3D float kernels, which the oracle does
+not cover, are held to the FP64 propagator's other kernels.
 """
 import numpy as np
 import pytest
 
-from rockseis_b200 import abi
-from rockseis_b200.rockseis import ModellingAcoustic2D, ModellingElastic2D
-from tests.cases import Case2D
+from rockseis_b200 import abi, synth
+from rockseis_b200.rockseis import Data3D, ModelElastic3D, ModellingAcoustic2D, ModellingElastic2D, Plan
+from tests.cases import Case2D, rel_l2
+from tests.test_gpu_modelling_3d import Case3D
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +53,41 @@ def test_more_points_than_threads(require_gpu):
     c = Case2D(abi.ACOUSTIC2D, nx=121, nz=41, nt=70, scoord=sc, nrec=1200, rdx=0.97)
     c.src.data *= np.linspace(0.5, 1.5, len(sc), dtype=np.float32)[:, None]
     assert np.array_equal(traces(c), c.oracle_traces())
+
+
+@pytest.mark.parametrize("zchunk", [0, 1, 2, 3, 16])
+@pytest.mark.parametrize("nx,ny,nz,lpml,order", [(33, 9, 8, 5, 8), (20, 26, 21, 3, 6), (24, 20, 34, 7, 8)])
+def test_acoustic3d_chunks_and_strips_bitwise(require_gpu, nx, ny, nz, lpml, order, zchunk):
+    c = Case3D(nx=nx, ny=ny, nz=nz, lpml=lpml, order=order, nt=60, fs=nz % 2, scoord=(103.3, 41.9, 32.2))
+    assert np.array_equal(c.gpu(zchunk=zchunk), c.oracle())
+
+
+def elastic3d(prec, nx, ny, nz, lpml, fs, zchunk=0, order=8, nt=60):
+    rng = np.random.default_rng(3)
+    m = ModelElastic3D(nx, ny, nz, lpml, 10.0, 10.0, 10.0, 0.0, 0.0, 0.0, fs, prec)
+    m.createModel()
+    vp = (1800 + 1200 * np.linspace(0, 1, nz)[:, None, None] * rng.uniform(0.9, 1.1, (nz, ny, nx))).astype(np.float32)
+    m.Vp[:], m.Vs[:], m.R[:] = vp, vp / np.float32(1.8), 310 * vp.astype(np.float64) ** 0.25
+    src = Data3D(1, nt, 1e-3, 0.0, prec)
+    src.scoords[:] = [[5.3 * nx, 4.9 * ny, 32.2]]
+    src.data[:] = 1e9 * synth.ricker(nt, 1e-3, 25.0)[None, :]
+    src.makeMap(m, 0)
+    rec = Data3D(12, nt, 1e-3, 0.0, prec)
+    rec.gcoords[:] = np.stack([np.linspace(25.0, 10.0 * (nx - 3), 12), np.linspace(15.5, 10.0 * (ny - 3), 12), np.full(12, 14.2)], 1)
+    rec.setField(abi.VZ)
+    rec.makeMap(m, 1)
+    p = Plan([m], [src], [rec], order, prec, zchunk=zchunk)
+    p.run()
+    return p.read_traces(0).astype(np.float64)
+
+
+@pytest.mark.parametrize("nx,ny,nz,lpml,fs,order", [(34, 21, 23, 7, 0, 8), (25, 33, 16, 10, 1, 8), (40, 18, 19, 5, 0, 5)])
+def test_elastic3d_float_against_fp64(require_gpu, nx, ny, nz, lpml, fs, order):
+    # float propagation over 60 steps of 18 derivatives; both float arithmetics were 2e-7 to 2e-6
+    # off the FP64 propagator (whose kernels are other ones) at these sizes
+    want = elastic3d(abi.F64, nx, ny, nz, lpml, fs, order=order)
+    exact = elastic3d(abi.F32_EXACT, nx, ny, nz, lpml, fs, order=order)
+    assert rel_l2(exact, want) < 1e-5
+    assert rel_l2(elastic3d(abi.F32_FAST, nx, ny, nz, lpml, fs, order=order), want) < 1e-5
+    for zchunk in (1, 3, 16):
+        assert np.array_equal(elastic3d(abi.F32_EXACT, nx, ny, nz, lpml, fs, zchunk, order), exact)
