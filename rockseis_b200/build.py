@@ -66,7 +66,7 @@ def _compile(src: str, obj: str, verbose: bool) -> None:
 # One small translation unit each so nvcc compiles them in parallel.
 VARIANTS_2D = [("f32x", "float", "MODE_IEEE"), ("f32f", "float", "MODE_FAST"), ("f64", "double", "MODE_IEEE")]
 TILES_2D = [(64, 32, 4, 1), (64, 64, 4, 1), (32, 32, 4, 1), (32, 16, 4, 1), (32, 32, 2, 1), (64, 32, 2, 1),
-            (32, 32, 2, 6), (32, 32, 2, 8), (64, 32, 2, 3), (32, 16, 2, 8)]
+            (32, 32, 2, 6), (32, 32, 2, 8), (64, 32, 2, 3), (32, 16, 2, 8), (32, 16, 1, 4)]
 TILES_F64 = (0, 3)   # FP64 oracle propagator: two shapes
 
 

@@ -299,7 +299,10 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
     if (shared_stream) stream = shared_stream;
     else CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
 
-    tilecfg = (c->tile >= 0 && c->tile < tile_count_2d()) ? c->tile : default_tile();
+    long long tiles32x16 = 0;
+    for (int i = 0; i < ns; i++)
+        tiles32x16 += (long long)((s[i].nx + 2 * c->lpml + 31) / 32) * ((s[i].nz + 2 * c->lpml + 15) / 16);
+    tilecfg = (c->tile >= 0 && c->tile < tile_count_2d()) ? c->tile : default_tile_2d(prec, phys, tiles32x16);
     // the FP64 oracle propagator is built for two tile shapes only
     if (prec == PREC_F64 && tilecfg != TILECFG_64x32 && tilecfg != TILECFG_32x16) tilecfg = TILECFG_64x32;
     const TileShape ts = tile_shape_2d(tilecfg);
@@ -639,15 +642,31 @@ void Plan::fill_desc(unsigned char *sd, unsigned char *irp, const ShotLayout &L,
     std::memcpy(irp, &r, sizeof r);
 }
 
-int Plan::default_tile() const
+int default_tile_2d(int prec, int phys, long long tiles)
 {
-    // Float: 32x16 tiles of 64 threads at eight CTAs per SM, whose 128-register budget holds
-    // the edge stencils and the C-PML memory (102 to 118 registers, no spills); the 80
-    // registers of 32x32 at six spill.  Measured on B200 beside it: four rows a thread at
-    // one CTA (one 541x341 acoustic shot 38 ms against 31, a 16-shot gradient 147 against
-    // 145), ten CTAs at 96 registers (sixteen elastic shots 84.6 against 77.5, the gradient
-    // 140 against 145).
-    return prec == PREC_F64 ? TILECFG_64x32 : TILECFG_FLOAT;
+    // Float: 32x16 tiles, of 64 threads with two rows each (102 to 118 registers, ten tiles
+    // on an SM) or of 128 with one (80 to 90 registers, six).  Two rows share loads and
+    // coefficients between them, one has half the chain.  So one row where a launch is a
+    // round of six, and past one round of ten up to where the rate counts; measured on B200
+    // by tiles an SM, us a step of two rows | one:
+    //   FAST acoustic  2: 10.6 | 8.7   8.3: 13.8 | 15.2   10.7: 19.0 | 17.1   19: 25.3 | 25.0   40: 34.4 | 36.0
+    //   FAST elastic   2: 15.6 | 12.0  9.5: 21.6 | 22.9   10.7: 27.6 | 24.8   19: 37.3 | 37.8   40: 58.0 | 62.3
+    //   EXACT acoustic 2: 11.2 | 8.7   8.3: 16.5 | 16.3   16: 20.5 | 19.2     28: 37.9 | 36.9   40: 36.4 | 38.0
+    //   EXACT elastic  2: 18.0 | 12.8  8.3: 25.2 | 22.4   16: 35.6 | 30.5     40: 77 | 69       82: 147 | 133
+    // Measured beside them: 32x32 of two rows (spills), four rows a thread at one CTA (one
+    // 541x341 acoustic shot 38 ms against 31 with two rows), 32x8 of one row (elastic 64.3
+    // at 40 an SM).
+    if (prec == PREC_F64) return TILECFG_64x32;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+        cudaGetLastError();
+        return TILECFG_FLOAT2;
+    }
+    const double per_sm = (double)tiles / sms;
+    if (prec == PREC_F32_EXACT)
+        return phys == PHYS_E2D || per_sm <= 32 ? TILECFG_FLOAT1 : TILECFG_FLOAT2;
+    return per_sm <= 6 || (per_sm > 10 && per_sm <= 18) ? TILECFG_FLOAT1 : TILECFG_FLOAT2;
 }
 
 rsgpu_status Plan::reset()

@@ -100,7 +100,8 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     const int sf = shot->src_field, rf = shot->rec_field;
     if (sf != RSGPU_PRESSURE && sf != RSGPU_VX && sf != RSGPU_VZ) { set_error("bad source field"); return RSGPU_ERR_ARG; }
     if (shot->nrec > 0 && rf != RSGPU_PRESSURE && rf != RSGPU_VX && rf != RSGPU_VZ) { set_error("bad receiver field"); return RSGPU_ERR_ARG; }
-    const int cfgi = (cfg->tile >= 0 && cfg->tile < tile_count_2d()) ? cfg->tile : TILECFG_FLOAT;
+    const int cfgi = (cfg->tile >= 0 && cfg->tile < tile_count_2d()) ? cfg->tile
+                     : default_tile_2d(prec, PHYS_A2D, (long long)((nxp + 31) / 32) * ((nzp + 15) / 16));
     const TileShape ts = tile_shape_2d(cfgi);
 
     // ---- injection plan (contributions in the reference's loop order) and receivers
@@ -166,7 +167,7 @@ extern "C" rsgpu_status rsgpu_modelling_a2d_noalloc(const rsgpu_config *cfg, con
     // What the limit does not count: the bytes that the vector layout of the C-PML memory
     // adds to the strips themselves, and half the tile table of the default shape (it was
     // counted with tiles of twice the height)
-    size_t widened = cfgi == TILECFG_FLOAT && cfg->tile != TILECFG_FLOAT ? tiles.size() / 2 * sizeof(Tile2D) : 0;
+    size_t widened = cfgi != cfg->tile ? tiles.size() / 2 * sizeof(Tile2D) : 0;
     auto take_psi = [&](size_t strips, size_t bytes) {
         widened += rup(bytes, 256) - rup(strips, 256);
         return take(bytes);

@@ -13,7 +13,9 @@ enum { PREC_F32_EXACT = 0, PREC_F32_FAST = 1, PREC_F64 = 2 };
 struct TileShape { int tx, tz, rz, minb; };
 TileShape tile_shape_2d(int cfg);
 int tile_count_2d();
-enum { TILECFG_64x32 = 0, TILECFG_32x16 = 3, TILECFG_FLOAT = 9 };
+enum { TILECFG_64x32 = 0, TILECFG_32x16 = 3, TILECFG_FLOAT2 = 9, TILECFG_FLOAT1 = 10 };   // the float defaults: rows a thread
+// The tile shape of a plan that names none: tiles = its 32x16 tiles.
+int default_tile_2d(int prec, int phys, long long tiles);
 
 // One half-step (half = 0 velocity, 1 stress) of every tile in args.
 // maps: per shot NMAP2D CUtensorMaps of the halo-loaded fields; err: device error word.

@@ -17,9 +17,10 @@ from tests.test_gpu_modelling_3d import Case3D
 pytestmark = pytest.mark.gpu
 
 
-def traces(c):
+def traces(c, tile=-1):
     cls = ModellingAcoustic2D if c.physics == abi.ACOUSTIC2D else ModellingElastic2D
     mod = cls(c.model, c.src, c.order, 1)
+    mod.tile = tile
     (mod.setRecP if c.rec.field == abi.PRESSURE else mod.setRecVx)(c.rec)
     assert mod.run() == 1
     return c.rec.data
@@ -37,14 +38,15 @@ def test_exact_division(require_gpu, physics, dx, amp):
     assert np.array_equal(traces(c), want)
 
 
+@pytest.mark.parametrize("tile", [9, 10])   # the two float defaults: two rows a thread, one row
 @pytest.mark.parametrize("physics", [abi.ACOUSTIC2D, abi.ELASTIC2D])
 @pytest.mark.parametrize("nx,nz,lpml,order,fs", [(15, 16, 1, 8, 0), (38, 17, 3, 8, 1), (31, 33, 5, 5, 0), (64, 16, 13, 8, 1),
                                                  (7, 40, 30, 8, 0), (121, 9, 20, 2, 0)])
-def test_strips_and_edges_bitwise(require_gpu, physics, nx, nz, lpml, order, fs):
+def test_strips_and_edges_bitwise(require_gpu, physics, nx, nz, lpml, order, fs, tile):
     # strips that start and end off the vectors' boundaries, and tiles that hold both of an axis' ends
     c = Case2D(physics, nx=nx, nz=nz, lpml=lpml, order=order, fs=fs, nt=90, scoord=(10.0 * nx / 2 + 3.3, 23.7),
                rfield=abi.VX if physics == abi.ELASTIC2D else abi.PRESSURE)
-    assert np.array_equal(traces(c), c.oracle_traces())
+    assert np.array_equal(traces(c, tile), c.oracle_traces())
 
 
 def test_more_points_than_threads(require_gpu):
