@@ -31,6 +31,7 @@
 #include "rsgpu_internal.h"
 #include "rsgpu_kernels.h"
 #include "pdl.cuh"
+#include "smem_limit.h"
 
 namespace rsgpu {
 
@@ -1337,45 +1338,26 @@ static __global__ void set_counter(int *it_dev, int value)
 }
 
 // ---------------------------------------------------------------- launchers
-template <typename K>
-static cudaError_t set_smem(K k, size_t bytes)
-{
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 template <typename T, int MODE, int TX, int TZ, int RZ, int MINB>
 cudaError_t launch_2d_cfg(int physics, int half, int flags, const Step2DArgs<T> &a, const CoefSet<T> *coefs,
                           const CUtensorMap *maps, int *err, int grid, cudaStream_t st)
 {
     using G = Geo2D<T, TX, TZ, RZ>;
-    const bool adj = (flags & LAUNCH_ADJ) != 0;
+    auto launch = [&](auto k, size_t smem, SmemLimit &limit) {
+        const cudaError_t e = limit.raise(k, smem);
+        return e != cudaSuccess ? e : launch_pdl(k, grid, G::NT, smem, st, a, coefs, maps, err);
+    };
+    static SmemLimit av, as, ev, es, ev_adj, es_adj;
     if (physics == PHYS_A2D) {
-        if (half == 0) {
-            static const cudaError_t e = set_smem(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, SmemA2V<T, TX, TZ>::bytes());
-            if (e != cudaSuccess) return e;
-            return launch_pdl(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, SmemA2V<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
-        } else {
-            static const cudaError_t e = set_smem(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, SmemA2S<T, TX, TZ>::bytes());
-            if (e != cudaSuccess) return e;
-            return launch_pdl(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, grid, G::NT, SmemA2S<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
-        }
-    } else {
-        if (half == 0) {
-            static const cudaError_t e0 = set_smem(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, SmemE2V<T, TX, TZ, false>::bytes());
-            static const cudaError_t e1 = set_smem(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, SmemE2V<T, TX, TZ, true>::bytes());
-            if (e0 != cudaSuccess) return e0;
-            if (e1 != cudaSuccess) return e1;
-            if (adj) return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, SmemE2V<T, TX, TZ, true>::bytes(), st, a, coefs, maps, err);
-            else return launch_pdl(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, SmemE2V<T, TX, TZ, false>::bytes(), st, a, coefs, maps, err);
-        } else {
-            static const cudaError_t e0 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, SmemE2S<T, TX, TZ>::bytes());
-            static const cudaError_t e1 = set_smem(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, SmemE2S<T, TX, TZ>::bytes());
-            if (e0 != cudaSuccess) return e0;
-            if (e1 != cudaSuccess) return e1;
-            if (adj) return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, grid, G::NT, SmemE2S<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
-            else return launch_pdl(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, grid, G::NT, SmemE2S<T, TX, TZ>::bytes(), st, a, coefs, maps, err);
-        }
+        if (half == 0) return launch(a2d_velocity<T, MODE, TX, TZ, RZ, MINB>, SmemA2V<T, TX, TZ>::bytes(), av);
+        return launch(a2d_stress<T, MODE, TX, TZ, RZ, MINB>, SmemA2S<T, TX, TZ>::bytes(), as);
     }
+    if (flags & LAUNCH_ADJ) {
+        if (half == 0) return launch(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, true>, SmemE2V<T, TX, TZ, true>::bytes(), ev_adj);
+        return launch(e2d_stress<T, MODE, TX, TZ, RZ, MINB, true>, SmemE2S<T, TX, TZ>::bytes(), es_adj);
+    }
+    if (half == 0) return launch(e2d_velocity<T, MODE, TX, TZ, RZ, MINB, false>, SmemE2V<T, TX, TZ, false>::bytes(), ev);
+    return launch(e2d_stress<T, MODE, TX, TZ, RZ, MINB, false>, SmemE2S<T, TX, TZ>::bytes(), es);
 }
 
 }  // namespace rsgpu

@@ -608,12 +608,14 @@ cudaError_t step3(int half, const void *args, const void *coefs, int grid, cudaS
     if constexpr (std::is_same<T, float>::value) {
         if (half == 0) {
             constexpr size_t sm = a3_smem_bytes<A3VelStage>();
-            static const cudaError_t e = cudaFuncSetAttribute(a3d_velocity_tma<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            static SmemLimit limit;
+            const cudaError_t e = limit.raise(a3d_velocity_tma<MODE>, sm);
             if (e != cudaSuccess) return e;
             a3d_velocity_tma<MODE><<<grid, block, sm, st>>>(a, (const CoefSet3<float> *)coefs);
         } else {
             constexpr size_t sm = a3_smem_bytes<A3StrStage>();
-            static const cudaError_t e = cudaFuncSetAttribute(a3d_stress_tma<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            static SmemLimit limit;
+            const cudaError_t e = limit.raise(a3d_stress_tma<MODE>, sm);
             if (e != cudaSuccess) return e;
             a3d_stress_tma<MODE><<<grid, block, sm, st>>>(a, (const CoefSet3<float> *)coefs);
         }

@@ -1017,14 +1017,14 @@ cudaError_t step_e3_tma(int half, const Step3DArgs<float> &a, const CoefSet3<flo
     const dim3 block(TX3, TY3);
     if (half == 0) {
         auto k = e3d_velocity_tma<MODE>;
-        static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          (int)tma_smem_bytes<VelStageT>());
+        static SmemLimit limit;
+        const cudaError_t e = limit.raise(k, tma_smem_bytes<VelStageT>());
         if (e != cudaSuccess) return e;
         k<<<grid, block, tma_smem_bytes<VelStageT>(), st>>>(a, coefs);
     } else {
         auto k = e3d_stress_tma<MODE, ADJ>;
-        static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          (int)tma_smem_bytes<StrStageT>());
+        static SmemLimit limit;
+        const cudaError_t e = limit.raise(k, tma_smem_bytes<StrStageT>());
         if (e != cudaSuccess) return e;
         k<<<grid, block, tma_smem_bytes<StrStageT>(), st>>>(a, coefs);
     }
@@ -1046,15 +1046,15 @@ cudaError_t step_e3(int half, const void *args, const void *coefs, int grid, cud
         if (half == 0) {
             if constexpr (ADJ || !std::is_same<T, float>::value) {
                 auto k = e3d_velocity<T, MODE, ADJ>;
-                static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                                  (int)sizeof(VelSmem<T>));
+                static SmemLimit limit;
+                const cudaError_t e = limit.raise(k, sizeof(VelSmem<T>));
                 if (e != cudaSuccess) return e;
                 k<<<grid, block, sizeof(VelSmem<T>), st>>>(a, cs);
             }
         } else if constexpr (!std::is_same<T, float>::value) {
             auto k = e3d_stress<T, MODE, ADJ>;
-            static const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                              (int)sizeof(StrSmem<T>));
+            static SmemLimit limit;
+            const cudaError_t e = limit.raise(k, sizeof(StrSmem<T>));
             if (e != cudaSuccess) return e;
             k<<<grid, block, sizeof(StrSmem<T>), st>>>(a, cs);
         }
