@@ -504,6 +504,7 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
             put_real(ro[j].fac, rec[j].fac);
         }
     }
+    staging.release();
     if (c->pml) std::memcpy(&tabs[o_pml - tab0], c->pml, (size_t)12 * lp * es);
     else pml_tables_host(lp, cfg.dt, prec, &tabs[o_pml - tab0]);
     CU(cudaMemcpyAsync(A + tab0, tabs.data(), tabs.size(), cudaMemcpyHostToDevice, stream));

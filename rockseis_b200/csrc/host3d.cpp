@@ -386,6 +386,7 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
                 if ((st = put_real(L.rfack[k], fac)) != RSGPU_OK) return st;
             }
     }
+    staging.release();
     {
         std::vector<unsigned char> tab((size_t)12 * lp * es);
         if (c->pml) std::memcpy(tab.data(), c->pml, tab.size());

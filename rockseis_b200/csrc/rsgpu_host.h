@@ -33,7 +33,8 @@ bool encode_field_map_host(void *map, void *base, int prec, int pitch, int rows,
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t st);
 void dev_free(void *p, cudaStream_t st);
 // Device staging memory of an upload: as large as the largest array wanted, or null where
-// that much is not free.  Released in its stream's order.
+// that much is not free.  Released in its stream's order, and before anything else is
+// allocated: a plan needs no more room than its own arrays.
 struct Staging {
     void *p = nullptr;
     size_t bytes = 0;
@@ -41,7 +42,7 @@ struct Staging {
     explicit Staging(cudaStream_t s) : st(s) {}
     Staging(const Staging &) = delete;
     Staging &operator=(const Staging &) = delete;
-    ~Staging() { dev_free(p, st); }
+    ~Staging() { release(); }
     void want(size_t b) { bytes = b > bytes ? b : bytes; }
     void get()
     {
@@ -49,6 +50,11 @@ struct Staging {
             cudaGetLastError();
             p = nullptr;
         }
+    }
+    void release()
+    {
+        dev_free(p, st);
+        p = nullptr;
     }
 };
 // Return the cached blocks of the current device's pool to the driver.
