@@ -134,10 +134,10 @@ __global__ void __launch_bounds__(256) corr_rtm_a2d(const Corr2D<T> *desc, int n
 // 3D: image[ihz][ihy][ihx][iz][iy][ix] += Pfw(x-h) * Padj(x+h) (lib/rtm.cpp:601-637);
 // one thread per (x, y) column, marching z.
 template <typename T, bool EXACT, typename G>
-__global__ void __launch_bounds__(256) corr_rtm_a3d(const Corr3D<T> *desc, int nc, int nhx, int nhy, int nhz)
+__global__ void __launch_bounds__(256) corr_rtm_a3d(const Corr3D<T> *desc, CorrChunks ch, int nhx, int nhy, int nhz)
 {
-    const Corr3D<T> c = desc[blockIdx.z / nc];
-    const int zs = blockIdx.z % nc * CORR_ZC;
+    const Corr3D<T> c = desc[blockIdx.z / ch.count];
+    const int zs = blockIdx.z % ch.count * ch.planes;
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= c.nx || iy >= c.ny) return;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(256) corr_rtm_a3d(const Corr3D<T> *desc, int n
                 G *img = (G *)c.img + (((long long)ihz * nhy + ihy) * nhx + ihx) * n3 + (long long)iy * c.nx + ix;
                 const T *ws = c.wsp + (long long)(iy - hy + L) * c.pitch + (ix - hx + L);
                 const T *wr = c.wrp + (long long)(iy + hy + L) * c.pitch + (ix + hx + L);
-                const int z0 = max(max(hz, -hz), zs), z1 = min(c.nz - max(hz, -hz), zs + CORR_ZC);
+                const int z0 = max(max(hz, -hz), zs), z1 = min(c.nz - max(hz, -hz), zs + ch.planes);
                 for (int iz = z0; iz < z1; iz++) {
                     const T a = ws[(long long)(iz - hz + L) * c.plane], b = wr[(long long)(iz + hz + L) * c.plane];
                     G *o = img + (long long)iz * c.nx * c.ny;
@@ -442,16 +442,16 @@ __global__ void __launch_bounds__(256) corr_fwi_e2d(const Corr2DE<T> *desc, T dx
 // takes the adjoint Vz of the cell at y-1 with Rz of the cell at z-1 (as written
 // there); it is reproduced as it is.
 template <typename T, bool EXACT, typename G>
-__global__ void __launch_bounds__(256) corr_fwi_a3d(const Corr3DF<T> *desc, int nc, T dx, T dy, T dz)
+__global__ void __launch_bounds__(256) corr_fwi_a3d(const Corr3DF<T> *desc, CorrChunks ch, T dx, T dy, T dz)
 {
-    const Corr3DF<T> c = desc[blockIdx.z / nc];
-    const int zs = blockIdx.z % nc * CORR_ZC;
+    const Corr3DF<T> c = desc[blockIdx.z / ch.count];
+    const int zs = blockIdx.z % ch.count * ch.planes;
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix < 1 || iy < 1 || ix >= c.nx || iy >= c.ny) return;
     const long long P = c.pitch, PL = c.plane;
     const int L = c.lpml;
-    for (int iz = max(1, zs); iz < min(c.nz, zs + CORR_ZC); iz++) {
+    for (int iz = max(1, zs); iz < min(c.nz, zs + ch.planes); iz++) {
         const long long q = (long long)(iz + L) * PL + (long long)(iy + L) * P + (ix + L);
         const long long u = ((long long)iz * c.ny + iy) * c.nx + ix;
         const T ws = c.wsp[q];
@@ -804,15 +804,15 @@ cudaError_t launch_corr_rtm_a2d(int prec, int acc, const void *desc, int nshots,
 cudaError_t launch_corr_rtm_a3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, int nzmax, int nhx,
                                 int nhy, int nhz, cudaStream_t st)
 {
-    const int nc = corr_chunks(nzmax);
-    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots * nc);
-    if (prec == PREC_F64) corr_rtm_a3d<double, true, double><<<grid, block, 0, st>>>((const Corr3D<double> *)desc, nc, nhx, nhy, nhz);
+    const CorrChunks ch = corr_chunks(nshots, nzmax);
+    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots * ch.count);
+    if (prec == PREC_F64) corr_rtm_a3d<double, true, double><<<grid, block, 0, st>>>((const Corr3D<double> *)desc, ch, nhx, nhy, nhz);
     else if (acc == ACC_F64) {
-        if (prec == PREC_F32_EXACT) corr_rtm_a3d<float, true, double><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, nc, nhx, nhy, nhz);
-        else corr_rtm_a3d<float, false, double><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, nc, nhx, nhy, nhz);
+        if (prec == PREC_F32_EXACT) corr_rtm_a3d<float, true, double><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, ch, nhx, nhy, nhz);
+        else corr_rtm_a3d<float, false, double><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, ch, nhx, nhy, nhz);
     } else {
-        if (prec == PREC_F32_EXACT) corr_rtm_a3d<float, true, float><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, nc, nhx, nhy, nhz);
-        else corr_rtm_a3d<float, false, float><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, nc, nhx, nhy, nhz);
+        if (prec == PREC_F32_EXACT) corr_rtm_a3d<float, true, float><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, ch, nhx, nhy, nhz);
+        else corr_rtm_a3d<float, false, float><<<grid, block, 0, st>>>((const Corr3D<float> *)desc, ch, nhx, nhy, nhz);
     }
     return cudaGetLastError();
 }
@@ -820,16 +820,16 @@ cudaError_t launch_corr_rtm_a3d(int prec, int acc, const void *desc, int nshots,
 cudaError_t launch_corr_fwi_a3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, int nzmax, double dx,
                                 double dy, double dz, cudaStream_t st)
 {
-    const int nc = corr_chunks(nzmax);
-    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots * nc);
+    const CorrChunks ch = corr_chunks(nshots, nzmax);
+    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots * ch.count);
     if (prec == PREC_F64)
-        corr_fwi_a3d<double, true, double><<<grid, block, 0, st>>>((const Corr3DF<double> *)desc, nc, dx, dy, dz);
+        corr_fwi_a3d<double, true, double><<<grid, block, 0, st>>>((const Corr3DF<double> *)desc, ch, dx, dy, dz);
     else if (prec == PREC_F32_EXACT) {
-        if (acc == ACC_F64) corr_fwi_a3d<float, true, double><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, nc, (float)dx, (float)dy, (float)dz);
-        else corr_fwi_a3d<float, true, float><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, nc, (float)dx, (float)dy, (float)dz);
+        if (acc == ACC_F64) corr_fwi_a3d<float, true, double><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, ch, (float)dx, (float)dy, (float)dz);
+        else corr_fwi_a3d<float, true, float><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, ch, (float)dx, (float)dy, (float)dz);
     } else {
-        if (acc == ACC_F64) corr_fwi_a3d<float, false, double><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, nc, (float)dx, (float)dy, (float)dz);
-        else corr_fwi_a3d<float, false, float><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, nc, (float)dx, (float)dy, (float)dz);
+        if (acc == ACC_F64) corr_fwi_a3d<float, false, double><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, ch, (float)dx, (float)dy, (float)dz);
+        else corr_fwi_a3d<float, false, float><<<grid, block, 0, st>>>((const Corr3DF<float> *)desc, ch, (float)dx, (float)dy, (float)dz);
     }
     return cudaGetLastError();
 }

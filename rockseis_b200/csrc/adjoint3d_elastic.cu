@@ -49,11 +49,11 @@ __device__ __forceinline__ T half_acc(T u, T w, T r, T dd, double h)
 }
 
 template <typename T, typename G>
-__global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, int nc, T dx, T dy, T dz)
+__global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, CorrChunks ch, T dx, T dy, T dz)
 {
     using O = X<T>;
-    const Corr3DE<T> c = desc[blockIdx.z / nc];
-    const int zs = blockIdx.z % nc * CORR_ZC;
+    const Corr3DE<T> c = desc[blockIdx.z / ch.count];
+    const int zs = blockIdx.z % ch.count * ch.planes;
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix < 1 || iy < 1 || ix >= c.nx - 1 || iy >= c.ny - 1) return;
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, int 
     const T *wrx = c.wr[0], *wry = c.wr[1], *wrz = c.wr[2];
     const T *rsxx = c.wr[3], *rsyy = c.wr[4], *rszz = c.wr[5], *rsyz = c.wr[6], *rsxz = c.wr[7], *rsxy = c.wr[8];
     const double DX = (double)dx, DY = (double)dy, DZ = (double)dz;
-    for (int iz = max(1, zs); iz < min(c.nz - 1, zs + CORR_ZC); iz++) {
+    for (int iz = max(1, zs); iz < min(c.nz - 1, zs + ch.planes); iz++) {
         const long long q = (long long)(iz + L) * PL + (long long)(iy + L) * P + (ix + L);
         const long long u = ((long long)iz * c.ny + iy) * c.nx + ix;
         // offsets of the neighbours: x +-1, y +-P, z +-PL
@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(256) corr_fwi_e3d(const Corr3DE<T> *desc, int 
 // columns whose z-derivatives appear, and the rz of the plane below), so a point
 // loads 49 values instead of about 100; x and y neighbours come from L1.
 template <typename G>
-__global__ void __launch_bounds__(256) corr_fwi_e3d_fast(const Corr3DE<float> *desc, int nc, float idx, float idy, float idz)
+__global__ void __launch_bounds__(256) corr_fwi_e3d_fast(const Corr3DE<float> *desc, CorrChunks ch, float idx, float idy, float idz)
 {
-    const Corr3DE<float> c = desc[blockIdx.z / nc];
-    const int z0 = max(1, (int)(blockIdx.z % nc) * CORR_ZC), ze = min(c.nz - 1, (int)(blockIdx.z % nc + 1) * CORR_ZC);
+    const Corr3DE<float> c = desc[blockIdx.z / ch.count];
+    const int z0 = max(1, (int)(blockIdx.z % ch.count) * ch.planes), ze = min(c.nz - 1, (int)(blockIdx.z % ch.count + 1) * ch.planes);
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix < 1 || iy < 1 || ix >= c.nx - 1 || iy >= c.ny - 1 || z0 >= ze) return;
@@ -291,19 +291,19 @@ __global__ void __launch_bounds__(256) residual_misfit_e3d(const Resid3E<T> *des
 cudaError_t launch_corr_fwi_e3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, int nzmax, double dx,
                                 double dy, double dz, cudaStream_t st)
 {
-    const int nc = corr_chunks(nzmax);
-    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots * nc);
+    const CorrChunks ch = corr_chunks(nshots, nzmax);
+    const dim3 block(32, 8), grid((nxmax + 31) / 32, (nymax + 7) / 8, nshots * ch.count);
     if (prec == PREC_F32_FAST) {
         const float ix = (float)(1.0 / dx), iy = (float)(1.0 / dy), iz = (float)(1.0 / dz);
-        if (acc == ACC_F64) corr_fwi_e3d_fast<double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, ix, iy, iz);
-        else corr_fwi_e3d_fast<float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, ix, iy, iz);
+        if (acc == ACC_F64) corr_fwi_e3d_fast<double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, ch, ix, iy, iz);
+        else corr_fwi_e3d_fast<float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, ch, ix, iy, iz);
     } else if (prec == PREC_F64)
-        corr_fwi_e3d<double, double><<<grid, block, 0, st>>>((const Corr3DE<double> *)desc, nc, dx, dy, dz);
+        corr_fwi_e3d<double, double><<<grid, block, 0, st>>>((const Corr3DE<double> *)desc, ch, dx, dy, dz);
     else if (acc == ACC_F64)
-        corr_fwi_e3d<float, double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, (float)dx, (float)dy,
+        corr_fwi_e3d<float, double><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, ch, (float)dx, (float)dy,
                                                             (float)dz);
     else
-        corr_fwi_e3d<float, float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, nc, (float)dx, (float)dy,
+        corr_fwi_e3d<float, float><<<grid, block, 0, st>>>((const Corr3DE<float> *)desc, ch, (float)dx, (float)dy,
                                                            (float)dz);
     return cudaGetLastError();
 }

@@ -177,13 +177,24 @@ cudaError_t launch_corr_fwi_e2d(int prec, int acc, const void *desc, int nshots,
 cudaError_t launch_scale_grad_e2d(int prec, int acc, const void *desc, int nshots, int nxmax, int nzmax,
                                   cudaStream_t st);
 cudaError_t launch_residual_e2d(int prec, int acc, const void *desc, int nshots, double *misfit, cudaStream_t st);
-// The 3D correlations: one thread per (x, y) column and CORR_ZC planes, blockIdx.z the
+// The 3D correlations: one thread per (x, y) column and a chunk of planes, blockIdx.z the
 // shot and the chunk.  A column's planes are independent but for a few values carried from
 // plane to plane; whole columns left most of the chip idle (one 121 x 111 x 101 elastic
 // window: 60 blocks, 620 us a launch; 137 us in chunks of 16, and with 8 the whole
 // gradient of two such windows takes 85 ms against 87).
 constexpr int CORR_ZC = 8;
-inline int corr_chunks(int nzmax) { return (nzmax + CORR_ZC - 1) / CORR_ZC; }
+struct CorrChunks { int planes, count; };
+// CORR_ZC planes, or as many more as keep nshots * count within a grid's 65,535 in z.
+inline CorrChunks corr_chunks(int nshots, int nzmax)
+{
+    CorrChunks c = {CORR_ZC, (nzmax + CORR_ZC - 1) / CORR_ZC};
+    const int most = nshots < 65535 ? 65535 / nshots : 1;
+    if (c.count > most) {
+        c.planes = (nzmax + most - 1) / most;
+        c.count = (nzmax + c.planes - 1) / c.planes;
+    }
+    return c;
+}
 cudaError_t launch_corr_rtm_a3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, int nzmax, int nhx,
                                 int nhy, int nhz, cudaStream_t st);
 cudaError_t launch_corr_fwi_a3d(int prec, int acc, const void *desc, int nshots, int nxmax, int nymax, int nzmax, double dx,
