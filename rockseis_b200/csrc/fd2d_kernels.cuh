@@ -30,55 +30,13 @@
 #include "rsgpu.h"
 #include "rsgpu_internal.h"
 #include "rsgpu_kernels.h"
+#include "exact_div.cuh"
 #include "pdl.cuh"
 #include "smem_limit.h"
 
 namespace rsgpu {
 
 enum { MODE_IEEE = 0, MODE_FAST = 2 };
-
-// ------------------------------------------------------------------ division by the spacing
-// Operands that the Rcp formula does not serve (tiny ones, whose error terms underflow;
-// all of them when the divisor failed its check), in double: the quotient is corrected
-// once, so it is exact where x/d is a double (ties of subnormal results among these) and
-// within 2^-52 elsewhere, where x/d is at least 2^-49 from any tie between floats.  A
-// travelling wave is preceded by a fringe of such values: dividing them with __fdiv_rn
-// took a 32 x 32 tile 23,000 cycles instead of 3,700 (its scaled path, lane by lane).
-static __device__ __noinline__ float div_slow(float x, float d, double rd)
-{
-    double q = __dmul_rn((double)x, rd);
-    q = __fma_rn(__fma_rn(-q, (double)d, (double)x), rd, q);
-    return isinf(x) ? x : __double2float_rn(q);
-}
-static __device__ __noinline__ float4 div_slow4(float4 x, float d, double rd)
-{
-    return make_float4(div_slow(x.x, d, rd), div_slow(x.y, d, rd), div_slow(x.z, d, rd), div_slow(x.w, d, rd));
-}
-// 2*bits - 1 of x: above r.lo for the operands the formula serves (zero wraps to the top)
-__device__ __forceinline__ unsigned div_key(float x) { return 2u * __float_as_uint(x) - 1u; }
-__device__ __forceinline__ float div_by(float x, float d, const Rcp<float> &r)
-{
-    float q = __fmaf_rn(x, r.h, __fmul_rn(x, r.l));
-    if (div_key(x) < r.lo) q = div_slow(x, d, r.rd);
-    return q;
-}
-__device__ __forceinline__ double div_by(double x, double d, const Rcp<double> &) { return __ddiv_rn(x, d); }
-// Four quotients with one test between them.
-__device__ __forceinline__ void div_by4(float (&x)[4], float d, const Rcp<float> &r)
-{
-    const float4 v = make_float4(x[0], x[1], x[2], x[3]);
-#pragma unroll
-    for (int j = 0; j < 4; j++) x[j] = __fmaf_rn(x[j], r.h, __fmul_rn(x[j], r.l));
-    if (min(min(div_key(v.x), div_key(v.y)), min(div_key(v.z), div_key(v.w))) < r.lo) {
-        const float4 s = div_slow4(v, d, r.rd);
-        x[0] = s.x; x[1] = s.y; x[2] = s.z; x[3] = s.w;
-    }
-}
-__device__ __forceinline__ void div_by4(double (&x)[4], double d, const Rcp<double> &)
-{
-#pragma unroll
-    for (int j = 0; j < 4; j++) x[j] = __ddiv_rn(x[j], d);
-}
 
 // ------------------------------------------------------------------ scalar arithmetic
 template <typename T, int MODE> struct Ar;
