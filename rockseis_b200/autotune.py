@@ -10,11 +10,14 @@ the time loop, reads the per-launch kernel times the plan records with CUDA
 events, and keeps the shape with the shortest velocity + stress half-steps.  The
 choice is cached in JSON under a key made of the device name, physics,
 arithmetic, order, shot count and padded grid sizes, so the search runs once per
-problem class.  Every shape computes the same numbers (the tile only changes
+problem class and library: an entry names the library it was measured with, and
+another build, whose kernels may rank otherwise, measures again.  Every shape computes the same numbers (the tile only changes
 which CTA updates a point), so the choice never changes results.
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 import time
@@ -49,6 +52,16 @@ def _device_name() -> str:
     except Exception:
         pass
     return "unknown-device"
+
+
+@functools.lru_cache(maxsize=1)
+def library_id() -> str:
+    """A digest of the library's file (58 MB: 0.15 s, once per process that tunes)."""
+    h = hashlib.blake2b(digest_size=8)
+    with open(abi.LIB_PATH, "rb") as f:
+        while block := f.read(1 << 20):
+            h.update(block)
+    return h.hexdigest()
 
 
 def problem_key(models, order: int, precision: int) -> str:
@@ -96,7 +109,7 @@ def tune_tile(models, sources, receivers, order, precision=abi.F32_EXACT, cache:
     path = cache or cache_path()
     key = problem_key(models, order, precision)
     table = _load(path)
-    if not refresh and key in table:
+    if not refresh and key in table and table[key].get("library") == library_id():
         return int(table[key]["tile"])
     shapes = tile_shapes(precision)
     if not shapes:
@@ -108,7 +121,7 @@ def tune_tile(models, sources, receivers, order, precision=abi.F32_EXACT, cache:
     best = min(ms, key=ms.get)
     table = _load(path)          # merge with entries written meanwhile
     table[key] = {"tile": best, "shape": list(shapes[best]), "ms_per_step": {str(k): round(v, 5) for k, v in ms.items()},
-                  "search_s": round(time.perf_counter() - t0, 3)}
+                  "library": library_id(), "search_s": round(time.perf_counter() - t0, 3)}
     _store(path, table)
     return best
 

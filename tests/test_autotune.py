@@ -59,3 +59,21 @@ def test_problem_key_separates_precision_and_order():
     ms = _models(2)
     keys = {autotune.problem_key(ms, o, p) for o in (4, 8) for p in (abi.F32_EXACT, abi.F32_FAST)}
     assert len(keys) == 4
+
+
+def test_entry_of_another_build_is_measured_again(tmp_path, monkeypatch):
+    monkeypatch.setattr(autotune, "tile_shapes", lambda p: {k: (32, 32, 2, 1) for k in (0, 3)})
+    monkeypatch.setattr(autotune, "measure_tile", lambda m, s, r, o, p, tile, w, n: {0: 3.0, 3: 1.5}[tile])
+    path, ms = str(tmp_path / "tiles.json"), _models()
+    key = autotune.problem_key(ms, 8, abi.F32_FAST)
+
+    def tuned(entry):
+        with open(path, "w") as f:
+            json.dump({key: entry, "another problem": {"tile": 1}}, f)
+        return autotune.tune_tile(ms, [None] * 3, [None] * 3, 8, abi.F32_FAST, cache=path)
+    assert tuned({"tile": 0, "ms_per_step": {"0": 1.0}}) == 3          # from before builds were named
+    assert tuned({"tile": 0, "library": "0123456789abcdef"}) == 3
+    table = json.load(open(path))
+    assert table[key]["library"] == autotune.library_id() and table[key]["tile"] == 3
+    assert table["another problem"] == {"tile": 1}
+    assert tuned({"tile": 0, "library": autotune.library_id()}) == 0   # this build's own pick stands
