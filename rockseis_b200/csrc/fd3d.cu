@@ -12,9 +12,10 @@
 //     into the same pass.
 // Double runs the plain kernels below, float the TMA-staged ones further down.
 // Arithmetic follows the reference operation by operation (MODE_IEEE: separately
-// rounded ops and IEEE division; MODE_FAST: FMA, coefficients pre-divided).  Near
-// the array ends the reference's reduced-order stencils are evaluated by
-// stencil_k (the same rules as in 2D).  One launch covers all tiles of all shots.
+// rounded ops and correctly rounded division; MODE_FAST: FMA, coefficients pre-divided).
+// Near the array ends the reference's reduced-order stencils are evaluated by stencil_ki
+// and, along z in float, from the register windows (the same rules as in 2D).  One launch
+// covers all tiles of all shots.
 #include <type_traits>
 
 #include "fd3d_common.cuh"
@@ -299,18 +300,6 @@ struct A3Smem {
 template <typename Stage>
 constexpr size_t a3_smem_bytes() { return sizeof(A3Smem<Stage>) + 128; }   // + alignment slack
 
-// Two derivatives of full order on the lanes of a pair: `at(k)` the operand pair at tap k of
-// the 16 (7 | 8 around the centre).
-template <int MODE, typename F>
-__device__ __forceinline__ float2 taps_lanes(F at, const float (&c2)[NCOEF][2], float d, const Rcp<float> &r)
-{
-    using A2 = Ar2<float, MODE>;
-    const float2 *cc = reinterpret_cast<const float2 *>(c2);
-    float2 acc = A2::mul(A2::sub(at(8), at(7)), cc[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A2::acc(acc, A2::sub(at(8 + k), at(7 - k)), cc[k]);
-    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
-}
 // The y-derivatives of rows y and y + 1 from 17 shared loads; b at the first row's tap 0.
 template <int MODE>
 __device__ __forceinline__ float2 taps_rows(const float *b, int s, const float *c, float d, const Rcp<float> &r)
@@ -327,21 +316,6 @@ __device__ __forceinline__ float2 taps_rows(const float *b, int s, const float *
     }
     return MODE == MODE_FAST ? acc : make_float2(div_by(acc.x, d, r), div_by(acc.y, d, r));
 }
-// Reduced-order z stencils at a plane near an array end (K the same for the block).
-template <int MODE>
-__device__ __forceinline__ float2 taps_lanes_k(const float2 (&q)[16], int K, const float *c, float d, const Rcp<float> &r)
-{
-    using A2 = Ar2<float, MODE>;
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < NCOEF; k++)
-        if (k < K) {
-            const float2 dl = A2::sub(q[8 + k], q[7 - k]), ck = make_float2(c[k], c[k]);
-            acc = k == 0 ? A2::mul(dl, ck) : A2::acc(acc, dl, ck);
-        }
-    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
-}
-
 // What a thread's two columns share in both half-steps.
 struct A3Cols {
     int ix, iy, col, xc, yc[2], Kx, Ky[2];

@@ -52,6 +52,33 @@ __device__ __forceinline__ T taps_reg_k(const T (&q)[16], int K, const T *c, T d
     return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
 }
 
+// Two derivatives of full order on the lanes of a pair: `at(k)` the operand pair at tap k of
+// the 16 (7 | 8 around the centre).
+template <int MODE, typename F>
+__device__ __forceinline__ float2 taps_lanes(F at, const float (&c2)[NCOEF][2], float d, const Rcp<float> &r)
+{
+    using A2 = Ar2<float, MODE>;
+    const float2 *cc = reinterpret_cast<const float2 *>(c2);
+    float2 acc = A2::mul(A2::sub(at(8), at(7)), cc[0]);
+#pragma unroll
+    for (int k = 1; k < NCOEF; k++) acc = A2::acc(acc, A2::sub(at(8 + k), at(7 - k)), cc[k]);
+    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
+}
+// The same at a plane near an array end: K pairs (the same for the block) of the row c.
+template <int MODE>
+__device__ __forceinline__ float2 taps_lanes_k(const float2 (&q)[16], int K, const float *c, float d, const Rcp<float> &r)
+{
+    using A2 = Ar2<float, MODE>;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < NCOEF; k++)
+        if (k < K) {
+            const float2 dl = A2::sub(q[8 + k], q[7 - k]), ck = make_float2(c[k], c[k]);
+            acc = k == 0 ? A2::mul(dl, ck) : A2::acc(acc, dl, ck);
+        }
+    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
+}
+
 // Column of the 2L strip cells of an axis that cell i holds (low strip, then high), -1: none.
 __device__ __forceinline__ int strip_col(int i, int n, int L)
 {

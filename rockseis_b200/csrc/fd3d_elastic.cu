@@ -30,40 +30,6 @@
 namespace rsgpu {
 namespace {
 
-// Copy the shot descriptor into shared memory: the field pointers are then read
-// from a space that the kernel's global stores cannot alias, so the compiler may
-// keep or re-read them freely instead of reloading them from global memory after
-// every store.  Visible after the block's next barrier.
-template <typename T>
-__device__ __forceinline__ void stage_shot(Shot3D<T> &dst, const Shot3D<T> *src)
-{
-    constexpr int n = sizeof(Shot3D<T>) / sizeof(int);
-    static_assert(sizeof(Shot3D<T>) % sizeof(int) == 0, "descriptor size");
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    if (tid < n) reinterpret_cast<int *>(&dst)[tid] = reinterpret_cast<const int *>(src)[tid];
-}
-
-// Staggered derivative with all NCOEF taps: b[0] = f[i-7] (forward) or f[i-8]
-// (backward); sum_k (b[8+k] - b[7-k]) c_k in the reference's order.
-template <typename T, int MODE>
-__device__ __forceinline__ T taps3(const T *b, int s, const T *cu, T d, const Rcp<T> &r)
-{
-    using A = Ar<T, MODE>;
-    T acc = A::mul(A::sub(b[8 * s], b[7 * s]), cu[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A::mad(acc, A::sub(b[(8 + k) * s], b[(7 - k) * s]), cu[k]);
-    return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
-}
-template <typename T, int MODE>
-__device__ __forceinline__ T taps3_reg(const T (&q)[16], const T *cu, T d, const Rcp<T> &r)
-{
-    using A = Ar<T, MODE>;
-    T acc = A::mul(A::sub(q[8], q[7]), cu[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A::mad(acc, A::sub(q[8 + k], q[7 - k]), cu[k]);
-    return (MODE == MODE_FAST) ? acc : A::div(acc, d, r);
-}
-
 // Operands of the velocity step: the stresses (forward) or the work arrays of
 // backwardstepVelocity (lib/waves.cpp:3307, 3353, 3399, 3446, 3491, 3535, 3582,
 // 3628, 3672), evaluated in the reference's expression order.
@@ -130,7 +96,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity(Step3DArgs<T> a, con
     VelSmem<T> &S = *reinterpret_cast<VelSmem<T> *>(smraw);
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
-    stage_shot(shs, a.shots + tl.shot);
+    stage_words(shs, a.shots + tl.shot, threadIdx.y * TX3 + threadIdx.x, TX3 * TY3);
     load_coefs3(S.cs, coefs);
     __syncthreads();
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -217,12 +183,12 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity(Step3DArgs<T> a, con
         // ---- Vx
         {
             const T *c = &S.xx[b][ty][tx + 8];
-            const T d1 = (Kxf == order) ? taps3<T, MODE>(c - 7, 1, cux, a.dx, a.rdx)
+            const T d1 = (Kxf == order) ? taps<T, MODE>(c - 7, 1, cux, a.dx, a.rdx)
                                         : stencil_k<T, MODE>(c, 1, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
             const T *cy = &S.xy[b][ty + 8][tx + 8];
-            const T d2 = (Kyb == order) ? taps3<T, MODE>(cy - 8 * WX, WX, cuy, a.dy, a.rdy)
+            const T d2 = (Kyb == order) ? taps<T, MODE>(cy - 8 * WX, WX, cuy, a.dy, a.rdy)
                                         : stencil_k<T, MODE>(cy, WX, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-            const T d3 = (Kzb == order) ? taps3_reg<T, MODE>(qxz, cuz, a.dz, a.rdz)
+            const T d3 = (Kzb == order) ? taps_reg<T, MODE>(qxz, cuz, a.dz, a.rdz)
                                         : stencil_z_op<T, MODE, ADJ>(sh, o, plane, Kzb, S.cs.cz + Kzb * CROW3, false, OP_XZ, a.dz, a.rdz);
             const T am = A::mul(a.dt, rx);
             vx = A::mad(vx, am, d1);
@@ -236,12 +202,12 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity(Step3DArgs<T> a, con
         // ---- Vy
         {
             const T *c = &S.xy[b][ty + 8][tx + 8];
-            const T d1 = (Kxb == order) ? taps3<T, MODE>(c - 8, 1, cux, a.dx, a.rdx)
+            const T d1 = (Kxb == order) ? taps<T, MODE>(c - 8, 1, cux, a.dx, a.rdx)
                                         : stencil_k<T, MODE>(c, 1, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
             const T *cy = &S.yy[b][ty + 8][tx];
-            const T d2 = (Kyf == order) ? taps3<T, MODE>(cy - 7 * TX3, TX3, cuy, a.dy, a.rdy)
+            const T d2 = (Kyf == order) ? taps<T, MODE>(cy - 7 * TX3, TX3, cuy, a.dy, a.rdy)
                                         : stencil_k<T, MODE>(cy, TX3, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
-            const T d3 = (Kzb == order) ? taps3_reg<T, MODE>(qyz, cuz, a.dz, a.rdz)
+            const T d3 = (Kzb == order) ? taps_reg<T, MODE>(qyz, cuz, a.dz, a.rdz)
                                         : stencil_z_op<T, MODE, ADJ>(sh, o, plane, Kzb, S.cs.cz + Kzb * CROW3, false, OP_YZ, a.dz, a.rdz);
             const T am = A::mul(a.dt, ry);
             vy = A::mad(vy, am, d1);
@@ -255,12 +221,12 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity(Step3DArgs<T> a, con
         // ---- Vz
         {
             const T *c = &S.xz[b][ty][tx + 8];
-            const T d1 = (Kxb == order) ? taps3<T, MODE>(c - 8, 1, cux, a.dx, a.rdx)
+            const T d1 = (Kxb == order) ? taps<T, MODE>(c - 8, 1, cux, a.dx, a.rdx)
                                         : stencil_k<T, MODE>(c, 1, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
             const T *cy = &S.yz[b][ty + 8][tx];
-            const T d2 = (Kyb == order) ? taps3<T, MODE>(cy - 8 * TX3, TX3, cuy, a.dy, a.rdy)
+            const T d2 = (Kyb == order) ? taps<T, MODE>(cy - 8 * TX3, TX3, cuy, a.dy, a.rdy)
                                         : stencil_k<T, MODE>(cy, TX3, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-            const T d3 = (Kzf == order) ? taps3_reg<T, MODE>(qzz, cuz, a.dz, a.rdz)
+            const T d3 = (Kzf == order) ? taps_reg<T, MODE>(qzz, cuz, a.dz, a.rdz)
                                         : stencil_z_op<T, MODE, ADJ>(sh, o, plane, Kzf, S.cs.cz + Kzf * CROW3, true, OP_ZZ, a.dz, a.rdz);
             const T am = A::mul(a.dt, rz);
             vz = A::mad(vz, am, d1);
@@ -309,7 +275,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress(Step3DArgs<T> a, const
     StrSmem<T> &S = *reinterpret_cast<StrSmem<T> *>(smraw);
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
-    stage_shot(shs, a.shots + tl.shot);
+    stage_words(shs, a.shots + tl.shot, threadIdx.y * TX3 + threadIdx.x, TX3 * TY3);
     load_coefs3(S.cs, coefs);
     __syncthreads();
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -390,11 +356,11 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress(Step3DArgs<T> a, const
         const T *cvx = &S.vx[b][ty + 8][tx + 8], *cvy = &S.vy[b][ty + 8][tx + 8], *cvz = &S.vz[b][ty + 8][tx + 8];
         // ---- normal stresses
         {
-            const T dxx = (Kxb == order) ? taps3<T, MODE>(cvx - 8, 1, cux, a.dx, a.rdx)
+            const T dxx = (Kxb == order) ? taps<T, MODE>(cvx - 8, 1, cux, a.dx, a.rdx)
                                          : stencil_k<T, MODE>(cvx, 1, Kxb, S.cs.cx + Kxb * CROW3, false, a.dx, a.rdx);
-            const T dyy = (Kyb == order) ? taps3<T, MODE>(cvy - 8 * WX, WX, cuy, a.dy, a.rdy)
+            const T dyy = (Kyb == order) ? taps<T, MODE>(cvy - 8 * WX, WX, cuy, a.dy, a.rdy)
                                          : stencil_k<T, MODE>(cvy, WX, Kyb, S.cs.cy + Kyb * CROW3, false, a.dy, a.rdy);
-            const T dzz = (Kzb == order) ? taps3_reg<T, MODE>(qz, cuz, a.dz, a.rdz)
+            const T dzz = (Kzb == order) ? taps_reg<T, MODE>(qz, cuz, a.dz, a.rdz)
                                          : stencil_k<T, MODE>(Vz + o, (int)plane, Kzb, S.cs.cz + Kzb * CROW3, false, a.dz, a.rdz);
             const bool fsrow = sh.fs && iz == L;
             if (!ADJ) {
@@ -430,9 +396,9 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress(Step3DArgs<T> a, const
         }
         // ---- Sxz: Dx+ Vz, Dz+ Vx
         {
-            const T d1 = (Kxf == order) ? taps3<T, MODE>(cvz - 7, 1, cux, a.dx, a.rdx)
+            const T d1 = (Kxf == order) ? taps<T, MODE>(cvz - 7, 1, cux, a.dx, a.rdx)
                                         : stencil_k<T, MODE>(cvz, 1, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
-            const T d2 = (Kzf == order) ? taps3_reg<T, MODE>(qx, cuz, a.dz, a.rdz)
+            const T d2 = (Kzf == order) ? taps_reg<T, MODE>(qx, cuz, a.dz, a.rdz)
                                         : stencil_k<T, MODE>(Vx + o, (int)plane, Kzf, S.cs.cz + Kzf * CROW3, true, a.dz, a.rdz);
             const T am = ADJ ? a.dt : A::mul(a.dt, mxz);
             sxz = A::mad(sxz, am, d1);
@@ -443,9 +409,9 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress(Step3DArgs<T> a, const
         }
         // ---- Syz: Dz+ Vy, Dy+ Vz
         {
-            const T d1 = (Kzf == order) ? taps3_reg<T, MODE>(qy, cuz, a.dz, a.rdz)
+            const T d1 = (Kzf == order) ? taps_reg<T, MODE>(qy, cuz, a.dz, a.rdz)
                                         : stencil_k<T, MODE>(Vy + o, (int)plane, Kzf, S.cs.cz + Kzf * CROW3, true, a.dz, a.rdz);
-            const T d2 = (Kyf == order) ? taps3<T, MODE>(cvz - 7 * WX, WX, cuy, a.dy, a.rdy)
+            const T d2 = (Kyf == order) ? taps<T, MODE>(cvz - 7 * WX, WX, cuy, a.dy, a.rdy)
                                         : stencil_k<T, MODE>(cvz, WX, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
             const T am = ADJ ? a.dt : A::mul(a.dt, myz);
             syz = A::mad(syz, am, d1);
@@ -456,9 +422,9 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress(Step3DArgs<T> a, const
         }
         // ---- Sxy: Dy+ Vx, Dx+ Vy
         {
-            const T d1 = (Kyf == order) ? taps3<T, MODE>(cvx - 7 * WX, WX, cuy, a.dy, a.rdy)
+            const T d1 = (Kyf == order) ? taps<T, MODE>(cvx - 7 * WX, WX, cuy, a.dy, a.rdy)
                                         : stencil_k<T, MODE>(cvx, WX, Kyf, S.cs.cy + Kyf * CROW3, true, a.dy, a.rdy);
-            const T d2 = (Kxf == order) ? taps3<T, MODE>(cvy - 7, 1, cux, a.dx, a.rdx)
+            const T d2 = (Kxf == order) ? taps<T, MODE>(cvy - 7, 1, cux, a.dx, a.rdx)
                                         : stencil_k<T, MODE>(cvy, 1, Kxf, S.cs.cx + Kxf * CROW3, true, a.dx, a.rdx);
             const T am = ADJ ? a.dt : A::mul(a.dt, mxy);
             sxy = A::mad(sxy, am, d1);
@@ -526,45 +492,12 @@ struct TmaSmem {
 template <typename Stage>
 constexpr size_t tma_smem_bytes() { return sizeof(TmaSmem<Stage>) + 128; }   // + alignment slack
 
-// (a - b) pairs of two arrays with the same tap spacing: sum_k c_k (p[(8+k)s] - p[(7-k)s])
+// The derivatives of two arrays along one axis as the lanes of a pair; p and q at tap 0.
 template <int MODE>
-__device__ __forceinline__ float2 taps_pair2(const float *p, const float *q, int sp, int sq,
-                                             const float (&c2)[NCOEF][2], float d, const Rcp<float> &r)
+__device__ __forceinline__ float2 taps_two(const float *p, const float *q, int sp, int sq, const float (&c2)[NCOEF][2],
+                                           float d, const Rcp<float> &r)
 {
-    using A2 = Ar2<float, MODE>;
-    const float2 *cc = reinterpret_cast<const float2 *>(c2);
-    float2 acc = A2::mul(A2::sub(make_float2(p[8 * sp], q[8 * sq]), make_float2(p[7 * sp], q[7 * sq])), cc[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++)
-        acc = A2::acc(acc, A2::sub(make_float2(p[(8 + k) * sp], q[(8 + k) * sq]),
-                                   make_float2(p[(7 - k) * sp], q[(7 - k) * sq])), cc[k]);
-    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
-}
-template <int MODE>
-__device__ __forceinline__ float2 taps_pair_reg(const float2 (&q)[16], const float (&c2)[NCOEF][2], float d,
-                                                const Rcp<float> &r)
-{
-    using A2 = Ar2<float, MODE>;
-    const float2 *cc = reinterpret_cast<const float2 *>(c2);
-    float2 acc = A2::mul(A2::sub(q[8], q[7]), cc[0]);
-#pragma unroll
-    for (int k = 1; k < NCOEF; k++) acc = A2::acc(acc, A2::sub(q[8 + k], q[7 - k]), cc[k]);
-    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
-}
-// The same at a plane near an array end: K pairs of the row c (the same for the block).
-template <int MODE>
-__device__ __forceinline__ float2 taps_pair_reg_k(const float2 (&q)[16], int K, const float *c, float d,
-                                                  const Rcp<float> &r)
-{
-    using A2 = Ar2<float, MODE>;
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < NCOEF; k++)
-        if (k < K) {
-            const float2 dl = A2::sub(q[8 + k], q[7 - k]), ck = make_float2(c[k], c[k]);
-            acc = k == 0 ? A2::mul(dl, ck) : A2::acc(acc, dl, ck);
-        }
-    return MODE == MODE_FAST ? acc : A2::div(acc, d, r);
+    return taps_lanes<MODE>([&](int t) { return make_float2(p[t * sp], q[t * sq]); }, c2, d, r);
 }
 
 template <int MODE>
@@ -577,7 +510,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
         *reinterpret_cast<TmaSmem<VelStageT> *>((reinterpret_cast<uintptr_t>(smraw) + 127) & ~uintptr_t(127));
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
-    stage_shot(shs, a.shots + tl.shot);
+    stage_words(shs, a.shots + tl.shot, threadIdx.y * TX3 + threadIdx.x, TX3 * TY3);
     load_coefs3(S.cs, coefs);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX3 + tx;
     const int x0 = tl.x0, y0 = tl.y0, L = a.lpml, order = a.order;
@@ -649,8 +582,8 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
         T dxx, dyy, dzz;
         float2 dxq, dyq, dzq;      // (Dx- XY, Dx- XZ), (Dy- XY, Dy- YZ), (Dz- XZ, Dz- YZ)
         if (!xe) {
-            dxx = taps3<T, MODE>(cxx - 7, 1, a.cf[0], a.dx, a.rdx);
-            dxq = taps_pair2<MODE>(cxy - 8, cxz - 8, 1, 1, a.cf2[0], a.dx, a.rdx);
+            dxx = taps<T, MODE>(cxx - 7, 1, a.cf[0], a.dx, a.rdx);
+            dxq = taps_two<MODE>(cxy - 8, cxz - 8, 1, 1, a.cf2[0], a.dx, a.rdx);
         } else {
             const int Kf = kfw(ix, nxp, order), Kb = kbw(ix, nxp, order);
             const T *cf = S.cs.cx + Kf * CROW3, *cb = S.cs.cx + Kb * CROW3;
@@ -659,8 +592,8 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
             dxq.y = stencil_ki<T, MODE>(cxz, 1, Kb, cb, false, a.dx, a.rdx);
         }
         if (!ye) {
-            dyq = taps_pair2<MODE>(cxy - 8 * WX, cyz - 8 * TX3, WX, TX3, a.cf2[1], a.dy, a.rdy);
-            dyy = taps3<T, MODE>(cyy - 7 * TX3, TX3, a.cf[1], a.dy, a.rdy);
+            dyq = taps_two<MODE>(cxy - 8 * WX, cyz - 8 * TX3, WX, TX3, a.cf2[1], a.dy, a.rdy);
+            dyy = taps<T, MODE>(cyy - 7 * TX3, TX3, a.cf[1], a.dy, a.rdy);
         } else {
             const int Kf = kfw(iy, nyp, order), Kb = kbw(iy, nyp, order);
             const T *cf = S.cs.cy + Kf * CROW3, *cb = S.cs.cy + Kb * CROW3;
@@ -670,10 +603,10 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_velocity_tma(Step3DArgs<float
         }
         const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
         if (Kzf == order && Kzb == order) {
-            dzq = taps_pair_reg<MODE>(qp, a.cf2[2], a.dz, a.rdz);
-            dzz = taps3_reg<T, MODE>(qzz, a.cf[2], a.dz, a.rdz);
+            dzq = taps_lanes<MODE>([&](int t) { return qp[t]; }, a.cf2[2], a.dz, a.rdz);
+            dzz = taps_reg<T, MODE>(qzz, a.cf[2], a.dz, a.rdz);
         } else {
-            dzq = taps_pair_reg_k<MODE>(qp, Kzb, S.cs.cz + Kzb * CROW3, a.dz, a.rdz);
+            dzq = taps_lanes_k<MODE>(qp, Kzb, S.cs.cz + Kzb * CROW3, a.dz, a.rdz);
             dzz = taps_reg_k<T, MODE>(qzz, Kzf, S.cs.cz + Kzf * CROW3, a.dz, a.rdz);
         }
         const T *fz = strip_factors(a.pml, L, iz, nzp, 0);
@@ -722,7 +655,7 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> 
         *reinterpret_cast<TmaSmem<StrStageT> *>((reinterpret_cast<uintptr_t>(smraw) + 127) & ~uintptr_t(127));
     __shared__ Shot3D<T> shs;
     const Tile3D tl = a.tiles[blockIdx.x];
-    stage_shot(shs, a.shots + tl.shot);
+    stage_words(shs, a.shots + tl.shot, threadIdx.y * TX3 + threadIdx.x, TX3 * TY3);
     load_coefs3(S.cs, coefs);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX3 + tx;
     const int x0 = tl.x0, y0 = tl.y0, L = a.lpml, order = a.order;
@@ -790,8 +723,8 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> 
         T dxx, dyy, dzz;
         float2 dxp, dyp, dzp;      // (Dx+ Vz, Dx+ Vy), (Dy+ Vz, Dy+ Vx), (Dz+ Vx, Dz+ Vy)
         if (!xe) {
-            dxx = taps3<T, MODE>(cvx - 8, 1, a.cf[0], a.dx, a.rdx);
-            dxp = taps_pair2<MODE>(cvz - 7, cvy - 7, 1, 1, a.cf2[0], a.dx, a.rdx);
+            dxx = taps<T, MODE>(cvx - 8, 1, a.cf[0], a.dx, a.rdx);
+            dxp = taps_two<MODE>(cvz - 7, cvy - 7, 1, 1, a.cf2[0], a.dx, a.rdx);
         } else {
             const int Kf = kfw(ix, nxp, order), Kb = kbw(ix, nxp, order);
             const T *cf = S.cs.cx + Kf * CROW3, *cb = S.cs.cx + Kb * CROW3;
@@ -800,8 +733,8 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> 
             dxp.y = stencil_ki<T, MODE>(cvy, 1, Kf, cf, true, a.dx, a.rdx);
         }
         if (!ye) {
-            dyy = taps3<T, MODE>(cvy - 8 * WX, WX, a.cf[1], a.dy, a.rdy);
-            dyp = taps_pair2<MODE>(cvz - 7 * WX, cvx - 7 * WX, WX, WX, a.cf2[1], a.dy, a.rdy);
+            dyy = taps<T, MODE>(cvy - 8 * WX, WX, a.cf[1], a.dy, a.rdy);
+            dyp = taps_two<MODE>(cvz - 7 * WX, cvx - 7 * WX, WX, WX, a.cf2[1], a.dy, a.rdy);
         } else {
             const int Kf = kfw(iy, nyp, order), Kb = kbw(iy, nyp, order);
             const T *cf = S.cs.cy + Kf * CROW3, *cb = S.cs.cy + Kb * CROW3;
@@ -811,11 +744,11 @@ __global__ void __launch_bounds__(TX3 *TY3, 2) e3d_stress_tma(Step3DArgs<float> 
         }
         const int Kzf = kfw(iz, nzp, order), Kzb = kbw(iz, nzp, order);
         if (Kzf == order && Kzb == order) {
-            dzz = taps3_reg<T, MODE>(qz, a.cf[2], a.dz, a.rdz);
-            dzp = taps_pair_reg<MODE>(qv, a.cf2[2], a.dz, a.rdz);
+            dzz = taps_reg<T, MODE>(qz, a.cf[2], a.dz, a.rdz);
+            dzp = taps_lanes<MODE>([&](int t) { return qv[t]; }, a.cf2[2], a.dz, a.rdz);
         } else {
             dzz = taps_reg_k<T, MODE>(qz, Kzb, S.cs.cz + Kzb * CROW3, a.dz, a.rdz);
-            dzp = taps_pair_reg_k<MODE>(qv, Kzf, S.cs.cz + Kzf * CROW3, a.dz, a.rdz);
+            dzp = taps_lanes_k<MODE>(qv, Kzf, S.cs.cz + Kzf * CROW3, a.dz, a.rdz);
         }
         const T *fz0 = strip_factors(a.pml, L, iz, nzp, 0);
         // the derivative term of memory array 3 + f along an axis, its memory updated

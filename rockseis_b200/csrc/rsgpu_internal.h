@@ -73,7 +73,6 @@ enum {
     TILE_ZEDGE = 2,
     TILE_XPML = 4,    // tile intersects the left/right C-PML strips
     TILE_ZPML = 8,
-    TILE_FSROW = 16,  // tile contains the free-surface row
 };
 
 // PML tables on the device: 12 arrays of lpml entries, in the order
