@@ -86,7 +86,8 @@ typedef struct {
                            A,B,C rbb; A,B,C rbb_stag (include/pml.h:31-81).  NULL: computed
                            by rsgpu_pml_tables with Smax = 1200. */
     int tile;           /* 2D kernel tile shape index (rsgpu_tile_shape), -1 = built-in default */
-    int zchunk;         /* 3D: planes marched by one CTA (0 = 64); 2D fused step: rows per
+    int zchunk;         /* 3D: planes marched by one CTA (0 = chosen from the batch: 20 to 40,
+                           or all planes of shorter windows); 2D fused step: rows per
                            work item (rounded up to 8; 0 = chosen from the batch size) */
     int launch_mode;    /* 2D propagation: 0 = library choice (the per-tile kernels, the
                            faster on B200), 1 = the same as 2 (a persistent variant of the

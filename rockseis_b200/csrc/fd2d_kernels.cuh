@@ -3,16 +3,17 @@
 // One kernel per half-step (velocity, stress), each covering every shot of a
 // batch in one launch: the grid walks a table of (shot, tile) work items, so
 // shots with different aperture windows share a launch.  Each CTA stages the
-// stencil inputs of its TX x TZ tile plus an 8-cell halo in shared memory with
-// TMA (cp.async.bulk.tensor, completion on an mbarrier), while its threads fetch
-// the point-wise inputs (velocities, moduli) straight into registers.  Every
-// thread then produces a 4(x) x RZ(z) block with the C-PML memory-variable
-// update and correction fused into the same pass:
+// stencil inputs of its TX x TZ tile, with an 8-cell halo along the axes that each is
+// differentiated along, in shared memory with TMA (cp.async.bulk.tensor, completion
+// on an mbarrier), while its threads fetch the point-wise inputs (velocities, moduli)
+// straight into registers.  Every thread then produces a 4(x) x RZ(z) block with the
+// C-PML memory-variable update and correction fused into the same pass:
 //   - x-derivatives: one 128-bit shared load per 4 taps, scalar arithmetic;
-//   - z-derivatives: column pairs, 64-bit shared loads, paired f32x2 arithmetic
-//     (FADD2/FMUL2/FFMA2), each lane rounded exactly like a scalar op;
-//   - interior tiles keep the 8 coefficients in registers; tiles within `order`
-//     cells of an array end use per-point coefficient rows (reduced order).
+//   - z-derivatives: exact, column pairs from 64-bit shared loads (dz_pair); fast, the
+//     window rows streamed as 128-bit loads into paired FMAs (dz_stream_f32);
+//   - the full-order coefficients are operands in the launch's parameter space; tiles
+//     within `order` cells of an array end predicate off the taps that their rows and
+//     columns lack (coefficient rows in shared memory).
 //
 // Arithmetic follows the reference operation by operation (Der::ddx_fw etc. in
 // lib/der.cpp:155-540, WavesAcoustic2D/WavesElastic2D::forwardstep* in
@@ -409,15 +410,12 @@ __device__ __forceinline__ void tile_prologue(unsigned char *sm, uint64_t *bar, 
 //                             [0] Vx, [1] Vz, [2] Sxx, [3] Szz, [4] Sxz (elastic)
 
 // Reduced-order stencil of K pairs at one point (reference rule near the array
-// ends): taps read from memory at `stride`, K known only at run time.  Used to
-// overwrite the few outputs of an edge tile whose K differs from the order.
-// Two forms with the same operations in the same order: a call (stencil_k), and
-// an inlined form unrolled over the NCOEF taps with the taps k >= K predicated
-// off (stencil_ki), which saves the edge lanes of a warp the call's register
-// saves at the price of registers in the caller.  Measured on B200, the inlined
-// form is faster in the elastic 2D tile kernels (16-shot batch +11 %) and the
-// acoustic 3D kernels (+14 %), slower in the acoustic 2D tile kernels of a
-// 64-shot FWI batch (-6 %) and in the elastic 3D kernels (-17 %).
+// ends): taps read from memory at `stride`, K known only at run time.  Two forms with
+// the same operations in the same order: a call (stencil_k), for the fused 2D step and
+// the plain elastic 3D kernels, where the inlined form costs the caller registers
+// (-17 % there on B200); and an inlined form unrolled over the NCOEF taps with the taps
+// k >= K predicated off (stencil_ki), for the 3D kernels that choose per block (TMA) and
+// the plain acoustic ones (+14 %).
 template <typename T, int MODE>
 __device__ __noinline__ T stencil_k(const T *center, int stride, int K, const T *c, bool fw, T d, const Rcp<T> &r)
 {

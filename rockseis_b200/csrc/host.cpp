@@ -645,18 +645,22 @@ void Plan::fill_desc(unsigned char *sd, unsigned char *irp, const ShotLayout &L,
 
 int default_tile_2d(int prec, int phys, long long tiles)
 {
-    // Float: 32x16 tiles, of 64 threads with two rows each (102 to 118 registers, ten tiles
-    // on an SM) or of 128 with one (80 to 90 registers, six).  Two rows share loads and
+    // Float: 32x16 tiles, of 64 threads with two rows each (102 to 118 registers, eight to ten
+    // tiles on an SM) or of 128 with one (80 to 90 registers, six).  Two rows share loads and
     // coefficients between them, one has half the chain.  So one row where a launch is a
-    // round of six, and past one round of ten up to where the rate counts; measured on B200
-    // by tiles an SM, us a step of two rows | one:
-    //   FAST acoustic  2: 10.6 | 8.7   8.3: 13.8 | 15.2   10.7: 19.0 | 17.1   19: 25.3 | 25.0   40: 34.4 | 36.0
-    //   FAST elastic   2: 15.6 | 12.0  9.5: 21.6 | 22.9   10.7: 27.6 | 24.8   19: 37.3 | 37.8   40: 58.0 | 62.3
-    //   EXACT acoustic 2: 11.2 | 8.7   8.3: 16.5 | 16.3   16: 20.5 | 19.2     28: 37.9 | 36.9   40: 36.4 | 38.0
-    //   EXACT elastic  2: 18.0 | 12.8  8.3: 25.2 | 22.4   16: 35.6 | 30.5     40: 77 | 69       82: 147 | 133
-    // Measured beside them: 32x32 of two rows (spills), four rows a thread at one CTA (one
-    // 541x341 acoustic shot 38 ms against 31 with two rows), 32x8 of one row (elastic 64.3
-    // at 40 an SM).
+    // round of six, and past one round of ten up to where the rate counts.  Measured on B200
+    // with 2 to 48 shots of 441x291 padded points, us a step of two rows | one:
+    //   tiles an SM     3.6          7.2          10.8         16.2         21.6         32           43           65          86
+    //   FAST acoustic   10.5 | 9.3   12.2 | 13.5  17.5 | 15.7  20.9 | 20.2  24.9 | 24.4  33.8 | 34.5  45.6 | 47.5  72 | 76    95 | 99
+    //   FAST elastic    16.6 | 13.8  19.4 | 19.4  26.4 | 24.4  32.1 | 31.8  40.7 | 41.2  57.5 | 62.2  75.7 | 82.0  108 | 118  136 | 152
+    //   EXACT acoustic  11.9 | 9.7   13.8 | 13.7  18.6 | 16.4  22.9 | 21.3  26.8 | 25.9  36.7 | 37.1  48.8 | 50.5  75 | 78    98 | 102
+    //   EXACT elastic   19.3 | 14.9  22.8 | 21.4  33.6 | 26.5  41.9 | 35.1  55.6 | 45.4  83.5 | 69.4  110 | 91     159 | 132  207 | 171
+    // Gradients run the same shape in both directions: 4 to 16 shots of that size, both
+    // physics, within 3 % of the best of these and the 32x32 shapes.  Measured beside them:
+    // 32x32 of two rows at six CTAs (sixteen elastic shots of 861x461 115 us a step against 110;
+    // sixteen acoustic ones of 641x241 27.7 against 31.7, left to an explicit tile or the tuner),
+    // four rows a thread at one CTA (one 541x341 acoustic shot 38 ms against 31 with two rows),
+    // 32x8 of one row (elastic 64.3 at 40 an SM).
     if (prec == PREC_F64) return TILECFG_64x32;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||

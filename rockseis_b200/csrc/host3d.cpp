@@ -65,7 +65,11 @@ Plan3D::~Plan3D()
 // longer).  Measured on B200: two elastic windows to 192x196x191 67.3 ms whole, 62.6 in 48
 // planes, 61.4 in 32; four acoustic ones to 226x235x221 59.6 in 56, 58.7 in 37; a gradient of
 // one 161x151x141 window 100 ms in 71, 94 in 36, 85 in 29, 92 in 24; one exact 151x141x131
-// window 20 ms a call in 64, 17 in 33, 15 in 27, 14 in 22.
+// window 20 ms a call in 64, 17 in 33, 15 in 27, 14 in 22.  The other kernels that march
+// chunks, as picked | in 32 | in 64 planes, ms: FP64 acoustic, windows to 151x141x131 and
+// 241x221x201, 22.2 | 24.6 | 28.6 and 31.2 | 30.4 | 34.6; FP64 elastic, to 131x121x111 and
+// 201x191x171, 45.5 | 43.0 | 74.5 and 112 | 113 | 122; exact elastic gradients (plain adjoint
+// velocity step), 141x131x121 and 201x191x171, 84.6 | 89.8 | 108 and 146 | 144 | 157.
 int Plan3D::pick_zchunk(const rsgpu_shot *s) const
 {
     constexpr int CHUNK_FILL = 8, CHUNK_TAIL = 2, ZC_MIN = 20, ZC_MAX = 40;

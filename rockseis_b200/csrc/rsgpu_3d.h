@@ -38,7 +38,7 @@ struct Shot3D {
     T *psix[6], *psiy[6], *psiz[6];
 };
 
-// Tensor maps of the acoustic 3D TMA kernels (FAST), per shot, over whole pitched
+// Tensor maps of the acoustic 3D TMA kernels (float), per shot, over whole pitched
 // arrays like the elastic ones:
 //   velocity: P {48 x 32} (x and y halos); Vx, Vy, Vz, Rx, Ry, Rz {32 x 16}
 //   stress:   Vx {48 x 16} (x halo); Vy {32 x 32} (y halo); P, L {32 x 16}
@@ -78,7 +78,7 @@ struct Step3DArgs {
     T dt, dx, dy, dz;
     Rcp<T> rdx, rdy, rdz;
     const T *pml;
-    const void *maps;          // elastic fast mode: NMAP_E3 CUtensorMaps per shot (null: no TMA kernels)
+    const void *maps;          // float: NMAP_A3 or NMAP_E3 CUtensorMaps per shot; null in double (no TMA kernels)
     int *err;                  // device error word (a bounded wait that gave up)
 };
 
