@@ -33,26 +33,26 @@ inline unsigned bits_of(float a)
 }
 #endif
 
+// 2*bits - 1 of x: above r.lo for the operands the formula serves (zero wraps to the top, above
+// infinities and NaN)
+__host__ __device__ __forceinline__ unsigned div_key(float x) { return 2u * bits_of(x) - 1u; }
 // Operands that the Rcp formula does not serve (tiny ones, whose error terms underflow;
 // all of them when the divisor failed its check), in double: the quotient is corrected
 // once, so it is exact where x/d is a double (ties of subnormal results among these) and
 // within 2^-52 elsewhere, where x/d is at least 2^-49 from any tie between floats; zeros
-// (neighbours of a tiny operand) keep their sign.  A travelling wave is preceded by a
-// fringe of such values: dividing them with __fdiv_rn took a 32 x 32 tile 23,000 cycles
-// instead of 3,700 (its scaled path, lane by lane).
+// (neighbours of a tiny operand) and infinities are returned as they are.  A travelling
+// wave is preceded by a fringe of such values: dividing them with __fdiv_rn took a 32 x 32
+// tile 23,000 cycles instead of 3,700 (its scaled path, lane by lane).
 static __host__ __device__ __attribute__((noinline)) float div_slow(float x, float d, double rd)
 {
     double q = mul_rn((double)x, rd);
     q = fma_rn(fma_rn(-q, (double)d, (double)x), rd, q);
-    const bool inf = bits_of(x) << 1 == 0xff000000u;
-    return inf || x == 0.0f ? x : to_float(q);
+    return div_key(x) >= div_key(INFINITY) ? x : to_float(q);
 }
 static __host__ __device__ __attribute__((noinline)) float4 div_slow4(float4 x, float d, double rd)
 {
     return make_float4(div_slow(x.x, d, rd), div_slow(x.y, d, rd), div_slow(x.z, d, rd), div_slow(x.w, d, rd));
 }
-// 2*bits - 1 of x: above r.lo for the operands the formula serves (zero wraps to the top)
-__host__ __device__ __forceinline__ unsigned div_key(float x) { return 2u * bits_of(x) - 1u; }
 __host__ __device__ __forceinline__ float div_by(float x, float d, const Rcp<float> &r)
 {
     float q = fma_rn(x, r.h, mul_rn(x, r.l));
