@@ -363,10 +363,12 @@ rsgpu_status Adjoint::create(const rsgpu_config *c, const rsgpu_adjoint_opts *o,
             // Snapshot2D::writeEdge (lib/snap.cpp:690-733): P on the columns x = lpml and
             // x = nx+lpml (the first C-PML column) over the interior rows, and on the rows
             // z = lpml and z = nz+lpml over the interior columns
+            // (the corner that the first column and row share, from the column alone: a cell
+            // restored by two blocks is a race, whose 16-bit values differ by block)
             const size_t p0 = L.f[A2_P] + org, l = (size_t)cfg.lpml;
             add(p0 + (l * L.pitch + l) * es, nz[i], 1, L.pitch);
             add(p0 + (l * L.pitch + nx[i] + l) * es, nz[i], 1, L.pitch);
-            add(p0 + (l * L.pitch + l) * es, 1, nx[i], L.pitch);
+            if (nx[i] > 1) add(p0 + (l * L.pitch + l + 1) * es, 1, nx[i] - 1, L.pitch);
             add(p0 + ((nz[i] + l) * L.pitch + l) * es, 1, nx[i], L.pitch);
             continue;
         }
