@@ -463,8 +463,9 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
     CU(cudaMemsetAsync(arena, 0, arena_bytes, stream));
     char *A = (char *)arena;
 
-    // ---- uploads: the parameters through a staging buffer (without one: row by row), and
-    // every table of the plan, contiguous in the arena, in one copy
+    // ---- uploads, all in the plan's stream (copies from pageable memory have read it when they
+    // return): the parameters through a staging buffer (without one: row by row), and every
+    // table of the plan, contiguous in the arena, in one copy
     const size_t tab0 = io[0].pt;
     std::vector<unsigned char> tabs(arena_bytes - tab0, 0);
     auto put_real = [&](size_t o, const std::vector<double> &v) {
@@ -569,7 +570,7 @@ rsgpu_status Plan::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, co
             }
         }
     }
-    CU(cudaMemcpy(d_meta, meta.data(), m_end, cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(d_meta, meta.data(), m_end, cudaMemcpyHostToDevice, stream));
     d_shots = (char *)d_meta + m_shots;
     d_injrec = (char *)d_meta + m_ir;
     d_tiles = (char *)d_meta + m_tiles;

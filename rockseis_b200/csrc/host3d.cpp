@@ -329,10 +329,9 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
         set_error("device allocation of %zu bytes failed", arena_bytes);
         return RSGPU_ERR_NOMEM;
     }
+    // the clearing and every upload below in the plan's stream (copies from pageable memory
+    // have read it when they return)
     CU(cudaMemsetAsync(arena, 0, arena_bytes, stream));
-    // the plan tables below go up with synchronous copies, which do not wait for the
-    // plan's non-blocking stream: let the clearing finish first
-    CU(cudaStreamSynchronize(stream));
     char *A = (char *)arena;
     std::vector<unsigned char> hb;
     auto put_real = [&](size_t o, const std::vector<double> &v) -> rsgpu_status {
@@ -342,11 +341,11 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
             if (es == 8) ((double *)hb.data())[k] = v[k];
             else ((float *)hb.data())[k] = (float)v[k];
         }
-        CU(cudaMemcpy(A + o, hb.data(), hb.size(), cudaMemcpyHostToDevice));
+        CU(cudaMemcpyAsync(A + o, hb.data(), hb.size(), cudaMemcpyHostToDevice, stream));
         return RSGPU_OK;
     };
     auto put_raw = [&](size_t o, const void *p, size_t bytes) -> rsgpu_status {
-        if (bytes) CU(cudaMemcpy(A + o, p, bytes, cudaMemcpyHostToDevice));
+        if (bytes) CU(cudaMemcpyAsync(A + o, p, bytes, cudaMemcpyHostToDevice, stream));
         return RSGPU_OK;
     };
     rsgpu_status st;
@@ -522,7 +521,7 @@ rsgpu_status Plan3D::create(const rsgpu_config *c, int ns, const rsgpu_shot *s, 
     std::memcpy(meta.data() + m_tiles, tiles.data(), tiles.size() * sizeof(Tile3D));
     std::memcpy(meta.data() + m_coef, coefs.data(), coefs.size());
     h_coefs = coefs;
-    CU(cudaMemcpy(d_meta, meta.data(), m_end, cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(d_meta, meta.data(), m_end, cudaMemcpyHostToDevice, stream));
     d_shots = (char *)d_meta + m_shots;
     d_injrec = (char *)d_meta + m_ir;
     d_tiles = (char *)d_meta + m_tiles;

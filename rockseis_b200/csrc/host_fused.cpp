@@ -165,7 +165,7 @@ rsgpu_status Plan::setup_fused(const std::vector<std::vector<int>> &inj_pts)
             }
     }
     CU(dev_alloc(&d_zm, bytes, stream));
-    CU(cudaMemcpy(d_zm, h.data(), bytes, cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(d_zm, h.data(), bytes, cudaMemcpyHostToDevice, stream));
     char *Z = (char *)d_zm;
     if (prec == PREC_F64)
         fill_zm_args<double>(zm_args, *this, Z + o_items, zm_nitems, Z + o_inj, Z + o_recs, nrecs, Z + o_maps);

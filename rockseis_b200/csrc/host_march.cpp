@@ -77,7 +77,7 @@ rsgpu_status Plan::setup_march(const std::vector<unsigned char> &coefs)
         }
     }
     CU(dev_alloc(&d_march, bytes, stream));
-    CU(cudaMemcpy(d_march, h.data(), bytes, cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(d_march, h.data(), bytes, cudaMemcpyHostToDevice, stream));
     March2DArgs &a = march_args;
     a.shots = (const Shot2D<float> *)d_shots;
     a.items = (const MarchItem *)d_march;

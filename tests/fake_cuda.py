@@ -21,7 +21,7 @@ FAKE_CUDA = r"""
 #include "rsgpu_host.h"
 
 static size_t capacity = ~size_t(0), used = 0;
-static int padded = 0, by_rows = 0;
+static int padded = 0, by_rows = 0, unordered = 0;
 static std::map<void *, size_t> live;
 static cudaStream_t const stream = (cudaStream_t)0x10;
 
@@ -54,7 +54,13 @@ cudaError_t cudaFreeAsync(void *p, cudaStream_t)
     return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) { std::memset(p, v, n); return cudaSuccess; }
-cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind kind)
+{
+    // outside the order of a non-blocking stream, and from pageable memory not even done on return
+    unordered += kind == cudaMemcpyHostToDevice;
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) { std::memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpy2DAsync(void *d, size_t dp, const void *s, size_t sp, size_t w, size_t h, cudaMemcpyKind, cudaStream_t)
 {
@@ -83,7 +89,9 @@ namespace rsgpu {
 int tile_count_2d() { return 11; }
 TileShape tile_shape_2d(int) { return {32, 16, 2, 8}; }
 int coef_row_stride() { return 9; }
-int zm_strip_width() { return 64; }
+int zm_strip_width() { return 112; }
+int zm_resident_ctas(int, int) { return 296; }
+int march_resident_ctas() { return 4; }
 cudaError_t upload_padded(void *dst, int pitch, long long plane, const void *src, int w, int h, int d, int es, void *staging, cudaStream_t)
 {
     padded++;

@@ -2,7 +2,7 @@
 
 A plan fits where its own arrays fit: the buffer that its uploads go through is given back
 before the later arrays are allocated, and where it is not to be had the uploads go row by
-row, with the same contents.
+row, with the same contents.  Every upload is ordered by the plan's stream.
 """
 import pytest
 
@@ -15,7 +15,7 @@ using namespace rsgpu;
 template <typename P>
 static int make(P &p, const rsgpu_config &c, std::vector<rsgpu_shot> &s, std::vector<unsigned char> &image)
 {
-    padded = by_rows = 0;
+    padded = by_rows = unordered = 0;
     const int st = p.create(&c, (int)s.size(), s.data());
     if (st == RSGPU_OK) image.assign((unsigned char *)p.arena, (unsigned char *)p.arena + p.arena_bytes);
     return st;
@@ -43,7 +43,7 @@ static void both(const char *name, rsgpu_config c, int ns, int nx, int ny, int n
         p.adjoint_steps = adjoint;
         if (make(p, c, s, a) != RSGPU_OK) exit(1);
         own = used;
-        printf("%s %d %d ", name, padded, by_rows);
+        printf("%s %d %d %d ", name, unordered, padded, by_rows);
     }
     if (used) exit(2);
     capacity = own;
@@ -71,6 +71,8 @@ int main()
     both<Plan3D>("e3", c, 2, 20, 9, 11, true);    // work arrays behind the uploads
     c.physics = RSGPU_ACOUSTIC3D;
     both<Plan3D>("a3", c, 3, 20, 9, 11, false);
+    c.physics = RSGPU_ELASTIC2D;
+    for (c.launch_mode = 3; c.launch_mode <= 4; c.launch_mode++) both<Plan>("e2", c, 2, 160, 0, 145, false);
 }
 """
 
@@ -84,7 +86,12 @@ def lines(tmp_path_factory):
 @pytest.mark.parametrize("row,uploads,staged", [(0, 150, True), (1, 6, False), (2, 16, True), (3, 12, False)])
 def test_plan_fits_where_its_arrays_fit(lines, row, uploads, staged):
     # staged: the later arrays leave the room that the staging buffer needs before them
-    _, padded, by_rows, status, padded2, by_rows2, same = lines[row]
+    _, _, padded, by_rows, status, padded2, by_rows2, same = lines[row]
     assert (padded, by_rows) == (uploads, 0)
     assert (status, same) == (0, 1)
     assert (padded2, by_rows2) == ((uploads, 0) if staged else (0, uploads))
+
+
+def test_uploads_are_ordered_by_the_plans_stream(lines):
+    assert len(lines) == 6 and all(status == 0 for _, _, _, _, status, *_ in lines)
+    assert [unordered for _, unordered, *_ in lines] == [0] * 6
